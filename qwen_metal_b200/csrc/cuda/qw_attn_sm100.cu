@@ -234,6 +234,26 @@ __device__ __forceinline__ bool mbar_wait(SharedControl *ctl, unsigned long long
     return mbar_wait_slow(ctl, bar, parity, status, where, tile);
 }
 
+// The same for all lanes of a warp at once: true when every lane saw the phase complete.
+__device__ __forceinline__ bool mbar_wait_warp(SharedControl *ctl, unsigned long long *bar,
+                                               uint32_t parity, uint32_t *status, uint32_t where,
+                                               uint32_t tile) {
+    return __all_sync(0xffffffffu, mbar_wait(ctl, bar, parity, status, where, tile)) != 0;
+}
+
+// A value the compiler knows to be the same in all lanes of the (converged) warp.
+template <typename T>
+__device__ __forceinline__ T uniform(T v) {
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(pred));
+    return pred != 0;
+}
+
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map,
                                             unsigned long long *bar, int c0, int c1, int c2) {
     asm volatile(
@@ -1033,7 +1053,10 @@ __device__ __forceinline__ void softmax_pair_role(const KernelParams &p, SharedC
 }
 
 // ---------------------------------------------------------------------------
-// MMA issue role (one thread).
+// MMA issue role: one warp.  All lanes run the loop and one is elected around the
+// instructions (always the same one, so its commits cover its MMAs): the operands of
+// the MMAs then stay in uniform registers, where in a one-lane branch each of them is
+// moved there first, more clocks per MMA than the 64 it executes in.
 // ---------------------------------------------------------------------------
 // High words of the two descriptor kinds (everything but the start address).
 constexpr uint32_t desc_hi(uint32_t sbo_bytes) {
@@ -1073,11 +1096,11 @@ __device__ __forceinline__ void issue_pv(uint32_t d_tmem, uint32_t p_tmem, uint3
 __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *ctl,
                                          uint8_t *smem_q, uint8_t *smem_kv, bool paired) {
     // Whole form: both sub-tiles walk the visited tiles from 0; u counts them.
-    const int n0 = ctl->tile_count[0], n1 = ctl->tile_count[1];
+    const int n0 = uniform(ctl->tile_count[0]), n1 = uniform(ctl->tile_count[1]);
     const int n_max = max(n0, n1);
     int j = 0;
     if (j >= n_max) return;
-    const uint32_t tmem = ctl->tmem_base;
+    const uint32_t tmem = uniform(ctl->tmem_base);
     // Low descriptor words: start address in 16-byte units plus the fixed LBO field.
     const uint32_t q_lo[2] = {(smem_u32(smem_q) >> 4) | kDescLoKMajor,
                               (smem_u32(smem_q + kTileBytes) >> 4) | kDescLoKMajor};
@@ -1095,23 +1118,24 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
 #pragma unroll
     for (int i = 0; i < 2; ++i)
         if (n_sub[i] > 0 &&
-            !mbar_wait(ctl, &ctl->bars[kBarQFull + i], 0, p.status, where | (kBarQFull + i), 0))
+            !mbar_wait_warp(ctl, &ctl->bars[kBarQFull + i], 0, p.status, where | (kBarQFull + i), 0))
             return;
     {
         uint32_t slot = t % kStages, par = (t / kStages) & 1u;
         ++t;
-        if (!mbar_wait(ctl, &ctl->bars[kBarKvFull + slot], par, p.status,
+        if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + slot], par, p.status,
                        where | (kBarKvFull + slot), (uint32_t)j))
             return;
         tc_fence_after();
         const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescLoKMajor;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-            if (j < n_sub[i]) {
+            if (j < n_sub[i] && elect_one()) {
                 issue_qk(s_tmem[i], q_lo[i], k_lo);
                 tc_commit(&ctl->bars[kBarSFull + i]);
             }
-        tc_commit(&ctl->bars[kBarKvEmpty + slot]);
+        if (elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + slot]);
+        __syncwarp();
     }
     while (j < n_max) {
         const int jn = j + 1;
@@ -1124,7 +1148,7 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             ++t;
         }
         QW_TRACE(2, 6, j);
-        if (!mbar_wait(ctl, &ctl->bars[kBarKvFull + v_slot], v_par, p.status,
+        if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + v_slot], v_par, p.status,
                        where | (kBarKvFull + v_slot), (uint32_t)j))
             return;
         QW_TRACE(2, 7, j);
@@ -1134,34 +1158,39 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (j < n_sub[i]) {
-                if (!mbar_wait(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
+                if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
                                where | (kBarPFull + i), (uint32_t)j))
                     return;
                 p_phase[i] ^= 1u;
                 tc_fence_after();
                 QW_TRACE(2, i, j);
-                issue_pv(o_tmem[i], s_tmem[i], v_lo, o_started[i], paired);
+                if (elect_one()) issue_pv(o_tmem[i], s_tmem[i], v_lo, o_started[i], paired);
+                __syncwarp();
                 o_started[i] = true;
                 QW_TRACE(2, 4 + i, j);
             }
-            if (i == 1) tc_commit(&ctl->bars[kBarKvEmpty + v_slot]);
+            if (i == 1 && elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + v_slot]);
+            __syncwarp();
             if (jn < n_max && jn < n_sub[i]) {
                 if (!k_ready) {
                     QW_TRACE(2, 8, jn);
-                    if (!mbar_wait(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
+                    if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
                                    where | (kBarKvFull + k_slot), (uint32_t)jn))
                         return;
                     tc_fence_after();
                     k_ready = true;
                     QW_TRACE(2, 9, jn);
                 }
-                issue_qk(s_tmem[i], q_lo[i], k_lo);
-                tc_commit(&ctl->bars[kBarSFull + i]);
+                if (elect_one()) {
+                    issue_qk(s_tmem[i], q_lo[i], k_lo);
+                    tc_commit(&ctl->bars[kBarSFull + i]);
+                }
+                __syncwarp();
                 QW_TRACE(2, 2 + i, jn);
 #ifdef QW_ATTN_TRACE_SERIAL
                 // Probe: wait until the group just issued has executed.
                 tc_commit(&ctl->bars[kBarDebug]);
-                if (!mbar_wait(ctl, &ctl->bars[kBarDebug], dbg_phase, p.status, where | kBarDebug, 0))
+                if (!mbar_wait_warp(ctl, &ctl->bars[kBarDebug], dbg_phase, p.status, where | kBarDebug, 0))
                     return;
                 dbg_phase ^= 1u;
                 QW_TRACE(2, 10 + i, jn);
@@ -1170,15 +1199,18 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
         }
         if (jn < n_max) {
             if (!k_ready &&
-                !mbar_wait(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
+                !mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
                            where | (kBarKvFull + k_slot), (uint32_t)jn))
                 return;
-            tc_commit(&ctl->bars[kBarKvEmpty + k_slot]);
+            if (elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + k_slot]);
+            __syncwarp();
         }
         j = jn;
     }
-    tc_commit(&ctl->bars[kBarOFinal + 0]);
-    tc_commit(&ctl->bars[kBarOFinal + 1]);
+    if (elect_one()) {
+        tc_commit(&ctl->bars[kBarOFinal + 0]);
+        tc_commit(&ctl->bars[kBarOFinal + 1]);
+    }
 }
 
 // Split form: sub-tile 0 walks visited tiles [0, la), sub-tile 1 [la, la + lb),
@@ -1190,9 +1222,9 @@ __device__ __forceinline__ uint32_t pair_b(int s) { return 2u * (uint32_t)(2 * s
 
 __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedControl *ctl,
                                                uint8_t *smem_q, uint8_t *smem_kv, bool paired) {
-    const int la = ctl->tile_count[0], lb = ctl->tile_count[1];
+    const int la = uniform(ctl->tile_count[0]), lb = uniform(ctl->tile_count[1]);
     if (la <= 0) return;
-    const uint32_t tmem = ctl->tmem_base;
+    const uint32_t tmem = uniform(ctl->tmem_base);
     const uint32_t q_lo = (smem_u32(smem_q) >> 4) | kDescLoKMajor;
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;
     const uint32_t s_tmem[2] = {tmem + kTmemS0, tmem + kTmemS1};
@@ -1204,7 +1236,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
 #define QW_RING_WAIT(t_, lo_fixed_, out_)                                                       \
     {                                                                                           \
         const uint32_t slot_ = (t_) % kStages, par_ = ((t_) / kStages) & 1u;                    \
-        if (!mbar_wait(ctl, &ctl->bars[kBarKvFull + slot_], par_, p.status,                     \
+        if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + slot_], par_, p.status,                     \
                        where | (kBarKvFull + slot_), (uint32_t)(t_)))                           \
             return;                                                                             \
         tc_fence_after();                                                                       \
@@ -1212,17 +1244,23 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
     }
 #define QW_RING_FREE(t_) tc_commit(&ctl->bars[kBarKvEmpty + ((t_) % kStages)])
 
-    if (!mbar_wait(ctl, &ctl->bars[kBarQFull + 0], 0, p.status, where | kBarQFull, 0)) return;
+    if (!mbar_wait_warp(ctl, &ctl->bars[kBarQFull + 0], 0, p.status, where | kBarQFull, 0)) return;
     uint32_t desc;
     QW_RING_WAIT(pair_a(0, lb), kDescLoKMajor, desc);
-    issue_qk(s_tmem[0], q_lo, desc);
-    tc_commit(&ctl->bars[kBarSFull + 0]);
-    QW_RING_FREE(pair_a(0, lb));
+    if (elect_one()) {
+        issue_qk(s_tmem[0], q_lo, desc);
+        tc_commit(&ctl->bars[kBarSFull + 0]);
+        QW_RING_FREE(pair_a(0, lb));
+    }
+    __syncwarp();
     if (lb > 0) {
         QW_RING_WAIT(pair_b(0), kDescLoKMajor, desc);
-        issue_qk(s_tmem[1], q_lo, desc);
-        tc_commit(&ctl->bars[kBarSFull + 1]);
-        QW_RING_FREE(pair_b(0));
+        if (elect_one()) {
+            issue_qk(s_tmem[1], q_lo, desc);
+            tc_commit(&ctl->bars[kBarSFull + 1]);
+            QW_RING_FREE(pair_b(0));
+        }
+        __syncwarp();
     }
     for (int s = 0; s < la; ++s) {
 #pragma unroll
@@ -1231,26 +1269,34 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             if (s >= count) continue;
             const uint32_t t_now = i ? pair_b(s) : pair_a(s, lb);
             QW_RING_WAIT(t_now + 1, kDescLoVMajor, desc);
-            if (!mbar_wait(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
+            if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
                            where | (kBarPFull + i), (uint32_t)s))
                 return;
             p_phase[i] ^= 1u;
             tc_fence_after();
-            issue_pv(o_tmem[i], s_tmem[i], desc, s > 0, paired);
-            QW_RING_FREE(t_now + 1);
+            if (elect_one()) {
+                issue_pv(o_tmem[i], s_tmem[i], desc, s > 0, paired);
+                QW_RING_FREE(t_now + 1);
+            }
+            __syncwarp();
             if (s + 1 < count) {
                 const uint32_t t_next = i ? pair_b(s + 1) : pair_a(s + 1, lb);
                 QW_RING_WAIT(t_next, kDescLoKMajor, desc);
-                issue_qk(s_tmem[i], q_lo, desc);
-                tc_commit(&ctl->bars[kBarSFull + i]);
-                QW_RING_FREE(t_next);
+                if (elect_one()) {
+                    issue_qk(s_tmem[i], q_lo, desc);
+                    tc_commit(&ctl->bars[kBarSFull + i]);
+                    QW_RING_FREE(t_next);
+                }
+                __syncwarp();
             }
         }
     }
 #undef QW_RING_WAIT
 #undef QW_RING_FREE
-    tc_commit(&ctl->bars[kBarOFinal + 0]);
-    tc_commit(&ctl->bars[kBarOFinal + 1]);
+    if (elect_one()) {
+        tc_commit(&ctl->bars[kBarOFinal + 0]);
+        tc_commit(&ctl->bars[kBarOFinal + 1]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1335,7 +1381,7 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
     SharedControl *ctl = reinterpret_cast<SharedControl *>(smem + kSmemData);
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be warp-uniform
     const int lane = tid & 31;
     // CTA -> unit.  Units are numbered batch-major, then head, then query block
     // with the heaviest blocks first (rows late in the joint sequence see the most
@@ -1484,10 +1530,8 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
     }
     if (tid < kSoftmaxThreads) {
     } else if (warp == kMmaWarp) {
-        if (lane == 0) {
-            if (split) mma_role_split(p, ctl, smem_q, smem_kv, paired);
-            else mma_role(p, ctl, smem_q, smem_kv, paired);
-        }
+        if (split) mma_role_split(p, ctl, smem_q, smem_kv, paired);
+        else mma_role(p, ctl, smem_q, smem_kv, paired);
     } else if (warp == kTmaWarp && lane == 0) {
         tma_role(p, ctl, smem_kv, &map_k, &map_v, b, kvh, split);
         // Q loads of active sub-tiles must have landed as well.
