@@ -204,6 +204,20 @@ __device__ __forceinline__ bool mbar_try(unsigned long long *bar, uint32_t parit
     return done != 0;
 }
 
+// Has the phase completed?  (test_wait answers at once; try_wait may suspend the warp
+// until it has.)
+__device__ __forceinline__ bool mbar_test(unsigned long long *bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 // Bounded wait.  Returns false when the budget ran out here (recorded) or
 // another thread of the CTA already gave up.
 __device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, unsigned long long *bar,
@@ -932,7 +946,9 @@ __device__ __forceinline__ void softmax_pair_role(const KernelParams &p, SharedC
             {
                 const int nsub = 1 - sub, ns = sub ? s + 1 : s;
                 if (ns < count[nsub]) {
-                    const bool ready = mbar_try(&ctl->bars[kBarSFull + nsub], phase[nsub]);
+                    // (asked without suspending: the next scores may in turn depend on
+                    // the P this warp has yet to publish, as they do with few key tiles)
+                    const bool ready = mbar_test(&ctl->bars[kBarSFull + nsub], phase[nsub]);
                     if (__all_sync(0xffffffffu, ready)) {
                         phase[nsub] ^= 1u;
                         tc_fence_after();
@@ -1154,7 +1170,10 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
         QW_TRACE(2, 7, j);
         const uint32_t v_lo = (kv_lo + v_slot * (kTileBytes >> 4)) | kDescLoVMajor;
         const uint32_t k_lo = (kv_lo + k_slot * (kTileBytes >> 4)) | kDescLoKMajor;
-        bool k_ready = false;
+        if (jn < n_max &&
+            !mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
+                       where | (kBarKvFull + k_slot), (uint32_t)jn))
+            return;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (j < n_sub[i]) {
@@ -1172,15 +1191,6 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             if (i == 1 && elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + v_slot]);
             __syncwarp();
             if (jn < n_max && jn < n_sub[i]) {
-                if (!k_ready) {
-                    QW_TRACE(2, 8, jn);
-                    if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
-                                   where | (kBarKvFull + k_slot), (uint32_t)jn))
-                        return;
-                    tc_fence_after();
-                    k_ready = true;
-                    QW_TRACE(2, 9, jn);
-                }
                 if (elect_one()) {
                     issue_qk(s_tmem[i], q_lo[i], k_lo);
                     tc_commit(&ctl->bars[kBarSFull + i]);
@@ -1198,10 +1208,6 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             }
         }
         if (jn < n_max) {
-            if (!k_ready &&
-                !mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
-                           where | (kBarKvFull + k_slot), (uint32_t)jn))
-                return;
             if (elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + k_slot]);
             __syncwarp();
         }
@@ -1480,12 +1486,18 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         // (split form: both warpgroups work on the same 128 rows)
         my_row = row0 + (split ? 0u : (uint32_t)sub * kTileM) + (uint32_t)tid_in_group;
         my_limit = row_limit(p, b, my_row);
-        // (paired: this thread also works on the same row of the other sub-tile)
-        if (paired)
-            other_limit = split ? my_limit
-                                : row_limit(p, b, row0 + (uint32_t)(1 - sub) * kTileM +
-                                                      (uint32_t)tid_in_group);
         int warp_max = my_limit;
+        // A row past the end is computed like its neighbours and never stored: with a
+        // limit of 0 it would send its whole warp through the masked path on every tile
+        // (600 -> 1500 clocks a tile for the row maximum alone).
+        if (my_row >= p.q_rows) my_limit = 0x7fffffff;
+        // (paired: this thread also works on the same row of the other sub-tile)
+        if (paired) {
+            const uint32_t other_row = row0 + (uint32_t)(1 - sub) * kTileM + (uint32_t)tid_in_group;
+            other_limit = split                    ? my_limit
+                          : other_row < p.q_rows ? row_limit(p, b, other_row)
+                                                   : 0x7fffffff;
+        }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1)
             warp_max = max(warp_max, __shfl_xor_sync(0xffffffffu, warp_max, off));
