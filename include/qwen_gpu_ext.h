@@ -216,9 +216,9 @@ int qw_gpu_tensor_read_lane(h3_gpu *gpu, const h3_gpu_tensor *tensor, void *host
                             size_t elements, int lane);
 /* Select the attention kernel: "sm100" (default; the 256-row blocks of the last,
  * partly filled wave of CTAs run split in two), "sm100-whole" (same kernel, no
- * block is ever split), "sm100-row" (same kernel; with a score bound the softmax
- * keeps one thread per query row instead of pairing the warpgroups on each
- * sub-tile) or "scalar" (diagnostic fp32 kernel).  Returns 0 on an unknown name. */
+ * block is ever split), "sm100-row" (the same as "sm100": one softmax thread per query
+ * row is the only organisation) or "scalar" (diagnostic fp32 kernel).  Returns 0 on an
+ * unknown name. */
 int qw_gpu_set_attention_kernel(h3_gpu *gpu, const char *name);
 /* Test hook for the attention kernel's bounded waits: later launches use a wait
  * budget of wait_cycles SM cycles and their TMA producer leaves out every key tile

@@ -33,8 +33,7 @@
 //
 // Softmax.  Callers that promise bounded row norms (the DiT layer's QK-norm) get
 // P = exp2(score*c - bound) against one fixed exponent: no row maximum, no
-// rescaling, scores streamed out of TMEM in 32-column chunks; short launches pair
-// both warpgroups on one sub-tile's keys at a time.  Other callers get the
+// rescaling, scores streamed out of TMEM in 32-column chunks.  Other callers get the
 // running maximum with lazy rescaling.
 //
 // Wave tail.  The grid is one CTA per (batch, head, 256-row block), heaviest
@@ -73,13 +72,19 @@ constexpr int kTileBytes = kTileN * kHeadDim * 2;  // 32 KiB
 constexpr int kHalfTileBytes = kTileBytes / 2;     // one 64-column TMA box
 constexpr int kThreads = 384;
 // setmaxnreg only redistributes the registers the CTA got at launch
-// (kThreads * 168 = 64512): 2 * 128 * 208 + 128 * 88 = 64512.  Asking for more
+// (kThreads * 168 = 64512): 2 * 128 * 224 + 128 * 56 = 64512.  Asking for more
 // would block the second softmax warpgroup forever.
 constexpr int kLaunchRegs = 168;
-constexpr int kSoftmaxRegs = 208;
-constexpr int kOtherRegs = 88;
+constexpr int kSoftmaxRegs = 224;
+constexpr int kOtherRegs = 56;
 static_assert(2 * 128 * kSoftmaxRegs + 128 * kOtherRegs <= kThreads * kLaunchRegs,
               "setmaxnreg budget exceeds the launch allocation");
+// P of a tile is published in two parts, the first kPart * 16 keys and the rest: P V of
+// the first part runs under the softmax of the rest, which takes it out of the chain
+// S -> softmax -> P V -> next S that bounds the kernel.  With the fixed exponent the later
+// cut is the better one (six heads, 4352 keys: 622 us with 4, 601 us with 6), with the
+// running maximum the earlier (8188 x 8211 keys: 1018 us with 4, 1079 us with 6).
+constexpr int kPartRunning = 4, kPartBounded = 6;
 constexpr int kSoftmaxThreads = 256;
 constexpr int kMmaWarp = 8;
 constexpr int kTmaWarp = 9;
@@ -96,7 +101,8 @@ enum Barrier : int {
     kBarKvFull = 2,                       // kStages
     kBarKvEmpty = kBarKvFull + kStages,   // kStages
     kBarSFull = kBarKvEmpty + kStages,    // 2: S_i complete in TMEM
-    kBarPFull = kBarSFull + 2,            // 2: P_i written (one arrival per warp)
+    kBarPFirst = kBarSFull + 2,           // 2: first part of P_i written (one arrival per warp)
+    kBarPFull = kBarPFirst + 2,           // 2: the rest of P_i written
     kBarOFinal = kBarPFull + 2,           // 2: last P V of sub-tile i complete
     kBarDebug = kBarOFinal + 2,           // trace builds: group completion probe
     kBarEpi = kBarDebug + 1,              // 2: output tile of sub-tile i staged in shared memory
@@ -118,8 +124,6 @@ struct __align__(16) SharedControl {
     int tile_first[2], tile_count[2];
     float merge_m[kTileM];  // split form: sub-tile 1's reference exponent and row sum
     float merge_l[kTileM];
-    // Paired organisation: row sums of the two key halves, [key half][sub-tile][row].
-    float pair_l[2][2][kTileM];
 };
 
 constexpr size_t kSmemData = (size_t)(2 + kStages) * kTileBytes;
@@ -144,7 +148,6 @@ struct KernelParams {
     // score_bound[1], so |q.k| <= their product and the softmax can use one fixed
     // reference exponent instead of a running row maximum.
     const float *score_bound;
-    int pair_org;  // fixed-exponent softmax: both warpgroups share each sub-tile's keys
     int head_major_out;
     // Sharded runs: the rows are stored at this rank's head columns of n_out
     // full-width outputs (peer-mapped pointers allowed).  out_heads_total is the
@@ -178,14 +181,6 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// The P and staging barriers count one arrival per softmax warp of the CTA (8).
-// Where only one warpgroup works on a sub-tile, each of its four warps arrives
-// for two.
-__device__ __forceinline__ void mbar_arrive_twice(unsigned long long *bar) {
-    mbar_arrive(bar);
-    mbar_arrive(bar);
-}
-
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
                  "r"(bytes)
@@ -197,20 +192,6 @@ __device__ __forceinline__ bool mbar_try(unsigned long long *bar, uint32_t parit
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-
-// Has the phase completed?  (test_wait answers at once; try_wait may suspend the warp
-// until it has.)
-__device__ __forceinline__ bool mbar_test(unsigned long long *bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done)
         : "r"(smem_u32(bar)), "r"(parity)
@@ -440,28 +421,6 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     return d;
 }
 
-// 2^x for a pair on the FMA pipe instead of the special-function unit, which
-// the exponentials of a 128x128 tile otherwise keep as busy as its MMAs keep the
-// tensor pipe: n = round(x) by the 1.5*2^23 trick, r = x - n in [-0.5, 0.5], a
-// cubic for 2^r (exact at r = 0, max relative error 1.2e-4, far below the bf16 rounding of P),
-// then n is added into the exponent field.  x is clamped at -127 (result 0).
-__device__ __forceinline__ float2 exp2_poly2(float2 x) {
-    const float kMagic = 12582912.0f;  // 1.5 * 2^23
-    x.x = fmaxf(x.x, -127.0f);
-    x.y = fmaxf(x.y, -127.0f);
-    const float2 t = fadd2(x, make_float2(kMagic, kMagic));
-    const float2 n = fadd2(t, make_float2(-kMagic, -kMagic));
-    const float2 r = ffma2(n, make_float2(-1.0f, -1.0f), x);
-    float2 q = ffma2(r, make_float2(0.05541782081127167f, 0.05541782081127167f),
-                     make_float2(0.24221134185791016f, 0.24221134185791016f));
-    q = ffma2(q, r, make_float2(0.6931995153427124f, 0.6931995153427124f));
-    q = ffma2(q, r, make_float2(1.0f, 1.0f));
-    float2 out;
-    out.x = __uint_as_float(__float_as_uint(q.x) + (__float_as_uint(t.x) << 23));
-    out.y = __uint_as_float(__float_as_uint(q.y) + (__float_as_uint(t.y) << 23));
-    return out;
-}
-
 // Pipeline event log, compiled in only with -DQW_ATTN_TRACE (a debugging build).
 #ifdef QW_ATTN_TRACE
 // Event log for pipeline analysis: (role, event, tile) and the SM clock, written
@@ -512,11 +471,19 @@ __device__ __forceinline__ int visited_tiles(int tiles, int lo, int hi) {
 // ---------------------------------------------------------------------------
 // Softmax + epilogue role: 128 threads per sub-tile, one query row each.
 // ---------------------------------------------------------------------------
+// The first part of P is complete once its stores, issued a chunk of exponentials ago,
+// have landed: P V of these keys starts under the softmax of the others.
+__device__ __forceinline__ void publish_p_first(unsigned long long *bar, int tid_in_group) {
+    tmem_wait_st();
+    tc_fence_before();
+    if ((tid_in_group & 31) == 0) mbar_arrive(bar);
+}
+
 // kBounded: the caller promised |score * scale * log2(e)| <= bound (see
 // KernelParams::score_bound), so P = exp2(score*c - bound) needs no row maximum:
 // the scores stream out of TMEM 32 columns at a time, each chunk's exponentials
 // run under the next chunk's load, and O is never rescaled.
-template <int kPoly, bool kBounded>
+template <bool kBounded>
 __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedControl *ctl,
                                              const OutMaps &maps_out, uint8_t *stage, int sub,
                                              int tid_in_group, int my_limit, uint32_t b, uint32_t h,
@@ -528,15 +495,15 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
     const uint32_t tmem_s = tmem + lane_base + (sub ? kTmemS1 : kTmemS0);
     const uint32_t tmem_o = tmem + lane_base + (sub ? kTmemO1 : kTmemO0);
     unsigned long long *bar_s = &ctl->bars[kBarSFull + sub];
+    unsigned long long *bar_p_first = &ctl->bars[kBarPFirst + sub];
     unsigned long long *bar_p = &ctl->bars[kBarPFull + sub];
     const int pad_lo = p.text_pad ? (int)p.text_len[b] : 0;
     const int pad_hi = (int)p.text_pad;
-    const float c = p.scale_log2;
-    const bool neg = c < 0.0f;
+    const float c = p.scale_log2;  // positive (the host sends other scales elsewhere)
 
     [[maybe_unused]] uint32_t trace_cursor = 0;
-    float m_run = -INFINITY;  // running extreme of the raw scores (max, or min when c < 0)
-    float m_ref = -INFINITY;  // extreme the stored exponents refer to
+    float m_run = -INFINITY;  // running maximum of the raw scores
+    float m_ref = -INFINITY;  // maximum the stored exponents refer to
     float l_run = 0.0f;
     uint32_t phase = 0;
     bool ok = true;
@@ -580,17 +547,12 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
                     float2 x = ffma2(make_float2(__uint_as_float(cur[2 * i]),
                                                  __uint_as_float(cur[2 * i + 1])),
                                      cs2, bias2);
-                    float2 pr;
-                    if ((i & 3) < kPoly) {
-                        pr = exp2_poly2(x);
-                    } else {
-                        pr.x = fast_exp2(x.x);
-                        pr.y = fast_exp2(x.y);
-                    }
+                    const float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
                     if (i & 1) sum_b = fadd2(sum_b, pr);
                     else sum_a = fadd2(sum_a, pr);
                     pk[i] = pack_bf16(pr.x, pr.y);
                 }
+                if (chunk == kPartBounded / 2) publish_p_first(bar_p_first, tid_in_group);
                 // P chunk c lands on columns [16c, 16c+16): scores already consumed.
                 QW_TMEM_ST16(tmem_s + chunk * 16, pk);
                 if (chunk == 1 && tid_in_group == 0) QW_TRACE(sub, 2, j);
@@ -598,7 +560,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
             if (tid_in_group == 0) QW_TRACE(sub, 3, j);
             tmem_wait_st();
             tc_fence_before();
-            if ((tid_in_group & 31) == 0) mbar_arrive_twice(bar_p);
+            if ((tid_in_group & 31) == 0) mbar_arrive(bar_p);
             if (tid_in_group == 0) QW_TRACE(sub, 4, j);
             ++processed;
         }
@@ -625,45 +587,33 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
         const int key0 = j * kTileN;
         const bool pad_hit = pad_hi > pad_lo && key0 < pad_hi && key0 + kTileN > pad_lo;
         const bool boundary = __any_sync(0xffffffffu, key0 + kTileN > my_limit) || pad_hit;
-        const float sign = neg ? -1.0f : 1.0f;
         if (boundary) {
 #pragma unroll
             for (int i = 0; i < 128; ++i) {
                 int key = key0 + i;
                 bool visible = key < my_limit && !(key >= pad_lo && key < pad_hi);
-                s[i] = visible ? s[i] : __float_as_uint(neg ? INFINITY : -INFINITY);
+                s[i] = visible ? s[i] : __float_as_uint(-INFINITY);
             }
         }
-        // Row extreme of sign*score (four independent chains).
+        // Row maximum (four independent chains).
         float e0 = -INFINITY, e1 = -INFINITY, e2 = -INFINITY, e3 = -INFINITY;
-        if (!neg) {
 #pragma unroll
-            for (int i = 0; i < 128; i += 8) {
-                e0 = fmax3(e0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
-                e1 = fmax3(e1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
-                e2 = fmax3(e2, __uint_as_float(s[i + 4]), __uint_as_float(s[i + 5]));
-                e3 = fmax3(e3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 128; i += 4) {
-                e0 = fmaxf(e0, -__uint_as_float(s[i]));
-                e1 = fmaxf(e1, -__uint_as_float(s[i + 1]));
-                e2 = fmaxf(e2, -__uint_as_float(s[i + 2]));
-                e3 = fmaxf(e3, -__uint_as_float(s[i + 3]));
-            }
+        for (int i = 0; i < 128; i += 8) {
+            e0 = fmax3(e0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+            e1 = fmax3(e1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+            e2 = fmax3(e2, __uint_as_float(s[i + 4]), __uint_as_float(s[i + 5]));
+            e3 = fmax3(e3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
         }
-        const float m_tile = fmaxf(fmaxf(e0, e1), fmaxf(e2, e3));  // in sign*score units
+        const float m_tile = fmaxf(fmaxf(e0, e1), fmaxf(e2, e3));
         const float m_new = fmaxf(m_run, m_tile);
         m_run = m_new;
-        const float ac = fabsf(c);
         // Does the reference point have to move?  (first finite value, or drift > threshold)
         const bool move = (m_new != -INFINITY) &&
-                          (m_ref == -INFINITY || (m_new - m_ref) * ac > kRescaleThreshold);
+                          (m_ref == -INFINITY || (m_new - m_ref) * c > kRescaleThreshold);
         const bool any_move = __any_sync(0xffffffffu, move && processed > 0 && m_ref != -INFINITY);
         float alpha = 1.0f;
         if (move) {
-            alpha = (m_ref == -INFINITY) ? 0.0f : fast_exp2((m_ref - m_new) * ac);
+            alpha = (m_ref == -INFINITY) ? 0.0f : fast_exp2((m_ref - m_new) * c);
             m_ref = m_new;
         }
         if (any_move) {
@@ -683,12 +633,10 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
         l_run *= alpha;
         if (tid_in_group == 0) QW_TRACE(sub, 2, j);
 
-        // P = exp2(sign*score*|c| - m_ref*|c|) as bf16 pairs, written over S.
-        const float bias = (m_ref == -INFINITY) ? 0.0f : -m_ref * ac;
-        const float cs = sign * ac;
-        // kPoly of every 4 pairs take the polynomial instead of the SFU.  P goes
-        // back to TMEM 32 keys (16 packed columns) at a time.
-        const float2 cs2 = make_float2(cs, cs), bias2 = make_float2(bias, bias);
+        // P = exp2(score*c - m_ref*c) as bf16 pairs, written over S 32 keys (16 packed
+        // columns) at a time.
+        const float bias = (m_ref == -INFINITY) ? 0.0f : -m_ref * c;
+        const float2 cs2 = make_float2(c, c), bias2 = make_float2(bias, bias);
         float2 sum_a = make_float2(0.0f, 0.0f), sum_b = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (int chunk = 0; chunk < 4; ++chunk) {
@@ -698,23 +646,18 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
                 const int e = chunk * 32 + 2 * i;
                 float2 x = ffma2(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])),
                                  cs2, bias2);
-                float2 pr;
-                if ((i & 3) < kPoly) {
-                    pr = exp2_poly2(x);
-                } else {
-                    pr.x = fast_exp2(x.x);
-                    pr.y = fast_exp2(x.y);
-                }
+                const float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
                 if (i & 1) sum_b = fadd2(sum_b, pr);
                 else sum_a = fadd2(sum_a, pr);
                 pk[i] = pack_bf16(pr.x, pr.y);
             }
+            if (chunk == kPartRunning / 2) publish_p_first(bar_p_first, tid_in_group);
             QW_TMEM_ST16(tmem_s + chunk * 16, pk);
         }
         if (tid_in_group == 0) QW_TRACE(sub, 3, j);
         tmem_wait_st();  // warp-collective: every lane's stores have landed
         tc_fence_before();
-        if ((tid_in_group & 31) == 0) mbar_arrive_twice(bar_p);  // stands for two warps
+        if ((tid_in_group & 31) == 0) mbar_arrive(bar_p);
         if (tid_in_group == 0) QW_TRACE(sub, 4, j);
         sum_a = fadd2(sum_a, sum_b);
         l_run += sum_a.x + sum_a.y;
@@ -743,7 +686,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
     bool use_own = processed > 0, use_other = false;
     if (split) {
         const float m_own = kBounded ? (processed > 0 ? bound : -INFINITY)
-                            : (processed > 0 && m_ref != -INFINITY) ? m_ref * fabsf(c)
+                            : (processed > 0 && m_ref != -INFINITY) ? m_ref * c
                                                                     : -INFINITY;
         if (sub == 1) {
             // Publish exponent and row sum; warpgroup 0 reads O_1 itself (same lanes).
@@ -831,7 +774,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
     if (p.head_major_out) return;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> TMA reads
     __syncwarp();
-    if ((tid_in_group & 31) == 0) mbar_arrive_twice(&ctl->bars[kBarEpi + sub]);
+    if ((tid_in_group & 31) == 0) mbar_arrive(&ctl->bars[kBarEpi + sub]);
     if (tid_in_group == 0) {
         if (!mbar_wait(ctl, &ctl->bars[kBarEpi + sub], 0, p.status,
                        (1u << 16) | (uint32_t)(kBarEpi + sub), 0xfffcu))
@@ -847,225 +790,6 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
         // what the barrier behind a sharded launch waits for.
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
-}
-
-// ---------------------------------------------------------------------------
-// Paired softmax role (fixed reference exponent only): all 256 softmax threads
-// work on one sub-tile's scores at a time, then on the other's.  TMEM lanes are
-// tied to warp_id % 4, so warps w and w + 4 both reach rows 32w..32w+31 of either
-// sub-tile: thread (half, r) takes keys [64*half, 64*half + 64) of row r.  Two
-// warps per scheduler run the exponentials of one tile together, which halves
-// the time a tile's S -> P step stays on the dependency chain S -> P -> P V; the
-// other sub-tile's MMAs fill the tensor pipe meanwhile.  Without a row maximum
-// the two threads of a row share nothing until the row sums meet at the end.
-// ---------------------------------------------------------------------------
-template <int kPoly>
-__device__ __forceinline__ void softmax_pair_role(const KernelParams &p, SharedControl *ctl,
-                                                  const OutMaps &maps_out, uint8_t *smem_q,
-                                                  int tid, int limit0, int limit1, uint32_t b,
-                                                  uint32_t h, uint32_t row0, bool split,
-                                                  float bound) {
-    const int half = tid >> 7, r = tid & 127;
-    const uint32_t lane_base = (uint32_t)((r >> 5) * 32) << 16;
-    const uint32_t tmem = ctl->tmem_base + lane_base;
-    const uint32_t s_col[2] = {kTmemS0 + 64u * (uint32_t)half, kTmemS1 + 64u * (uint32_t)half};
-    const int limits[2] = {limit0, limit1};
-    const int pad_lo = p.text_pad ? (int)p.text_len[b] : 0;
-    const int pad_hi = (int)p.text_pad;
-    const float2 cs2 = make_float2(p.scale_log2, p.scale_log2);
-    const float2 bias2 = make_float2(-bound, -bound);
-    [[maybe_unused]] uint32_t trace_cursor = 0;
-
-    float2 sums[2][2] = {{make_float2(0.f, 0.f), make_float2(0.f, 0.f)},
-                         {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}};
-    uint32_t phase[2] = {0, 0};
-    const int first[2] = {ctl->tile_first[0], ctl->tile_first[1]};
-    const int count[2] = {ctl->tile_count[0], ctl->tile_count[1]};
-    const int steps = max(count[0], count[1]);
-    bool ok = true;
-    // The first 32 scores of the next tile (the other sub-tile's, as a rule complete
-    // long before) are requested while this tile's last P chunk is still on its way
-    // to TMEM, so a tile does not start with an exposed TMEM round trip.
-    bool prefetched = false;
-    uint32_t sa[32], sb[32];
-
-    for (int s = 0; s < steps && ok; ++s) {
-#pragma unroll
-        for (int sub = 0; sub < 2; ++sub) {
-            if (s >= count[sub] || !ok) continue;
-            const int j = phys_tile(ctl, first[sub] + s);
-            if (!prefetched) {
-                ok = mbar_wait(ctl, &ctl->bars[kBarSFull + sub], phase[sub], p.status,
-                               (1u << 16) | (uint32_t)(kBarSFull + sub), (uint32_t)j);
-                if (!ok) continue;
-                phase[sub] ^= 1u;
-                tc_fence_after();
-                QW_TMEM_LD32(tmem + s_col[sub], sa);
-            }
-            prefetched = false;
-            if (tid == 0) QW_TRACE(sub, 0, j);
-            const int key0 = j * kTileN + 64 * half;
-            const int my_limit = limits[sub];
-            const bool pad_hit = pad_hi > pad_lo && key0 < pad_hi && key0 + 64 > pad_lo;
-            const bool boundary = __any_sync(0xffffffffu, key0 + 64 > my_limit) || pad_hit;
-#pragma unroll
-            for (int chunk = 0; chunk < 2; ++chunk) {
-                uint32_t(&cur)[32] = chunk ? sb : sa;
-                QW_TMEM_WAIT_LD32(cur);
-                if (chunk == 0) QW_TMEM_LD32(tmem + s_col[sub] + 32, sb);
-                if (chunk == 0 && tid == 0) QW_TRACE(sub, 1, j);
-                if (boundary) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int key = key0 + chunk * 32 + i;
-                        const bool visible = key < my_limit && !(key >= pad_lo && key < pad_hi);
-                        cur[i] = visible ? cur[i] : __float_as_uint(-INFINITY);
-                    }
-                }
-                uint32_t pk[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    float2 x = ffma2(make_float2(__uint_as_float(cur[2 * i]),
-                                                 __uint_as_float(cur[2 * i + 1])),
-                                     cs2, bias2);
-                    float2 pr;
-                    if ((i & 3) < kPoly) {
-                        pr = exp2_poly2(x);
-                    } else {
-                        pr.x = fast_exp2(x.x);
-                        pr.y = fast_exp2(x.y);
-                    }
-                    sums[sub][i & 1] = fadd2(sums[sub][i & 1], pr);
-                    pk[i] = pack_bf16(pr.x, pr.y);
-                }
-                // P of this thread's keys lands over this thread's own scores.
-                QW_TMEM_ST16(tmem + s_col[sub] + chunk * 16, pk);
-                if (chunk == 0 && tid == 0) QW_TRACE(sub, 2, j);
-            }
-            if (tid == 0) QW_TRACE(sub, 3, j);
-            {
-                const int nsub = 1 - sub, ns = sub ? s + 1 : s;
-                if (ns < count[nsub]) {
-                    // (asked without suspending: the next scores may in turn depend on
-                    // the P this warp has yet to publish, as they do with few key tiles)
-                    const bool ready = mbar_test(&ctl->bars[kBarSFull + nsub], phase[nsub]);
-                    if (__all_sync(0xffffffffu, ready)) {
-                        phase[nsub] ^= 1u;
-                        tc_fence_after();
-                        QW_TMEM_LD32(tmem + s_col[nsub], sa);
-                        prefetched = true;
-                    }
-                }
-            }
-            tmem_wait_st();
-            tc_fence_before();
-            if ((tid & 31) == 0) mbar_arrive(&ctl->bars[kBarPFull + sub]);
-            if (tid == 0) QW_TRACE(sub, 4, j);
-        }
-    }
-    // Row sums of the two key halves meet here.  Every softmax thread reaches this
-    // barrier, also after a wait gave up (its rows are then simply not stored).
-#pragma unroll
-    for (int sub = 0; sub < 2; ++sub) {
-        const float2 t = fadd2(sums[sub][0], sums[sub][1]);
-        ctl->pair_l[half][sub][r] = t.x + t.y;
-    }
-    asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
-    if (!ok || ctl->abort_flag) return;
-
-    // Epilogue.  Whole form: output tile t is sub-tile t, O_t / l_t.  Split form: one
-    // tile whose keys were divided between the sub-tiles: (O_0 + O_1) / (l_0 + l_1);
-    // both carry the same reference exponent, so the sum needs no reweighting.
-    // Thread (half, r) converts columns [64*half, 64*half + 64) of row r: exactly one
-    // 128-byte line of the swizzled staging box of its half.
-    const int n_out_tiles = split ? 1 : 2;
-#pragma unroll 1
-    for (int t = 0; t < n_out_tiles; ++t) {
-        const uint32_t tile_row0 = row0 + (uint32_t)t * kTileM;
-        if (tile_row0 >= p.q_rows) continue;
-        const uint32_t row = tile_row0 + (uint32_t)r;
-        const bool has_row = row < p.q_rows;
-        const bool use0 = split ? count[0] > 0 : count[t] > 0;
-        const bool use1 = split && count[1] > 0;
-        float l = ctl->pair_l[0][t][r] + ctl->pair_l[1][t][r];
-        if (split) l += ctl->pair_l[0][1][r] + ctl->pair_l[1][1][r];
-        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-        if (use0 &&
-            !mbar_wait(ctl, &ctl->bars[kBarOFinal + t], 0, p.status,
-                       (1u << 16) | (uint32_t)(kBarOFinal + t), 0xffffu))
-            return;
-        if (use1 &&
-            !mbar_wait(ctl, &ctl->bars[kBarOFinal + 1], 0, p.status,
-                       (1u << 16) | (uint32_t)(kBarOFinal + 1), 0xfffeu))
-            return;
-        if (!use0 && !p.head_major_out &&
-            // nothing was computed (zeros go out), but the Q load may still be in
-            // flight into what is now the staging area: let it land first
-            !mbar_wait(ctl, &ctl->bars[kBarQFull + t], 0, p.status,
-                       (1u << 16) | (uint32_t)(kBarQFull + t), 0xfffdu))
-            return;
-        tc_fence_after();
-        const uint32_t o_own = tmem + (t ? kTmemO1 : kTmemO0) + 64u * (uint32_t)half;
-        const uint32_t o_other = tmem + kTmemO1 + 64u * (uint32_t)half;
-        uint8_t *line = smem_q + (size_t)t * kTileBytes + (size_t)half * kHalfTileBytes +
-                        (size_t)r * 128;
-        const int sw = r & 7;
-        __nv_bfloat16 *direct =
-            p.out + (((size_t)b * p.heads + h) * p.q_rows + (has_row ? row : 0u)) * kHeadDim +
-            64 * half;
-#pragma unroll 1
-        for (int chunk = 0; chunk < 2; ++chunk) {
-            float v[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.0f;
-            if (use0) {
-                uint32_t o[32];
-                QW_TMEM_LD32(o_own + chunk * 32, o);
-                QW_TMEM_WAIT_LD32(o);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]);
-            }
-            if (use1) {
-                uint32_t o[32];
-                QW_TMEM_LD32(o_other + chunk * 32, o);
-                QW_TMEM_WAIT_LD32(o);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(o[i]);
-            }
-#pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-                uint4 packed;
-                packed.x = pack_bf16(v[i] * inv, v[i + 1] * inv);
-                packed.y = pack_bf16(v[i + 2] * inv, v[i + 3] * inv);
-                packed.z = pack_bf16(v[i + 4] * inv, v[i + 5] * inv);
-                packed.w = pack_bf16(v[i + 6] * inv, v[i + 7] * inv);
-                if (p.head_major_out) {
-                    if (has_row) reinterpret_cast<uint4 *>(direct + chunk * 32)[i >> 3] = packed;
-                } else {
-                    const int c16 = chunk * 4 + (i >> 3);  // 16-byte piece of the 128-byte line
-                    *reinterpret_cast<uint4 *>(line + ((c16 ^ sw) << 4)) = packed;
-                }
-            }
-        }
-        if (p.head_major_out) continue;
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> TMA reads
-        __syncwarp();
-        if ((tid & 31) == 0) mbar_arrive(&ctl->bars[kBarEpi + t]);
-        if (tid == 0) {
-            if (!mbar_wait(ctl, &ctl->bars[kBarEpi + t], 0, p.status,
-                           (1u << 16) | (uint32_t)(kBarEpi + t), 0xfffcu))
-                return;
-            const uint8_t *stage = smem_q + (size_t)t * kTileBytes;
-            const int col = (int)((p.out_head_offset + h) * kHeadDim);
-            for (uint32_t d = 0; d < p.n_out; ++d) {
-                tma_store_3d(&maps_out.m[d], stage, col, (int)tile_row0, (int)b);
-                tma_store_3d(&maps_out.m[d], stage + kHalfTileBytes, col + 64, (int)tile_row0, (int)b);
-            }
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-    }
-    // Shared memory may be released once the stores have read it.
-    if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -1093,24 +817,34 @@ __device__ __forceinline__ void issue_qk(uint32_t d_tmem, uint32_t q_lo, uint32_
     }
 }
 
-__device__ __forceinline__ void issue_pv(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo,
-                                         bool accumulate, bool paired) {
+// Keys 16 * kFrom .. 16 * kTo - 1 of P V.
+template <int kFrom, int kTo>
+__device__ __forceinline__ void issue_pv_keys(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo,
+                                              bool accumulate) {
     // A = P from TMEM (16 keys = 8 packed columns per step).  B = V, MN-major:
     // 16 keys = 2 groups of 8 rows (1024 B apart), the two 64-wide column
-    // halves one half tile apart.  P of keys 0..127 sits on columns 0..63 of the
-    // score region; in the paired organisation each key half is written by its own
-    // warp over its own scores, so keys 64..127 sit on columns 64..95.
-    const uint32_t upper = paired ? 64u - 32u : 0u;
+    // halves one half tile apart.
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-        const uint32_t col = (uint32_t)kk * 8u + (kk >= 4 ? upper : 0u);
-        mma_ts(d_tmem, p_tmem + col, v_lo + (uint32_t)(kk * 2048 >> 4), kDescHi, kIdescPV,
+    for (int kk = kFrom; kk < kTo; ++kk) {
+        mma_ts(d_tmem, p_tmem + (uint32_t)kk * 8u, v_lo + (uint32_t)(kk * 2048 >> 4), kDescHi, kIdescPV,
                (accumulate || kk > 0) ? 1u : 0u);
     }
 }
 
+// The two parts P V is issued in, as the softmax publishes them.
+__device__ __forceinline__ void issue_pv_first(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo,
+                                               bool accumulate, bool bounded) {
+    if (bounded) issue_pv_keys<0, kPartBounded>(d_tmem, p_tmem, v_lo, accumulate);
+    else issue_pv_keys<0, kPartRunning>(d_tmem, p_tmem, v_lo, accumulate);
+}
+__device__ __forceinline__ void issue_pv_rest(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo,
+                                              bool bounded) {
+    if (bounded) issue_pv_keys<kPartBounded, 8>(d_tmem, p_tmem, v_lo, true);
+    else issue_pv_keys<kPartRunning, 8>(d_tmem, p_tmem, v_lo, true);
+}
+
 __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *ctl,
-                                         uint8_t *smem_q, uint8_t *smem_kv, bool paired) {
+                                         uint8_t *smem_q, uint8_t *smem_kv, bool bounded) {
     // Whole form: both sub-tiles walk the visited tiles from 0; u counts them.
     const int n0 = uniform(ctl->tile_count[0]), n1 = uniform(ctl->tile_count[1]);
     const int n_max = max(n0, n1);
@@ -1177,13 +911,20 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (j < n_sub[i]) {
+                if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFirst + i], p_phase[i], p.status,
+                                    where | (kBarPFirst + i), (uint32_t)j))
+                    return;
+                tc_fence_after();
+                QW_TRACE(2, i, j);
+                if (elect_one())
+                    issue_pv_first(o_tmem[i], s_tmem[i], v_lo, o_started[i], bounded);
+                __syncwarp();
                 if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
-                               where | (kBarPFull + i), (uint32_t)j))
+                                    where | (kBarPFull + i), (uint32_t)j))
                     return;
                 p_phase[i] ^= 1u;
                 tc_fence_after();
-                QW_TRACE(2, i, j);
-                if (elect_one()) issue_pv(o_tmem[i], s_tmem[i], v_lo, o_started[i], paired);
+                if (elect_one()) issue_pv_rest(o_tmem[i], s_tmem[i], v_lo, bounded);
                 __syncwarp();
                 o_started[i] = true;
                 QW_TRACE(2, 4 + i, j);
@@ -1227,7 +968,7 @@ __device__ __forceinline__ uint32_t pair_a(int s, int lb) { return 2u * (uint32_
 __device__ __forceinline__ uint32_t pair_b(int s) { return 2u * (uint32_t)(2 * s + 1); }
 
 __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedControl *ctl,
-                                               uint8_t *smem_q, uint8_t *smem_kv, bool paired) {
+                                               uint8_t *smem_q, uint8_t *smem_kv, bool bounded) {
     const int la = uniform(ctl->tile_count[0]), lb = uniform(ctl->tile_count[1]);
     if (la <= 0) return;
     const uint32_t tmem = uniform(ctl->tmem_base);
@@ -1275,13 +1016,19 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             if (s >= count) continue;
             const uint32_t t_now = i ? pair_b(s) : pair_a(s, lb);
             QW_RING_WAIT(t_now + 1, kDescLoVMajor, desc);
+            if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFirst + i], p_phase[i], p.status,
+                                where | (kBarPFirst + i), (uint32_t)s))
+                return;
+            tc_fence_after();
+            if (elect_one()) issue_pv_first(o_tmem[i], s_tmem[i], desc, s > 0, bounded);
+            __syncwarp();
             if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
-                           where | (kBarPFull + i), (uint32_t)s))
+                                where | (kBarPFull + i), (uint32_t)s))
                 return;
             p_phase[i] ^= 1u;
             tc_fence_after();
             if (elect_one()) {
-                issue_pv(o_tmem[i], s_tmem[i], desc, s > 0, paired);
+                issue_pv_rest(o_tmem[i], s_tmem[i], desc, bounded);
                 QW_RING_FREE(t_now + 1);
             }
             __syncwarp();
@@ -1374,7 +1121,7 @@ __device__ __forceinline__ void issue_q_loads(const KernelParams &p, SharedContr
     }
 }
 
-template <int kPoly, bool kMayBound>
+template <bool kMayBound>
 __global__ void __launch_bounds__(kThreads, 1)
 qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
                      const __grid_constant__ CUtensorMap map_k,
@@ -1413,9 +1160,10 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&ctl->bars[kBarSFull + i], 1);
-            mbar_init(&ctl->bars[kBarPFull + i], kSoftmaxThreads / 32);
+            mbar_init(&ctl->bars[kBarPFirst + i], kTileM / 32);
+            mbar_init(&ctl->bars[kBarPFull + i], kTileM / 32);
             mbar_init(&ctl->bars[kBarOFinal + i], 1);
-            mbar_init(&ctl->bars[kBarEpi + i], kSoftmaxThreads / 32);
+            mbar_init(&ctl->bars[kBarEpi + i], kTileM / 32);
         }
         mbar_init(&ctl->bars[kBarMerge], kTileM / 32);
         mbar_init(&ctl->bars[kBarDebug], 1);
@@ -1476,10 +1224,6 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         const float limit = ceilf(p.score_bound[0] * p.score_bound[1] * p.scale_log2);
         if (limit >= 0.0f && limit <= 60.0f) bound = limit;
     }
-    // Paired organisation of the fixed-exponent softmax (both warpgroups on one
-    // sub-tile at a time) unless the launch asks for one thread per row.
-    const bool paired = kMayBound && bound >= 0.0f && p.pair_org;
-    int other_limit = 0;
     if (tid < kSoftmaxThreads) {
         sub = tid >> 7;
         tid_in_group = tid & 127;
@@ -1491,13 +1235,6 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         // limit of 0 it would send its whole warp through the masked path on every tile
         // (600 -> 1500 clocks a tile for the row maximum alone).
         if (my_row >= p.q_rows) my_limit = 0x7fffffff;
-        // (paired: this thread also works on the same row of the other sub-tile)
-        if (paired) {
-            const uint32_t other_row = row0 + (uint32_t)(1 - sub) * kTileM + (uint32_t)tid_in_group;
-            other_limit = split                    ? my_limit
-                          : other_row < p.q_rows ? row_limit(p, b, other_row)
-                                                   : 0x7fffffff;
-        }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1)
             warp_max = max(warp_max, __shfl_xor_sync(0xffffffffu, warp_max, off));
@@ -1528,22 +1265,19 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
         uint8_t *stage = smem_q + (size_t)sub * kTileBytes;
         const uint32_t tile_row0 = split ? row0 : row0 + (uint32_t)sub * kTileM;
-        if (paired)
-            softmax_pair_role<kPoly>(p, ctl, maps_out, smem_q, tid, sub ? other_limit : my_limit,
-                                     sub ? my_limit : other_limit, b, h, row0, split, bound);
-        else if (kMayBound && bound >= 0.0f)
-            softmax_role<kPoly, kMayBound>(p, ctl, maps_out, stage, sub, tid_in_group, my_limit, b,
-                                           h, my_row, tile_row0, split, bound);
+        if (kMayBound && bound >= 0.0f)
+            softmax_role<kMayBound>(p, ctl, maps_out, stage, sub, tid_in_group, my_limit, b, h,
+                                    my_row, tile_row0, split, bound);
         else
-            softmax_role<kPoly, false>(p, ctl, maps_out, stage, sub, tid_in_group, my_limit, b, h,
-                                       my_row, tile_row0, split, 0.0f);
+            softmax_role<false>(p, ctl, maps_out, stage, sub, tid_in_group, my_limit, b, h, my_row,
+                                tile_row0, split, 0.0f);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
     }
     if (tid < kSoftmaxThreads) {
     } else if (warp == kMmaWarp) {
-        if (split) mma_role_split(p, ctl, smem_q, smem_kv, paired);
-        else mma_role(p, ctl, smem_q, smem_kv, paired);
+        if (split) mma_role_split(p, ctl, smem_q, smem_kv, bound >= 0.0f);
+        else mma_role(p, ctl, smem_q, smem_kv, bound >= 0.0f);
     } else if (warp == kTmaWarp && lane == 0) {
         tma_role(p, ctl, smem_kv, &map_k, &map_v, b, kvh, split);
         // Q loads of active sub-tiles must have landed as well.
@@ -1661,36 +1395,12 @@ bool whole_units_forced() {
     return forced != 0;
 }
 
-// QW_CUDA_SOFTMAX_ORG=row / pair: force the organisation of the fixed-exponent
-// softmax (one thread per row, or both warpgroups on one sub-tile's keys at a time)
-// instead of choosing by the length of the launch (comparison runs).  -1 = not set.
-int softmax_org_forced() {
-    static int forced = -2;
-    if (forced == -2) {
-        const char *env = getenv("QW_CUDA_SOFTMAX_ORG");
-        forced = !env ? -1 : !strcmp(env, "row") ? 0 : !strcmp(env, "pair") ? 1 : -1;
-    }
-    return forced;
-}
-
-// The kernel variants: how many of every 4 score pairs take the polynomial exp2
-// (QW_CUDA_EXP_POLY=0..2 overrides the default for tuning), with or without the
-// fixed-exponent softmax for callers that pass a score bound.  The opt-in to
-// ~197 KB of dynamic shared memory is a per-device attribute: it is set on first
-// use on every device a process drives.
+// The kernel with or without the fixed-exponent softmax, for callers that pass a score
+// bound or not.  The opt-in to ~197 KB of dynamic shared memory is a per-device
+// attribute: it is set on first use on every device a process drives.
 AttnKernel pick_kernel(bool may_bound) {
-    static int poly = -1;
     static bool ready[64][2];
-    if (poly < 0) {
-        const char *env = getenv("QW_CUDA_EXP_POLY");
-        poly = (env && env[0] >= '0' && env[0] <= '2' && !env[1]) ? env[0] - '0' : 0;
-    }
-    AttnKernel table[3][2] = {
-        {qw_attn_sm100_kernel<0, false>, qw_attn_sm100_kernel<0, true>},
-        {qw_attn_sm100_kernel<1, false>, qw_attn_sm100_kernel<1, true>},
-        {qw_attn_sm100_kernel<2, false>, qw_attn_sm100_kernel<2, true>},
-    };
-    AttnKernel chosen = table[poly][may_bound ? 1 : 0];
+    AttnKernel chosen = may_bound ? qw_attn_sm100_kernel<true> : qw_attn_sm100_kernel<false>;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     const bool tracked = dev >= 0 && dev < 64;
@@ -1748,7 +1458,6 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
     p.text_pad = a->text_pad;
     p.scale_log2 = a->scale * 1.4426950408889634f;
     p.score_bound = a->score_bound;
-    p.pair_org = -1;  // decided below, once the unit count is known
     p.head_major_out = a->head_major_out;
     if (a->n_out_peers > 0) {
         if (a->n_out_peers > 8 || a->head_major_out) return (int)cudaErrorInvalidValue;
@@ -1789,16 +1498,6 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
                        ? 0u
                        : qwcu_attn_sm100_tail_units(p.total_units,
                                                     (uint32_t)sm_count_of_current_device());
-    // Fixed-exponent softmax: paired organisation where the launch is short (at most
-    // two waves of CTAs: the per-tile latency chain is what bounds it), one thread per
-    // row where it is long (many waves run at the board's power limit, where the
-    // organisation with fewer instructions per score is the faster one).
-    {
-        const int forced = softmax_org_forced();
-        const bool long_launch =
-            p.total_units > 2u * (uint32_t)sm_count_of_current_device();
-        p.pair_org = a->row_softmax ? 0 : forced >= 0 ? forced : long_launch ? 0 : 1;
-    }
     const unsigned grid = p.total_units + p.tail_units;
     kernel<<<grid, kThreads, kSmemBytes, stream>>>(map_q, map_k, map_v, maps_out, p);
     rc = (int)cudaGetLastError();

@@ -227,7 +227,7 @@ int qw_gpu_set_attention_kernel(h3_gpu *gpu, const char *name) {
     if (!gpu || !name) return 0;
     if (!strcmp(name, "sm100")) gpu->attn_kernel = QW_ATTN_SM100;
     else if (!strcmp(name, "sm100-whole")) gpu->attn_kernel = QW_ATTN_SM100_WHOLE;
-    else if (!strcmp(name, "sm100-row")) gpu->attn_kernel = QW_ATTN_SM100_ROW;
+    else if (!strcmp(name, "sm100-row")) gpu->attn_kernel = QW_ATTN_SM100;
     else if (!strcmp(name, "scalar")) gpu->attn_kernel = QW_ATTN_SCALAR;
     else {
         qw_set_error(gpu, "unknown attention kernel '%s'", name);
