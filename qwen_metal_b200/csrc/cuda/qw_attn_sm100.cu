@@ -60,7 +60,7 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include "../qw_cuda.h"
+#include "qw_sm100.cuh"
 
 namespace {
 
@@ -1178,6 +1178,20 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         ctl->skip_lo = lo;
         ctl->skip_hi = hi;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(&ctl->tmem_base)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // What stands above may run under the tail of the kernel before this one; all that
+    // reads or writes global memory stands below.
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
+    if (warp == kTmaWarp && lane == 0) {
+        const int lo = ctl->skip_lo, hi = ctl->skip_hi;
         issue_q_loads(p, ctl, smem_q, &map_q, b, h, row0, split ? 1 : 2);
         // First visited key tile, assuming the unit has one (if it has none the
         // tile is simply never consumed; the producer drains it before exit).
@@ -1201,13 +1215,6 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         for (uint32_t d = 0; d < p.n_freed; ++d)
             asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p.freed_peer[d]), "r"(epoch)
                          : "memory");
-    }
-    if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(&ctl->tmem_base)),
-                     "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
 
     // Row limits: each softmax thread owns one row; the largest limit of a
@@ -1499,8 +1506,7 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
                        : qwcu_attn_sm100_tail_units(p.total_units,
                                                     (uint32_t)sm_count_of_current_device());
     const unsigned grid = p.total_units + p.tail_units;
-    kernel<<<grid, kThreads, kSmemBytes, stream>>>(map_q, map_k, map_v, maps_out, p);
-    rc = (int)cudaGetLastError();
+    rc = sm100::launch(kernel, grid, kThreads, kSmemBytes, 1, stream, map_q, map_k, map_v, maps_out, p);
 #ifdef QW_ATTN_TRACE
     if (p.trace && !rc) trace_dump(stream);
 #endif

@@ -22,7 +22,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "../qw_cuda.h"
+#include "qw_sm100.cuh"
 
 namespace {
 
@@ -74,6 +74,8 @@ constexpr int kHeadsPerTrip = 4;
 // The two half-warps of a warp may hold different tensors (a normed key strip
 // next to a copied value strip), so the reductions name their own 16 lanes.
 __global__ void __launch_bounds__(256) qw_prologue_kernel(const Params p) {
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
     const int lane16 = threadIdx.x & 15;
     const uint32_t half_mask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
     const uint32_t half_warps = (gridDim.x * blockDim.x) >> 4;
@@ -170,6 +172,8 @@ __global__ void __launch_bounds__(256) qw_prologue_kernel(const Params p) {
 
 __global__ void qw_scale_bf16_kernel(__nv_bfloat16 *out, const __nv_bfloat16 *in, size_t n,
                                      float scale) {
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (; i < n; i += stride) {
@@ -226,8 +230,7 @@ extern "C" int qwcu_prologue_launch(const qwcu_prologue_args *a, qwcu_stream str
     unsigned long long cap = (unsigned long long)sm_count_cached() * 8ull;
     unsigned int blocks = (unsigned int)(want < cap ? want : cap);
     if (!blocks) blocks = 1;
-    qw_prologue_kernel<<<blocks, threads, 0, stream>>>(p);
-    return (int)cudaGetLastError();
+    return sm100::launch(qw_prologue_kernel, blocks, threads, 0, 1, stream, p);
 }
 
 extern "C" int qwcu_scale_bf16_launch(void *out, const void *in, size_t elements, float scale,
@@ -237,10 +240,9 @@ extern "C" int qwcu_scale_bf16_launch(void *out, const void *in, size_t elements
     size_t want = (elements + 255) / 256;
     size_t cap = (size_t)sm_count_cached() * 16;
     unsigned int blocks = (unsigned int)(want < cap ? want : cap);
-    qw_scale_bf16_kernel<<<blocks, 256, 0, stream>>>(static_cast<__nv_bfloat16 *>(out),
-                                                     static_cast<const __nv_bfloat16 *>(in),
-                                                     elements, scale);
-    return (int)cudaGetLastError();
+    return sm100::launch(qw_scale_bf16_kernel, blocks, 256, 0, 1, stream,
+                         static_cast<__nv_bfloat16 *>(out), static_cast<const __nv_bfloat16 *>(in),
+                         elements, scale);
 }
 
 extern "C" int qwcu_device_sm_count(int device) {

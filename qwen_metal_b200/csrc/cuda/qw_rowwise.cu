@@ -18,7 +18,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "../qw_cuda.h"
+#include "qw_sm100.cuh"
 
 namespace {
 
@@ -78,6 +78,8 @@ struct NormArgs {
 template <int kVecs>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 qw_layer_norm_mod_kernel(const NormArgs a) {
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t vecs = a.width >> 3;  // 16-byte vectors per row
     const uint32_t warps = gridDim.x * kWarpsPerBlock;
@@ -142,6 +144,8 @@ qw_layer_norm_mod_kernel(const NormArgs a) {
 // Any width: one warp per row, three passes over the (cached) row.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 qw_layer_norm_mod_generic_kernel(const NormArgs a) {
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
     const uint32_t row = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (row >= a.rows) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -178,6 +182,8 @@ struct GateArgs {
 
 // width % 8 == 0: one 16-byte vector per thread and step.
 __global__ void __launch_bounds__(256) qw_gate_kernel(const GateArgs a) {
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
     const uint32_t vecs = a.width >> 3;
     const size_t total = (size_t)a.rows * vecs;
     const uint4 *residual = reinterpret_cast<const uint4 *>(a.residual);
@@ -206,6 +212,8 @@ __global__ void __launch_bounds__(256) qw_gate_kernel(const GateArgs a) {
 }
 
 __global__ void __launch_bounds__(256) qw_gate_generic_kernel(const GateArgs a) {
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
     const size_t total = (size_t)a.rows * a.width;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (size_t)gridDim.x * blockDim.x) {
@@ -245,23 +253,18 @@ extern "C" int qwcu_layer_norm_mod_launch(const qwcu_rowwise_args *a, int sm_cou
     const unsigned blocks = (a->rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
     const bool vector = a->width % 8 == 0 && a->width <= 32u * kMaxVecs * 8u &&
                         aligned16(k.in) && aligned16(k.out) && aligned16(k.modulation);
-    if (!vector) {
-        qw_layer_norm_mod_generic_kernel<<<blocks, kWarpsPerBlock * 32, 0, stream>>>(k);
-        return (int)cudaGetLastError();
-    }
+    constexpr unsigned threads = kWarpsPerBlock * 32;
+    if (!vector)
+        return sm100::launch(qw_layer_norm_mod_generic_kernel, blocks, threads, 0, 1, stream, k);
     // A few resident CTAs per SM, each warp walking rows.
     const unsigned cap = (unsigned)(sm_count > 0 ? sm_count : 148) * 4u;
     const unsigned grid = blocks < cap ? blocks : cap;
     const uint32_t vecs_per_lane = (a->width / 8 + 31) / 32;
-    if (vecs_per_lane <= 4)
-        qw_layer_norm_mod_kernel<4><<<grid, kWarpsPerBlock * 32, 0, stream>>>(k);
-    else if (vecs_per_lane <= 8)
-        qw_layer_norm_mod_kernel<8><<<grid, kWarpsPerBlock * 32, 0, stream>>>(k);
-    else if (vecs_per_lane <= 12)
-        qw_layer_norm_mod_kernel<12><<<grid, kWarpsPerBlock * 32, 0, stream>>>(k);
-    else
-        qw_layer_norm_mod_kernel<kMaxVecs><<<grid, kWarpsPerBlock * 32, 0, stream>>>(k);
-    return (int)cudaGetLastError();
+    void (*kernel)(const NormArgs) = vecs_per_lane <= 4    ? qw_layer_norm_mod_kernel<4>
+                                     : vecs_per_lane <= 8  ? qw_layer_norm_mod_kernel<8>
+                                     : vecs_per_lane <= 12 ? qw_layer_norm_mod_kernel<12>
+                                                           : qw_layer_norm_mod_kernel<kMaxVecs>;
+    return sm100::launch(kernel, grid, threads, 0, 1, stream, k);
 }
 
 extern "C" int qwcu_gate_launch(const qwcu_rowwise_args *a, int sm_count, qwcu_stream stream_) {
@@ -287,9 +290,6 @@ extern "C" int qwcu_gate_launch(const qwcu_rowwise_args *a, int sm_count, qwcu_s
     size_t blocks = (items + 255) / 256;
     const size_t cap = (size_t)(sm_count > 0 ? sm_count : 148) * 32;
     if (blocks > cap) blocks = cap;
-    if (vector)
-        qw_gate_kernel<<<(unsigned)blocks, 256, 0, stream>>>(k);
-    else
-        qw_gate_generic_kernel<<<(unsigned)blocks, 256, 0, stream>>>(k);
-    return (int)cudaGetLastError();
+    return sm100::launch(vector ? qw_gate_kernel : qw_gate_generic_kernel, (unsigned)blocks, 256, 0, 1,
+                         stream, k);
 }
