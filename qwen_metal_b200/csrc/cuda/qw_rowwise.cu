@@ -72,24 +72,45 @@ struct NormArgs {
     uint32_t *status;
 };
 
-// width % 8 == 0 and width <= 32 * kVecs * 8.  A warp walks rows (stride = warps
-// in the grid); the grid holds a few resident CTAs per SM, so no time goes into
-// launching a CTA per handful of rows.
-template <int kVecs>
+// Sum over the kRowWarps warps that share a row (slot: one per reduction, so that the
+// second needs no barrier against the first; a CTA of several warps per row has one row
+// and walks no further).
+template <int kRowWarps>
+__device__ __forceinline__ float row_sum(float v, float (&part)[kWarpsPerBlock]) {
+    v = warp_sum(v);
+    if constexpr (kRowWarps == 1) return v;
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kRowWarps; ++i) v += part[i];
+    return v;
+}
+
+// width % 8 == 0 and width <= 32 * kRowWarps * kVecs * 8.
+// kRowWarps == 1: a warp walks rows (stride = warps in the grid); the grid holds a few
+// resident CTAs per SM, so no time goes into launching a CTA per handful of rows.
+// kRowWarps == kWarpsPerBlock: a CTA per row, for so few rows that a warp of the first
+// form would have one row at most: its time is then the latency of one row, and four
+// warps get through it sooner (320 rows of 3072: a 256^2 chain of four layers 340 -> 317 us,
+// 1152 rows: 512^2 523 -> 509 us).
+template <int kVecs, int kRowWarps>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 qw_layer_norm_mod_kernel(const NormArgs a) {
     sm100::grid_launch_dependents();
     sm100::grid_wait();
-    const uint32_t lane = threadIdx.x & 31u;
+    __shared__ float part[2][kWarpsPerBlock];
+    constexpr uint32_t kLanes = 32u * kRowWarps, kRowsPerBlock = kWarpsPerBlock / kRowWarps;
+    const uint32_t lane = threadIdx.x % kLanes;
     const uint32_t vecs = a.width >> 3;  // 16-byte vectors per row
-    const uint32_t warps = gridDim.x * kWarpsPerBlock;
-    for (uint32_t row = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); row < a.rows;
-         row += warps) {
+    const uint32_t stride = gridDim.x * kRowsPerBlock;
+    for (uint32_t row = blockIdx.x * kRowsPerBlock + threadIdx.x / kLanes; row < a.rows;
+         row += stride) {
         const uint4 *src = reinterpret_cast<const uint4 *>(a.in + (size_t)row * a.width);
         uint4 x[kVecs];
 #pragma unroll
         for (int i = 0; i < kVecs; ++i) {
-            const uint32_t v = lane + 32u * i;
+            const uint32_t v = lane + kLanes * i;
             x[i] = v < vecs ? __ldcs(src + v) : make_uint4(0, 0, 0, 0);
         }
         const uint32_t map = checked_map(a.row_map, row, a.maps, a.status);
@@ -103,11 +124,11 @@ qw_layer_norm_mod_kernel(const NormArgs a) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) sum += bf16_lo(w[k]) + bf16_hi(w[k]);
         }
-        const float mean = warp_sum(sum) / (float)a.width;
+        const float mean = row_sum<kRowWarps>(sum, part[0]) / (float)a.width;
         float square = 0.0f;
 #pragma unroll
         for (int i = 0; i < kVecs; ++i) {
-            if (lane + 32u * i < vecs) {  // padding vectors hold zeros, not (0 - mean)
+            if (lane + kLanes * i < vecs) {  // padding vectors hold zeros, not (0 - mean)
                 const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -117,12 +138,12 @@ qw_layer_norm_mod_kernel(const NormArgs a) {
                 }
             }
         }
-        const float inverse = rsqrtf(warp_sum(square) / (float)a.width + a.epsilon);
+        const float inverse = rsqrtf(row_sum<kRowWarps>(square, part[1]) / (float)a.width + a.epsilon);
 
         uint4 *dst = reinterpret_cast<uint4 *>(a.out + (size_t)row * a.width);
 #pragma unroll
         for (int i = 0; i < kVecs; ++i) {
-            const uint32_t v = lane + 32u * i;
+            const uint32_t v = lane + kLanes * i;
             if (v < vecs) {
                 const uint4 s = __ldg(scale + v);
                 const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
@@ -256,14 +277,21 @@ extern "C" int qwcu_layer_norm_mod_launch(const qwcu_rowwise_args *a, int sm_cou
     constexpr unsigned threads = kWarpsPerBlock * 32;
     if (!vector)
         return sm100::launch(qw_layer_norm_mod_generic_kernel, blocks, threads, 0, 1, stream, k);
-    // A few resident CTAs per SM, each warp walking rows.
+    // A few resident CTAs per SM, each warp walking rows; with fewer rows than those
+    // warps a CTA takes one row.
     const unsigned cap = (unsigned)(sm_count > 0 ? sm_count : 148) * 4u;
-    const unsigned grid = blocks < cap ? blocks : cap;
+    const bool few = blocks <= cap;
+    const unsigned grid = few ? a->rows : cap;
     const uint32_t vecs_per_lane = (a->width / 8 + 31) / 32;
-    void (*kernel)(const NormArgs) = vecs_per_lane <= 4    ? qw_layer_norm_mod_kernel<4>
-                                     : vecs_per_lane <= 8  ? qw_layer_norm_mod_kernel<8>
-                                     : vecs_per_lane <= 12 ? qw_layer_norm_mod_kernel<12>
-                                                           : qw_layer_norm_mod_kernel<kMaxVecs>;
+    void (*kernel)(const NormArgs);
+    if (vecs_per_lane <= 4)
+        kernel = few ? qw_layer_norm_mod_kernel<1, 4> : qw_layer_norm_mod_kernel<4, 1>;
+    else if (vecs_per_lane <= 8)
+        kernel = few ? qw_layer_norm_mod_kernel<2, 4> : qw_layer_norm_mod_kernel<8, 1>;
+    else if (vecs_per_lane <= 12)
+        kernel = few ? qw_layer_norm_mod_kernel<3, 4> : qw_layer_norm_mod_kernel<12, 1>;
+    else
+        kernel = few ? qw_layer_norm_mod_kernel<4, 4> : qw_layer_norm_mod_kernel<kMaxVecs, 1>;
     return sm100::launch(kernel, grid, threads, 0, 1, stream, k);
 }
 

@@ -162,3 +162,16 @@ def test_modulation_row_index_outside_the_tensor_is_reported(gpu):
                O.layer_norm_mod(x, mod, good, rows, width, slots, 1, 1e-6))
     for t in (xt, mt, rt, ot, small):
         gpu.free(t)
+
+
+@pytest.mark.parametrize("rows,width", [
+    (1, 8), (3, 1024), (5, 1032), (2, 2056), (7, 3080), (3, 4096),  # a CTA per row: the vectors' edges
+    (2368, 136), (2369, 136),  # the last row count of that form on 148 SMs, the first of the other
+])
+def test_norm_mod_forms_match_oracle(gpu, rows, width):
+    rng = np.random.default_rng(rows + width)
+    x = workloads.normal_bf16(rng, (rows, width))
+    mod = workloads.normal_bf16(rng, (2, 3, width))
+    row_map = rng.integers(0, 2, rows).astype(np.uint32)
+    got = run_norm(gpu, x, mod, row_map, rows, width, 3, 1)
+    check_norm(got, O.layer_norm_mod(x, mod, row_map, rows, width, 3, 1, 1e-6))
