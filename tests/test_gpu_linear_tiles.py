@@ -20,6 +20,7 @@ pytestmark = pytest.mark.gpu
     (300, 72, 11520, True),     # 90 pair tiles on 74 pairs: 16 of them as halves
     (384, 200, 12288, False),   # single CTAs of 128 x 256: one wave where pairs need two
     (4097, 64, 3072, False),    # several tiles per pair: both accumulators, both phases
+    (200, 1160, 520, True),     # W rows of 2320 bytes: prefetched in whole and partial pieces
 ])
 def test_every_tile_shape_matches_oracle(gpu, rows, k, n, bias):
     rng = np.random.default_rng(rows + k + n)
