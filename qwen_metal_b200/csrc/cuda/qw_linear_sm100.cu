@@ -44,7 +44,6 @@ constexpr int kStoreBytes = 32 * 128;  // a warp's staging box: 32 rows x 64 col
 constexpr int kMaxSmem = 227 * 1024;
 constexpr int kMaxStages = 8;
 constexpr int kMaxOutputs = 3;
-constexpr uint32_t kPrefetchBytes = 1024;  // of a W row, at a time into L2
 constexpr int kBand = 2048;  // rows of A whose tiles run side by side (L2 reuse of W)
 
 enum Barrier : int {
@@ -81,7 +80,6 @@ struct Params {
     uint32_t m_tiles, n_tiles;   // n_tiles over all outputs
     uint32_t band;               // M tiles that run side by side
     uint32_t whole, items;       // items [0, whole) are tiles, the rest half tiles (kN / 2 columns)
-    const uint8_t *w[kMaxOutputs];      // bf16 [n_each][k]
     const uint16_t *bias[kMaxOutputs];  // bf16 [n_each] or null
     uint32_t *status;
     // Optional fused epilogue for outputs 0 and 1 (q and k of the DiT block): per-head
@@ -218,20 +216,6 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
     }
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
-    // Weights are read from HBM 128 bytes of every row at a time, which few M tiles do not
-    // make up for by reuse: the first item's share is asked into L2 ahead of the ring,
-    // kPrefetchBytes of a row at a time, and under the tail of the kernel before this one
-    // (a prefetch changes nothing that anybody can see, so it need not wait for it).
-    // 512^2 layers 509 -> 501 us, 768^2 954 -> 946 us; longer ones indifferent.
-    if (warp >= 2 && first < p.items) {
-        const Item it = item_at<kN>(p, first);
-        const uint32_t t = threadIdx.x - 64, share = it.cols / kGroup;
-        const uint32_t row = it.col0 + rank * share + t % kRows, row_bytes = p.k * 2;
-        if (it.tm == 0 && t % kRows < share && row < p.n_each)
-            for (uint32_t at = t / kRows * kPrefetchBytes; at < row_bytes; at += 2 * kPrefetchBytes)
-                l2_prefetch(p.w[it.which] + (size_t)row * row_bytes + at,
-                            min(kPrefetchBytes, row_bytes - at));
-    }
     grid_launch_dependents();
     grid_wait();
 
@@ -499,7 +483,6 @@ extern "C" int qwcu_linear_sm100_launch(const qwcu_linear_args *a, int sm_count,
         if (((uintptr_t)a->w[i] | (uintptr_t)a->c[i]) & 15u) return (int)cudaErrorMisalignedAddress;
         if ((rc = make_map_2d(&maps.w[i], a->w[i], a->n, a->k, 64))) return rc;
         if ((rc = make_map_2d(&maps.c[i], a->c[i], a->m, a->n, 32))) return rc;
-        p.w[i] = static_cast<const uint8_t *>(a->w[i]);
         p.bias[i] = static_cast<const uint16_t *>(a->bias[i]);
     }
     p.m = a->m;

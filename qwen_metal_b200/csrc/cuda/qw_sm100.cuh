@@ -155,10 +155,6 @@ __device__ __forceinline__ void tma_store_wait_read() {
 __device__ __forceinline__ void tma_prefetch(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
-// Whole 16-byte pieces at a 16-byte boundary.
-__device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void fence_async_shared() {  // generic writes -> TMA reads
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
