@@ -8,8 +8,9 @@
 // Persistent CTAs.  Large problems run on CTA pairs (tcgen05 cta_group::2): a pair owns
 // a 256 (M) x 256 (N) tile, each CTA holds 128 rows of A and half of the W rows, so a
 // K step of 64 costs a CTA 32 KB of shared memory instead of 48 KB and the tensor
-// cores read each W row once per pair.  Problems too small to fill the pairs run on
-// single CTAs with 128-row tiles, 64 to 256 columns wide (choose() below).
+// cores read each W row once per pair.  Problems that do not fill the pairs take pairs of
+// 128 columns or, where the CTAs of one wave do what pairs need two for, single CTAs of
+// 128 (M) x 256 (N) (choose() below).
 //   warp 0     : TMA producer  (128B-swizzled boxes of 64 columns)
 //   warp 1     : MMA issuer    (of the pair's first CTA)
 //   warps 2..9 : epilogue      (TMEM -> registers -> bf16 -> a staging box of 32 rows x
@@ -399,12 +400,15 @@ struct Variant {
     int group, n, smem;
     // Measured nanoseconds of one K step of 64 on a tile, and of one on a half tile.  The
     // 256-column pair is bound by the tensor cores, the others by the 70 bytes a clock
-    // that L2 delivers to an SM (24 KB a step for 128 columns, 48 KB on a single CTA).
+    // that L2 delivers to an SM (24 KB a step for 128 columns, 48 KB on a single CTA).  A half
+    // tile moves what a 128-column pair does through a shorter ring: 12288 x 3072 columns at
+    // 128 rows 46.5 us as halves, 40.8 us as 128-column tiles, 4096 x 4096 at 64 rows 20.1 and
+    // 17.3 us, so halves are for a last wave behind whole tiles only.
     int step_ns, half_ns;
 };
 
 const Variant kVariants[] = {
-    {qw_linear_sm100_kernel<2, 256>, 2, 256, Config<2, 256>::kSmem, 250, 215},
+    {qw_linear_sm100_kernel<2, 256>, 2, 256, Config<2, 256>::kSmem, 250, 240},
     {qw_linear_sm100_kernel<2, 128>, 2, 128, Config<2, 128>::kSmem, 215, 0},
     {qw_linear_sm100_kernel<1, 256>, 1, 256, Config<1, 256>::kSmem, 360, 0},
 };
@@ -418,14 +422,14 @@ struct Choice {
 // The variant whose waves take the least time per K step.  The tiles of a last, partly
 // filled wave are cut in two along N when the halves still fit one wave (256-column
 // tiles of pairs only).
-bool choose(Choice *best, const qwcu_linear_args *a, uint32_t sms) {
+bool choose(Choice *best, uint32_t m, uint32_t n, uint32_t n_outputs, uint32_t sms) {
     uint64_t best_cost = 0;
     best->v = nullptr;
     for (int i = 0; i < kVariantCount; ++i) {
         const Variant *v = &kVariants[i];
         const uint64_t slots = sms / (uint32_t)v->group;
-        const uint64_t m_tiles = (a->m + kRows * v->group - 1) / (kRows * v->group);
-        const uint64_t per_output = (a->n + v->n - 1) / v->n, n_tiles = per_output * a->n_outputs;
+        const uint64_t m_tiles = (m + kRows * v->group - 1) / (kRows * v->group);
+        const uint64_t per_output = (n + v->n - 1) / v->n, n_tiles = per_output * n_outputs;
         const uint64_t tiles = m_tiles * n_tiles;
         if (tiles > 0x3fffffffull || !slots) continue;
         const uint64_t rest = tiles % slots;
@@ -454,7 +458,18 @@ bool kernel_ready(const Variant *v) {
     return true;
 }
 
+uint32_t usable_sms(int sm_count) { return (uint32_t)(sm_count > 1 ? sm_count : 148); }
+
 }  // namespace
+
+extern "C" int qwcu_linear_sm100_plan(uint32_t m, uint32_t n, uint32_t n_outputs, int sm_count,
+                                      qwcu_linear_plan *plan) {
+    Choice choice;
+    if (!m || !n || !n_outputs || !choose(&choice, m, n, n_outputs, usable_sms(sm_count)))
+        return (int)cudaErrorInvalidValue;
+    *plan = {(uint32_t)choice.v->group, (uint32_t)choice.v->n, choice.whole, choice.items};
+    return 0;
+}
 
 extern "C" int qwcu_linear_sm100_launch(const qwcu_linear_args *a, int sm_count,
                                         qwcu_stream stream_) {
@@ -466,9 +481,9 @@ extern "C" int qwcu_linear_sm100_launch(const qwcu_linear_args *a, int sm_count,
     if (fused && (a->n % 128 || !a->rope_cos || !a->rope_sin || !a->table_rows))
         return (int)cudaErrorInvalidValue;
     if (a->bound_out && !(a->norm_weight[0] && a->norm_weight[1])) return (int)cudaErrorInvalidValue;
-    const uint32_t sms = (uint32_t)(sm_count > 1 ? sm_count : 148);
+    const uint32_t sms = usable_sms(sm_count);
     Choice choice;
-    if (!choose(&choice, a, sms)) return (int)cudaErrorInvalidValue;
+    if (!choose(&choice, a->m, a->n, a->n_outputs, sms)) return (int)cudaErrorInvalidValue;
     const Variant *v = choice.v;
     if (!kernel_ready(v)) return (int)cudaGetLastError();
     Maps maps;

@@ -217,6 +217,13 @@ typedef struct {
 } qwcu_linear_args;
 
 int qwcu_linear_sm100_launch(const qwcu_linear_args *args, int sm_count, qwcu_stream stream);
+/* The tiles a launch of these sizes runs with on sm_count SMs (host-side arithmetic
+ * only): CTAs per tile, its columns, whole tiles, whole and half tiles together. */
+typedef struct {
+    uint32_t ctas, columns, whole, items;
+} qwcu_linear_plan;
+int qwcu_linear_sm100_plan(uint32_t m, uint32_t n, uint32_t n_outputs, int sm_count,
+                           qwcu_linear_plan *plan);
 
 /* Device properties needed by the host side. */
 int qwcu_device_sm_count(int device);

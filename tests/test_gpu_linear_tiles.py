@@ -2,12 +2,14 @@
 its tiles (first, last and ragged rows and columns, a K tail, several tiles per CTA
 pair, the half tiles of a partly filled last wave), against the CPU oracle on the rows
 around the tile borders.  Tolerance as for the GEMM elsewhere: fp32 sums in another
-order, one rounding to bf16."""
+order, one rounding to bf16.  linear_plans.py holds what each size is dispatched to on
+148 SMs; the tests fail where it is something else."""
 import numpy as np
 import pytest
 
+import linear_plans as P
 import oracle_lib as O
-from qwen_metal_b200 import workloads
+from qwen_metal_b200 import abi, workloads
 from test_gpu_linear import check_gemm, weights
 
 pytestmark = pytest.mark.gpu
@@ -17,12 +19,16 @@ pytestmark = pytest.mark.gpu
     (1, 8, 8, True),            # the smallest: one row, one 16-byte column group
     (257, 136, 264, True),      # 128-column pair tiles, one row and 8 columns over
     (513, 72, 5120, False),     # 256-column pair tiles, one wave
-    (300, 72, 11520, True),     # 90 pair tiles on 74 pairs: 16 of them as halves
+    (300, 72, 11520, True),     # single CTAs: one wave where pairs need a whole one and a half one
     (384, 200, 12288, False),   # single CTAs of 128 x 256: one wave where pairs need two
     (4097, 64, 3072, False),    # several tiles per pair: both accumulators, both phases
-    (200, 1160, 520, True),     # W rows of 2320 bytes: prefetched in whole and partial pieces
+    (200, 1160, 520, True),     # 128-column pair tiles, 18 K steps and 8 columns
+    (5000, 64, 384, True),      # 128-column pair tiles in one wave where 256 columns leave half a tile
+    (1100, 72, 5120, True),     # 256-column pair tiles, the last wave as halves
+    (1152, 64, 9216, False),    # the same behind two tiles per pair
 ])
 def test_every_tile_shape_matches_oracle(gpu, rows, k, n, bias):
+    P.check(gpu, rows, n, 1)
     rng = np.random.default_rng(rows + k + n)
     x, w = workloads.normal_bf16(rng, (rows, k)), weights(rng, n, k)
     b = workloads.normal_bf16(rng, (n,)) if bias else None
@@ -36,4 +42,44 @@ def test_every_tile_shape_matches_oracle(gpu, rows, k, n, bias):
     sample = np.array(sorted(r for r in edges if 0 <= r < rows), np.uint32)
     check_gemm(got[sample], O.linear(x, w, b, rows, k, n, sample)[sample], f"{rows}x{k}x{n}")
     for t in [xt, wt, ot] + ([bt] if bias else []):
+        gpu.free(t)
+
+
+@pytest.mark.parametrize("seq,dim", [
+    (200, 512),    # 128-column pair tiles: a head per tile
+    (300, 4096),   # single CTAs: two heads per tile, the second by the second warp group
+    (1152, 3072),  # pairs: two whole tiles on either accumulator, then halves of one head
+    (513, 2688),   # 21 heads: the last tile of every output holds one
+])
+def test_fused_epilogue_on_every_tile_shape(gpu, seq, dim):
+    """q/k/v with the norm and the rotation in the epilogue: the plain projection against
+    the oracle on a row sample, the fused one bit for bit against the oracle's norm and
+    rotation of the plain one's bf16 output, v equal to the plain one's."""
+    P.check(gpu, seq, dim, 3)
+    rng = np.random.default_rng(seq + dim)
+    lib, heads = gpu.lib, dim // 128
+    x = workloads.normal_bf16(rng, (seq, dim))
+    ws = [weights(rng, dim, dim) for _ in range(3)]
+    wq, wk = (workloads.normal_bf16(rng, (128,), 1.0, 0.1) for _ in range(2))
+    cos, sin = abi.rope_tables(seq - 144, 12, 12)
+    xt, wts = gpu.bf16(x), [gpu.bf16(w) for w in ws]
+    plain, fused = ([gpu.new_bf16(seq * dim) for _ in range(3)] for _ in range(2))
+    wqt, wkt, ct, st, bt = gpu.bf16(wq), gpu.bf16(wk), gpu.f32(cos), gpu.f32(sin), gpu.new_f32(2)
+    gpu.begin()
+    gpu.check(lib.qw_gpu_qkv_bf16(gpu.handle, *plain, xt, *wts, seq, dim), "qkv")
+    gpu.check(lib.qw_gpu_qkv_norm_rope_bf16(gpu.handle, *fused, xt, *wts, wqt, wkt, ct, st, bt, 1, seq,
+                                            dim, 1e-6), "qkv norm rope")
+    gpu.submit()
+    got = [gpu.read_bf16(t, seq * dim).reshape(seq, dim) for t in plain]
+    sample = np.array([0, 31, 32, 127, 128, seq // 2, seq - 1], np.uint32)
+    for name, g, w in zip("qkv", got, ws):
+        check_gemm(g[sample], O.linear(x, w, None, seq, dim, dim, sample)[sample], f"{name} {seq}x{dim}")
+    normed = [O.head_rms_norm(g.reshape(seq, heads, 128), w, seq, heads, 1e-6)
+              for g, w in zip(got, (wq, wk))]
+    want_q, want_k = O.qk_rope(*normed, cos, sin, seq, heads)
+    fq, fk, fv = (gpu.read_bf16(t, seq * dim).reshape(seq, heads, 128) for t in fused)
+    assert np.array_equal(fq, want_q.reshape(fq.shape)), float((fq != want_q.reshape(fq.shape)).mean())
+    assert np.array_equal(fk, want_k.reshape(fk.shape)), float((fk != want_k.reshape(fk.shape)).mean())
+    assert np.array_equal(fv.reshape(seq, dim), got[2])
+    for t in [xt, wqt, wkt, ct, st, bt] + wts + plain + fused:
         gpu.free(t)

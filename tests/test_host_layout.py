@@ -91,6 +91,26 @@ def test_split_tail_rule():
         assert tail in (0, units % sms) and 2 * tail <= sms + sms // 16
 
 
+def test_linear_plans():
+    """The GEMM's tiles (host arithmetic of the launcher): the sizes the GPU tests name,
+    and over random sizes that whole and half tiles cover the outputs exactly once, half
+    tiles only in a last wave that they fit."""
+    import linear_plans as P
+    lib = abi.load()
+    for size, want in P.PLANS.items():
+        assert P.plan_on(lib, *size).fields() == want, size
+    rng = np.random.default_rng(7)
+    for _ in range(3000):
+        m, outputs = int(np.exp(rng.uniform(0, 11))), int(rng.choice([1, 3]))
+        n = 8 * int(np.exp(rng.uniform(0, 8)))
+        p = P.plan_on(lib, m, n, outputs)
+        assert (p.ctas, p.columns) in ((2, 256), (2, 128), (1, 256))
+        tiles = -(-m // (128 * p.ctas)) * -(-n // p.columns) * outputs
+        halves, slots = p.items - p.whole, P.SMS // p.ctas
+        assert p.whole + halves // 2 == tiles and halves % 2 == 0
+        assert halves == 0 or (halves <= slots and p.whole % slots == 0 and p.columns == 256)
+
+
 def test_prefix_limits_random_layouts_and_mask_semantics():
     """Seeded random run layouts: the library's limits equal the oracle's bit for bit,
     and they mean what the reference's mask means (qwen_dit.m:1651-1665): a text row
