@@ -227,6 +227,11 @@ int qw_gpu_set_attention_kernel(h3_gpu *gpu, const char *name);
  * drained, TMEM freed) and h3_gpu_submit returns 0 with the place of the first
  * expiry.  (0, 0) restores normal operation. */
 int qw_gpu_debug_attention_waits(h3_gpu *gpu, long long wait_cycles, int withhold_from_tile);
+/* The same for the linear layers' kernel: K steps (>= 1, counted from a CTA's first; 0 =
+ * none) from which the first and the second CTA of a pair load nothing.  (0, 0, 0)
+ * restores normal operation. */
+int qw_gpu_debug_linear_waits(h3_gpu *gpu, long long wait_cycles, uint32_t withhold_first,
+                              uint32_t withhold_second);
 /* Launches enqueued by this context's ops since creation (own kernels only). */
 uint64_t qw_gpu_kernel_launches(const h3_gpu *gpu);
 

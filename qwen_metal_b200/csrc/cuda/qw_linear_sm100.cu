@@ -25,7 +25,8 @@
 // are reproduced, which makes the result the same as GEMM -> h3_gpu_head_rms_norm_bf16
 // -> qw_gpu_qk_rope_bf16 without the two extra passes over q and k.
 //
-// Every wait is bounded (status words, abort flag).
+// Every wait is bounded (status words, abort flag).  A CTA leaves nothing in flight, also
+// after a wait has run out: see the end of the kernel.
 
 #include <string.h>
 
@@ -59,8 +60,10 @@ struct __align__(16) Control {
     Mbar bars[kBarCount];
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
+    uint32_t issued[2];  // of the pair's CTAs: K steps loaded, kGaveUp when a wait ran out
     float norm_w[2][128];
 };
+constexpr uint32_t kGaveUp = 0x80000000u;
 
 template <int kGroup, int kN>
 struct Config {
@@ -91,6 +94,10 @@ struct Params {
     uint32_t table_rows;               // table row = output row % table_rows
     float epsilon;
     float *bound_out;  // optional: [0], [1] = bounds of the 2-norm of any q row, k row
+    // Bounded-wait exercise (tests only): budget in SM cycles, and the K step (counted over
+    // its items) from which a CTA of the pair loads nothing.
+    long long wait_cycles;
+    uint32_t withhold_from[2];
 };
 
 struct Maps {
@@ -192,7 +199,7 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
     const uint32_t rank = kGroup == 2 ? cluster_rank() : 0u;
     const uint32_t first = blockIdx.x / kGroup, step = gridDim.x / kGroup;
     const uint32_t k_steps = (p.k + kTileK - 1) / kTileK;
-    const Waiter wait = {&ctl->abort_flag, p.status, kWaitCycles};
+    const Waiter wait = {&ctl->abort_flag, p.status, p.wait_cycles};
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < C::kStages; ++i) {
@@ -220,45 +227,52 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
     grid_launch_dependents();
     grid_wait();
 
+    // This CTA's loads of K step ks of an item, the t-th step it loads: its rows of A and
+    // its share of the W rows.
+    const auto load_step = [&](const Item &it, uint32_t ks, uint32_t t) {
+        const uint32_t slot = t % C::kStages, share = it.cols / kGroup;  // (in boxes of 64)
+        const int a_row = (int)((it.tm * kGroup + rank) * kRows);
+        const int w_row = (int)(it.col0 + rank * share);
+        Mbar *bar = &ctl->bars[kBarFull + slot];
+        const uint32_t bar_at = kGroup == 2 ? map_to_rank(bar, 0) : smem_u32(bar);
+        uint8_t *dst = ring + slot * C::kStageBytes;
+        const int k0 = (int)(ks * kTileK);
+        if (elect_one()) {
+            if (rank == 0) mbar_expect_tx(bar, (kABytes + share * (kTileK * 2)) * kGroup);
+            tma_load_2d<kGroup>(dst, &maps.a, bar_at, k0, a_row);
+#pragma unroll
+            for (int box = 0; box < C::kBBytes / kBoxBytes; ++box)
+                if ((uint32_t)box * 64u < share)
+                    tma_load_2d<kGroup>(dst + kABytes + box * kBoxBytes, &maps.w[it.which], bar_at, k0,
+                                        w_row + box * 64);
+        }
+        __syncwarp();
+    };
+
     if (warp == 0) {
-        // ---- producer: this CTA's rows of A and its share of the W rows
+        // ---- producer
         uint32_t t = 0;
         bool ok = true;
         for (uint32_t i = first; i < p.items && ok; i += step) {
             const Item it = item_at<kN>(p, i);
-            const uint32_t share = it.cols / kGroup;  // W rows of this CTA, in boxes of 64
-            const uint32_t bytes = (kABytes + share * (kTileK * 2)) * kGroup;
-            const int a_row = (int)((it.tm * kGroup + rank) * kRows);
-            const int w_row = (int)(it.col0 + rank * share);
             for (uint32_t ks = 0; ks < k_steps; ++ks, ++t) {
                 const uint32_t slot = t % C::kStages, par = ((t / C::kStages) & 1u) ^ 1u;
-                ok = mbar_wait_warp(wait, &ctl->bars[kBarEmpty + slot], par, (3u << 16) | slot, i);
+                ok = t < p.withhold_from[rank] &&
+                     mbar_wait_warp(wait, &ctl->bars[kBarEmpty + slot], par, (3u << 16) | slot, i);
                 if (!ok) break;
-                Mbar *bar = &ctl->bars[kBarFull + slot];
-                const uint32_t bar_at = kGroup == 2 ? map_to_rank(bar, 0) : smem_u32(bar);
-                uint8_t *dst = ring + slot * C::kStageBytes;
-                const int k0 = (int)(ks * kTileK);
-                if (elect_one()) {
-                    if (rank == 0) mbar_expect_tx(bar, bytes);
-                    tma_load_2d<kGroup>(dst, &maps.a, bar_at, k0, a_row);
-#pragma unroll
-                    for (int box = 0; box < C::kBBytes / kBoxBytes; ++box)
-                        if ((uint32_t)box * 64u < share)
-                            tma_load_2d<kGroup>(dst + kABytes + box * kBoxBytes, &maps.w[it.which],
-                                                bar_at, k0, w_row + box * 64);
-                }
-                __syncwarp();
+                load_step(it, ks, t);
             }
         }
-        // In normal operation every load has been consumed before the last accumulator
-        // is complete; after an expired wait the ones in flight still have to land.
-        if (!ok && rank == 0) {
-            const uint32_t from = t > (uint32_t)C::kStages ? t - C::kStages : 0;
-            for (uint32_t u = from; u < t; ++u) {
-                const long long start = clock64();
-                while (!mbar_try(&ctl->bars[kBarFull + u % C::kStages], (u / C::kStages) & 1u))
-                    if (clock64() - start > kWaitCycles) break;
-            }
+        // Wait until the last steps are consumed: then their loads (the peer's too) have
+        // landed and the commits that report here, those of the pair's first CTA among
+        // them, have arrived.
+        for (uint32_t u = t > (uint32_t)C::kStages ? t - C::kStages : 0; u < t && ok; ++u)
+            ok = mbar_wait_warp(wait, &ctl->bars[kBarEmpty + u % C::kStages], (u / C::kStages) & 1u,
+                                (3u << 16) | (u % C::kStages), p.items);
+        if (lane < kGroup) {
+            const uint32_t word = ok ? t : t | kGaveUp;
+            if constexpr (kGroup == 2) st_at(map_to_rank(&ctl->issued[rank], (uint32_t)lane), word);
+            else ctl->issued[0] = word;
         }
     } else if (warp == 1 && rank == 0) {
         // ---- MMA issuer (for both CTAs of a pair)
@@ -296,6 +310,9 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
             }
             if (!ok) break;
         }
+        // Nothing that was issued runs on into the release of TMEM and shared memory (all of
+        // it is done already, unless a wait has run out).
+        if (t) mbar_drain(&ctl->bars[kBarEmpty + (t - 1) % C::kStages], ((t - 1) / C::kStages) & 1u, p.wait_cycles);
     } else if (warp >= 2) {
         // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) ..., thread = one row; the
         // warps of the second group take the second half of a wide tile's columns
@@ -383,14 +400,31 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
         }
         if (lane == 0) tma_store_wait_read<0>();
     }
-    tc_fence_before();
-    __syncwarp();
-    if constexpr (kGroup == 2) cluster_sync();
-    else __syncthreads();
-    if (warp == 1) {
+    const auto sync_all = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if constexpr (kGroup == 2) cluster_sync();
+        else __syncthreads();
         tc_fence_after();
-        tmem_dealloc<kGroup>(tmem, C::kTmemCols);
+    };
+    sync_all();
+    if ((ctl->issued[0] | (kGroup == 2 ? ctl->issued[1] : 0u)) & kGaveUp) {
+        // A wait has run out somewhere, and loads may be in flight.  Only the first CTA's
+        // barriers count them, both CTAs' bytes of a step together, so the CTA that got less
+        // far loads the steps it is behind (their slots are free: the other one has seen
+        // them consumed) and the first CTA waits for the last step of every slot.
+        const uint32_t t0 = ctl->issued[0] & ~kGaveUp;
+        const uint32_t t1 = kGroup == 2 ? ctl->issued[1] & ~kGaveUp : t0, most = max(t0, t1);
+        if (warp == 0) {
+            for (uint32_t t = rank ? t1 : t0; t < most; ++t)
+                load_step(item_at<kN>(p, first + t / k_steps * step), t % k_steps, t);
+            if (rank == 0)
+                for (uint32_t t = most > (uint32_t)C::kStages ? most - C::kStages : 0; t < most; ++t)
+                    mbar_drain(&ctl->bars[kBarFull + t % C::kStages], (t / C::kStages) & 1u, p.wait_cycles);
+        }
+        sync_all();
     }
+    if (warp == 1) tmem_dealloc<kGroup>(tmem, C::kTmemCols);
 }
 
 typedef void (*LinearKernel)(const Maps, const Params);
@@ -517,6 +551,8 @@ extern "C" int qwcu_linear_sm100_launch(const qwcu_linear_args *a, int sm_count,
     p.table_rows = a->table_rows ? a->table_rows : 1;
     p.epsilon = a->epsilon;
     p.bound_out = a->bound_out;
+    p.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kWaitCycles;
+    for (int r = 0; r < 2; ++r) p.withhold_from[r] = a->withhold_from[r] ? a->withhold_from[r] : UINT32_MAX;
     const uint32_t slots = sms / (uint32_t)v->group;
     const uint32_t clusters = choice.items < slots ? choice.items : slots;
     return launch(v->kernel, clusters * (uint32_t)v->group, kThreads, (size_t)v->smem, v->group, stream,

@@ -91,6 +91,9 @@ __device__ __forceinline__ void mbar_arrive_at(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                  : "memory");
 }
+__device__ __forceinline__ void st_at(uint32_t cluster_addr, uint32_t value) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(value) : "memory");
+}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -349,6 +352,13 @@ __device__ __forceinline__ bool mbar_wait(const Waiter &w, Mbar *bar, uint32_t p
 __device__ __forceinline__ bool mbar_wait_warp(const Waiter &w, Mbar *bar, uint32_t parity,
                                                uint32_t where, uint32_t tile) {
     return __all_sync(0xffffffffu, mbar_wait(w, bar, parity, where, tile)) != 0;
+}
+
+// Wait without reporting, for what is in flight when the roles leave.
+__device__ __forceinline__ void mbar_drain(Mbar *bar, uint32_t parity, long long budget) {
+    const long long start = clock64();
+    while (!mbar_try(bar, parity))
+        if (clock64() - start > budget) break;
 }
 
 // ---- host: tensor maps ----------------------------------------------------------------

@@ -409,6 +409,17 @@ int qw_gpu_debug_attention_waits(h3_gpu *gpu, long long wait_cycles, int withhol
     return 1;
 }
 
+/* The same for the GEMM kernel: the producers of a pair's first and second CTA leave
+ * out every K step from withhold_first / withhold_second on. */
+int qw_gpu_debug_linear_waits(h3_gpu *gpu, long long wait_cycles, uint32_t withhold_first,
+                              uint32_t withhold_second) {
+    if (!gpu || wait_cycles < 0) return 0;
+    gpu->linear_wait_cycles = wait_cycles;
+    gpu->linear_withhold[0] = withhold_first;
+    gpu->linear_withhold[1] = withhold_second;
+    return 1;
+}
+
 /* ---- copy lanes (no counterpart in the reference) -------------------------
  * A host program that streams inputs in and results out overlaps three things:
  * the upload of the next layer, the compute of this one, the read-back of the

@@ -214,6 +214,11 @@ typedef struct {
     float epsilon;
     float *bound_out;
     uint32_t *status;
+    /* Bounded-wait exercise (tests only): wait budget in SM cycles (0 = default, about
+     * 0.2 s) and, for the first and the second CTA of a pair, the K step (>= 1, counted
+     * from a CTA's first) from which its producer loads nothing (0 = none withheld). */
+    long long wait_cycles;
+    uint32_t withhold_from[2];
 } qwcu_linear_args;
 
 int qwcu_linear_sm100_launch(const qwcu_linear_args *args, int sm_count, qwcu_stream stream);

@@ -29,6 +29,8 @@ struct h3_gpu {
     int attn_kernel;
     long long attn_wait_cycles; /* tests: budget of the attention kernel's waits (0 = default) */
     int attn_withhold_tile;     /* tests: first key tile the producer leaves out (0 = none) */
+    long long linear_wait_cycles; /* the same for the GEMM kernel */
+    uint32_t linear_withhold[2];  /* first K step left out by the CTAs of a pair (0 = none) */
     /* A multi-GPU group's communication stream; submit waits for it too. */
     cudaStream_t aux_stream;
     cudaEvent_t aux_joined;

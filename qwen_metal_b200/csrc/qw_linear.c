@@ -9,6 +9,8 @@
 static int launch_linear(h3_gpu *gpu, qwcu_linear_args *args, const char *what) {
     if (!qw_bind(gpu)) return 0;
     args->status = gpu->status_dev;
+    args->wait_cycles = gpu->linear_wait_cycles;
+    for (int i = 0; i < 2; i++) args->withhold_from[i] = gpu->linear_withhold[i];
     int rc = qwcu_linear_sm100_launch(args, qwcu_device_sm_count(gpu->device), gpu->stream);
     qw_count_launch(gpu, rc, what);
     return rc == 0;

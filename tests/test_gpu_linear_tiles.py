@@ -83,3 +83,43 @@ def test_fused_epilogue_on_every_tile_shape(gpu, seq, dim):
     assert np.array_equal(fv.reshape(seq, dim), got[2])
     for t in [xt, wqt, wkt, ct, st, bt] + wts + plain + fused:
         gpu.free(t)
+
+
+@pytest.mark.parametrize("rows,k,n", [
+    (200, 1024, 520),    # 128-column pair tiles, one per pair
+    (1100, 1024, 5120),  # 256-column pair tiles, whole and half
+    (300, 1024, 11520),  # single CTAs
+])
+@pytest.mark.parametrize("withheld", [(5, 5), (5, 7), (7, 5), (3, 0), (0, 4)])
+def test_expired_waits_leave_nothing_in_flight(gpu, rows, k, n, withheld):
+    """The GEMM's waits run out cleanly.  With a budget of about a millisecond and
+    producers that leave out every K step from some point on -- the same for both CTAs of a
+    pair, or one earlier than the other, so that the copies of the other are in flight for
+    steps that never become complete -- the kernel records where, brings every copy it
+    issued to its end, frees its TMEM and returns; h3_gpu_submit reports it, and the next
+    launch on the context gives the bits it gave before."""
+    P.check(gpu, rows, n, 1)
+    if P.plan(gpu, rows, n, 1).ctas == 1 and not withheld[0]:
+        pytest.skip("a single CTA has no second producer")
+    lib = gpu.lib
+    rng = np.random.default_rng(rows)
+    xt, wt = gpu.bf16(workloads.normal_bf16(rng, (rows, k))), gpu.bf16(weights(rng, n, k))
+    ot = gpu.new_bf16(rows * n)
+
+    def launch():
+        gpu.begin()
+        assert lib.h3_gpu_linear_bf16(gpu.handle, ot, xt, wt, None, rows, k, n) == 1
+        return lib.h3_gpu_submit(gpu.handle)
+
+    assert launch() == 1
+    want = gpu.read_bf16(ot, rows * n)
+    try:
+        assert lib.qw_gpu_debug_linear_waits(gpu.handle, 2_000_000, *withheld)
+        assert launch() == 0
+        assert "wait ran out" in gpu.error(), gpu.error()
+    finally:
+        assert lib.qw_gpu_debug_linear_waits(gpu.handle, 0, 0, 0)
+    assert launch() == 1
+    assert np.array_equal(gpu.read_bf16(ot, rows * n), want)
+    for t in (xt, wt, ot):
+        gpu.free(t)
