@@ -478,17 +478,20 @@ bool choose(Choice *best, uint32_t m, uint32_t n, uint32_t n_outputs, uint32_t s
     return best->v != nullptr;
 }
 
-// The opt-in to more than 48 KB of dynamic shared memory is a per-device attribute.
-bool kernel_ready(const Variant *v) {
-    static bool ready[64][kVariantCount];
+// The opt-in to more than 48 KB of dynamic shared memory is a per-device attribute.  The
+// first launch sets it for all variants: a size that takes another one may follow inside a
+// graph capture.
+bool kernels_ready() {
+    static bool ready[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     const bool tracked = dev >= 0 && dev < 64;
-    if (tracked && ready[dev][v - kVariants]) return true;
-    if (cudaFuncSetAttribute(v->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v->smem) !=
-        cudaSuccess)
-        return false;
-    if (tracked) ready[dev][v - kVariants] = true;
+    if (tracked && ready[dev]) return true;
+    for (const Variant &v : kVariants)
+        if (cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem) !=
+            cudaSuccess)
+            return false;
+    if (tracked) ready[dev] = true;
     return true;
 }
 
@@ -519,7 +522,7 @@ extern "C" int qwcu_linear_sm100_launch(const qwcu_linear_args *a, int sm_count,
     Choice choice;
     if (!choose(&choice, a->m, a->n, a->n_outputs, sms)) return (int)cudaErrorInvalidValue;
     const Variant *v = choice.v;
-    if (!kernel_ready(v)) return (int)cudaGetLastError();
+    if (!kernels_ready()) return (int)cudaGetLastError();
     Maps maps;
     memset(&maps, 0, sizeof(maps));
     int rc;

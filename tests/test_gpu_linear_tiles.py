@@ -123,3 +123,13 @@ def test_expired_waits_leave_nothing_in_flight(gpu, rows, k, n, withheld):
     assert np.array_equal(gpu.read_bf16(ot, rows * n), want)
     for t in (xt, wt, ot):
         gpu.free(t)
+
+
+def test_a_tile_shape_met_first_inside_a_capture():
+    """The op has run before the capture, but at a size that takes another kernel."""
+    import os
+    import subprocess
+    import sys
+    worker = os.path.join(os.path.dirname(os.path.abspath(__file__)), "capture_worker.py")
+    done = subprocess.run([sys.executable, worker], capture_output=True, text=True, timeout=240)
+    assert done.returncode == 0, done.stdout[-2000:] + done.stderr[-2000:]
