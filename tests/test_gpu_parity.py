@@ -738,6 +738,36 @@ def test_rope_tables_on_device_match_host(gpu):
     assert b"bad arguments" in err.value
 
 
+@pytest.mark.parametrize("rows", [592, 593, 1184, 1185, 2369, 3552, 3553])
+def test_prologue_grid_sizes(gpu, rows):
+    """A row's result does not depend on the grid: on 148 SMs the CTAs of these launches
+    are left to the scheduler (74), held to one, two or three per SM (75 .. 444) and left
+    alone again (445); each equals launches of 100 rows."""
+    lib, heads = gpu.lib, 2
+    rng = np.random.default_rng(rows)
+    q, k = (randn_bf16(rng, (rows, heads * 128)) for _ in range(2))
+    wq, wk = (randn_bf16(rng, (128,), 1.0, 0.1) for _ in range(2))
+    angle = rng.uniform(0, 6.0, (rows, 64))
+    cos, sin = np.cos(angle).astype(np.float32), np.sin(angle).astype(np.float32)
+
+    def run(lo, hi):
+        n = (hi - lo) * heads * 128
+        ts = [gpu.bf16(q[lo:hi]), gpu.bf16(k[lo:hi]), gpu.bf16(wq), gpu.bf16(wk), gpu.f32(cos[lo:hi]),
+              gpu.f32(sin[lo:hi]), gpu.new_bf16(n), gpu.new_bf16(n), gpu.new_f32(2)]
+        gpu.begin()
+        gpu.check(lib.qw_gpu_qk_norm_rope_bound_bf16(gpu.handle, ts[6], ts[7], *ts[:6], ts[8], 1, hi - lo,
+                                                     heads, 128, workloads.EPS), "prologue")
+        gpu.submit()
+        out = [gpu.read_bf16(t, n).reshape(hi - lo, -1) for t in ts[6:8]]
+        for t in ts:
+            gpu.free(t)
+        return out
+
+    parts = [run(lo, min(lo + 100, rows)) for lo in range(0, rows, 100)]
+    for got, want in zip(run(0, rows), zip(*parts)):
+        assert np.array_equal(got, np.concatenate(want))
+
+
 # --------------------------------------------------------------------------
 # edit path after the first step: target rows only, against the K/V cache
 # --------------------------------------------------------------------------
