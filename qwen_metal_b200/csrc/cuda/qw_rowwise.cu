@@ -277,21 +277,31 @@ extern "C" int qwcu_layer_norm_mod_launch(const qwcu_rowwise_args *a, int sm_cou
     constexpr unsigned threads = kWarpsPerBlock * 32;
     if (!vector)
         return sm100::launch(qw_layer_norm_mod_generic_kernel, blocks, threads, 0, 1, stream, k);
-    // A few resident CTAs per SM, each warp walking rows; with fewer rows than those
-    // warps a CTA takes one row.
-    const unsigned cap = (unsigned)(sm_count > 0 ? sm_count : 148) * 4u;
-    const bool few = blocks <= cap;
-    const unsigned grid = few ? a->rows : cap;
+    // With fewer rows than the warps of four CTAs per SM a CTA takes one row.  More rows:
+    // warps that walk rows, in as many CTAs as the registers let be resident.  Started under
+    // the tail of the kernel before it, a smaller grid would pile up on the SMs that are free
+    // first (8704 rows of 1024: 10.9 us with 4 per SM, 6.6 us with 8; of 2048: 14.1 us with 4,
+    // 10.6 us with 5), and a larger one has a second wave (of 4096: 39.5 us with 4, 31.5 us
+    // with 3).
+    const unsigned sms = (unsigned)(sm_count > 0 ? sm_count : 148);
+    const bool few = blocks <= sms * 4u;
     const uint32_t vecs_per_lane = (a->width / 8 + 31) / 32;
     void (*kernel)(const NormArgs);
-    if (vecs_per_lane <= 4)
+    unsigned resident;
+    if (vecs_per_lane <= 4) {
         kernel = few ? qw_layer_norm_mod_kernel<1, 4> : qw_layer_norm_mod_kernel<4, 1>;
-    else if (vecs_per_lane <= 8)
+        resident = 8;
+    } else if (vecs_per_lane <= 8) {
         kernel = few ? qw_layer_norm_mod_kernel<2, 4> : qw_layer_norm_mod_kernel<8, 1>;
-    else if (vecs_per_lane <= 12)
+        resident = 5;
+    } else if (vecs_per_lane <= 12) {
         kernel = few ? qw_layer_norm_mod_kernel<3, 4> : qw_layer_norm_mod_kernel<12, 1>;
-    else
+        resident = 4;
+    } else {
         kernel = few ? qw_layer_norm_mod_kernel<4, 4> : qw_layer_norm_mod_kernel<kMaxVecs, 1>;
+        resident = 3;
+    }
+    const unsigned grid = few ? a->rows : blocks < sms * resident ? blocks : sms * resident;
     return sm100::launch(kernel, grid, threads, 0, 1, stream, k);
 }
 

@@ -167,6 +167,7 @@ def test_modulation_row_index_outside_the_tensor_is_reported(gpu):
 @pytest.mark.parametrize("rows,width", [
     (1, 8), (3, 1024), (5, 1032), (2, 2056), (7, 3080), (3, 4096),  # a CTA per row: the vectors' edges
     (2368, 136), (2369, 136),  # the last row count of that form on 148 SMs, the first of the other
+    (4737, 136), (2961, 1032), (2369, 4096),  # a second row for the first warp of 8, 5 and 3 CTAs per SM
 ])
 def test_norm_mod_forms_match_oracle(gpu, rows, width):
     rng = np.random.default_rng(rows + width)
