@@ -52,10 +52,6 @@
 // scale applied to fp32 scores, P rounded to bf16 before P V, fp32 accumulate,
 // output acc / l rounded to bf16; rows without a visible key store zeros.
 
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-#include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -63,6 +59,8 @@
 #include "qw_sm100.cuh"
 
 namespace {
+
+using namespace sm100;
 
 constexpr int kHeadDim = 128;
 constexpr int kTileM = 128;  // query rows per sub-tile (= TMEM lanes)
@@ -93,8 +91,6 @@ constexpr uint32_t kTmemS0 = 0, kTmemS1 = 128, kTmemO0 = 256, kTmemO1 = 384;
 // Lazy rescale threshold in the exp2 domain: P may grow to 2^8 before O and l
 // are brought back to the running maximum.
 constexpr float kRescaleThreshold = 8.0f;
-// Wait budget in SM clock cycles (~0.2 s); a healthy wait is microseconds.
-constexpr long long kWaitCycles = 400000000LL;
 
 enum Barrier : int {
     kBarQFull = 0,                        // 2: Q sub-tile i landed
@@ -104,14 +100,13 @@ enum Barrier : int {
     kBarPFirst = kBarSFull + 2,           // 2: first part of P_i written (one arrival per warp)
     kBarPFull = kBarPFirst + 2,           // 2: the rest of P_i written
     kBarOFinal = kBarPFull + 2,           // 2: last P V of sub-tile i complete
-    kBarDebug = kBarOFinal + 2,           // trace builds: group completion probe
-    kBarEpi = kBarDebug + 1,              // 2: output tile of sub-tile i staged in shared memory
+    kBarEpi = kBarOFinal + 2,             // 2: output tile of sub-tile i staged in shared memory
     kBarMerge = kBarEpi + 2,              // split form: sub-tile 1 published its exponent and row sum
     kBarCount = kBarMerge + 1
 };
 
 struct __align__(16) SharedControl {
-    unsigned long long bars[kBarCount];
+    Mbar bars[kBarCount];
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
     long long wait_cycles;  // budget of every bounded wait of this CTA
@@ -169,39 +164,10 @@ struct KernelParams {
     int withhold_from;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(unsigned long long *bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-
-// Bounded wait.  Returns false when the budget ran out here (recorded) or
-// another thread of the CTA already gave up.
-__device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, unsigned long long *bar,
+// Bounded wait.  Returns false when the budget ran out here (recorded) or another thread
+// of the CTA already gave up.  (The GEMM's, out of line after a few probes, is not used
+// here: the softmax waits with its registers full.)
+__device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, Mbar *bar,
                                             uint32_t parity, uint32_t *status, uint32_t where,
                                             uint32_t tile) {
     long long start = clock64();
@@ -222,7 +188,7 @@ __device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, unsigned long
     }
 }
 
-__device__ __forceinline__ bool mbar_wait(SharedControl *ctl, unsigned long long *bar,
+__device__ __forceinline__ bool mbar_wait(SharedControl *ctl, Mbar *bar,
                                           uint32_t parity, uint32_t *status, uint32_t where,
                                           uint32_t tile) {
     if (mbar_try(bar, parity)) return true;
@@ -230,7 +196,7 @@ __device__ __forceinline__ bool mbar_wait(SharedControl *ctl, unsigned long long
 }
 
 // The same for all lanes of a warp at once: true when every lane saw the phase complete.
-__device__ __forceinline__ bool mbar_wait_warp(SharedControl *ctl, unsigned long long *bar,
+__device__ __forceinline__ bool mbar_wait_warp(SharedControl *ctl, Mbar *bar,
                                                uint32_t parity, uint32_t *status, uint32_t where,
                                                uint32_t tile) {
     return __all_sync(0xffffffffu, mbar_wait(ctl, bar, parity, status, where, tile)) != 0;
@@ -241,91 +207,15 @@ template <typename T>
 __device__ __forceinline__ T uniform(T v) {
     return __shfl_sync(0xffffffffu, v, 0);
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(pred));
-    return pred != 0;
-}
-
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map,
-                                            unsigned long long *bar, int c0, int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-
 // Output tensor maps, one per destination (one on a single GPU, one per rank
 // when the heads are sharded and every rank receives the rows).
 struct OutMaps {
     CUtensorMap m[8];
 };
 
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void *src, int c0, int c1,
-                                             int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-        ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tc_commit(unsigned long long *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
-}
-
-// Shared-memory matrix descriptors (sm_100 format) are built as two 32-bit words
-// further down (desc_hi / desc_lo_fixed): start address >> 4 in bits 0-13, leading
-// byte offset >> 4 in bits 16-29, stride byte offset >> 4 in bits 32-45, descriptor
-// version 1 in bit 46, 128B swizzle = 2 in bits 61-63.
-
-// Instruction descriptor, kind::f16: bf16 x bf16 -> fp32, M = 128, N = 128.
-constexpr uint32_t make_idesc(bool b_mn_major) {
-    return (1u << 4)                      // D format: f32
-           | (1u << 7)                    // A format: bf16
-           | (1u << 10)                   // B format: bf16
-           | ((b_mn_major ? 1u : 0u) << 16)
-           | ((uint32_t)(kTileN >> 3) << 17)
-           | ((uint32_t)(kTileM >> 4) << 24);
-}
-constexpr uint32_t kIdescQK = make_idesc(false);
-constexpr uint32_t kIdescPV = make_idesc(true);
-
-// Descriptors travel as (low word, high word): stepping through a tile only
-// changes the start-address field in the low word, so each MMA costs one
-// integer add per operand on the issuing thread.
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
-                                       uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-        "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-        "setp.ne.b32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi,
-                                       uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
+// Instruction descriptors, M = 128, N = 128.
+constexpr uint32_t kIdescQK = instr_desc(kTileM, kTileN, false);
+constexpr uint32_t kIdescPV = instr_desc(kTileM, kTileN, true);
 
 #define QW_TMEM_LD32(taddr, r)                                                                  \
     asm volatile(                                                                               \
@@ -380,20 +270,10 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_
 __device__ __forceinline__ void tmem_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() {
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
 }
 
 // Packed fp32 pairs (one issue slot for two lanes of work on sm_100).
@@ -429,8 +309,9 @@ constexpr int kTraceSlots = 4096;
 __device__ __forceinline__ void trace_event(const KernelParams &p, int role, int event, int tile,
                                             uint32_t &cursor) {
     // One private region per role and a register cursor: a plain store, no
-    // round trip, so the log barely perturbs what it measures.
-    if (p.trace && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && cursor < 1000) {
+    // round trip, so the log barely perturbs what it measures.  (The MMA warp runs its
+    // loop with all lanes: one writes.)
+    if (p.trace && (threadIdx.x & 31) == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && cursor < 1000) {
         p.trace[1 + role * 1024 + cursor] =
             ((unsigned long long)(role << 20 | event << 12 | (tile & 0xfff)) << 40) |
             ((unsigned long long)clock64() & 0xffffffffffull);
@@ -473,7 +354,7 @@ __device__ __forceinline__ int visited_tiles(int tiles, int lo, int hi) {
 // ---------------------------------------------------------------------------
 // The first part of P is complete once its stores, issued a chunk of exponentials ago,
 // have landed: P V of these keys starts under the softmax of the others.
-__device__ __forceinline__ void publish_p_first(unsigned long long *bar, int tid_in_group) {
+__device__ __forceinline__ void publish_p_first(Mbar *bar, int tid_in_group) {
     tmem_wait_st();
     tc_fence_before();
     if ((tid_in_group & 31) == 0) mbar_arrive(bar);
@@ -514,9 +395,9 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
     const uint32_t tmem = ctl->tmem_base;
     const uint32_t tmem_s = tmem + lane_base + (sub ? kTmemS1 : kTmemS0);
     const uint32_t tmem_o = tmem + lane_base + (sub ? kTmemO1 : kTmemO0);
-    unsigned long long *bar_s = &ctl->bars[kBarSFull + sub];
-    unsigned long long *bar_p_first = &ctl->bars[kBarPFirst + sub];
-    unsigned long long *bar_p = &ctl->bars[kBarPFull + sub];
+    Mbar *bar_s = &ctl->bars[kBarSFull + sub];
+    Mbar *bar_p_first = &ctl->bars[kBarPFirst + sub];
+    Mbar *bar_p = &ctl->bars[kBarPFull + sub];
     const int pad_lo = p.text_pad ? (int)p.text_len[b] : 0;
     const int pad_hi = (int)p.text_pad;
     const float c = p.scale_log2;  // positive (the host sends other scales elsewhere)
@@ -781,7 +662,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
         }
     }
     if (p.head_major_out) return;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> TMA reads
+    fence_async_shared();
     __syncwarp();
     if ((tid_in_group & 31) == 0) mbar_arrive(&ctl->bars[kBarEpi + sub]);
     if (tid_in_group == 0) {
@@ -793,11 +674,11 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
             tma_store_3d(&maps_out.m[d], stage, col, (int)tile_row0, (int)b);
             tma_store_3d(&maps_out.m[d], stage + kHalfTileBytes, col + 64, (int)tile_row0, (int)b);
         }
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        tma_store_commit();
         // Shared memory may be released once the stores have read it; the
         // writes themselves are complete when the grid completes, which is
         // what the barrier behind a sharded launch waits for.
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        tma_store_wait_read<0>();
     }
 }
 
@@ -807,14 +688,9 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
 // the MMAs then stay in uniform registers, where in a one-lane branch each of them is
 // moved there first, more clocks per MMA than the 64 it executes in.
 // ---------------------------------------------------------------------------
-// High words of the two descriptor kinds (everything but the start address).
-constexpr uint32_t desc_hi(uint32_t sbo_bytes) {
-    return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);  // SBO, version 1, SWIZZLE_128B
-}
-constexpr uint32_t desc_lo_fixed(uint32_t lbo_bytes) { return ((lbo_bytes >> 4) & 0x3FFFu) << 16; }
-constexpr uint32_t kDescHi = desc_hi(1024);
-constexpr uint32_t kDescLoKMajor = desc_lo_fixed(16);               // LBO unused for K-major SW128
-constexpr uint32_t kDescLoVMajor = desc_lo_fixed(kHalfTileBytes);   // next 64-column half
+// Low descriptor words, everything but the start address; V's two 64-column halves lie half
+// a tile apart.
+constexpr uint32_t kDescLoVMajor = desc_lo(kHalfTileBytes);
 
 __device__ __forceinline__ void issue_qk(uint32_t d_tmem, uint32_t q_lo, uint32_t k_lo) {
     // K-major operands, 128B swizzle: 8-row groups 1024 B apart; the second
@@ -822,7 +698,7 @@ __device__ __forceinline__ void issue_qk(uint32_t d_tmem, uint32_t q_lo, uint32_
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
         const uint32_t off = ((uint32_t)(kk >> 2) * kHalfTileBytes + (uint32_t)(kk & 3) * 32u) >> 4;
-        mma_ss(d_tmem, q_lo + off, kDescHi, k_lo + off, kDescHi, kIdescQK, kk > 0 ? 1u : 0u);
+        mma_ss<1>(d_tmem, q_lo + off, k_lo + off, kIdescQK, kk > 0 ? 1u : 0u);
     }
 }
 
@@ -835,7 +711,7 @@ __device__ __forceinline__ void issue_pv_keys(uint32_t d_tmem, uint32_t p_tmem, 
     // halves one half tile apart.
 #pragma unroll
     for (int kk = kFrom; kk < kTo; ++kk) {
-        mma_ts(d_tmem, p_tmem + (uint32_t)kk * 8u, v_lo + (uint32_t)(kk * 2048 >> 4), kDescHi, kIdescPV,
+        mma_ts(d_tmem, p_tmem + (uint32_t)kk * 8u, v_lo + (uint32_t)(kk * 2048 >> 4), kIdescPV,
                (accumulate || kk > 0) ? 1u : 0u);
     }
 }
@@ -861,8 +737,8 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
     if (j >= n_max) return;
     const uint32_t tmem = uniform(ctl->tmem_base);
     // Low descriptor words: start address in 16-byte units plus the fixed LBO field.
-    const uint32_t q_lo[2] = {(smem_u32(smem_q) >> 4) | kDescLoKMajor,
-                              (smem_u32(smem_q + kTileBytes) >> 4) | kDescLoKMajor};
+    const uint32_t q_lo[2] = {(smem_u32(smem_q) >> 4) | kDescKMajor,
+                              (smem_u32(smem_q + kTileBytes) >> 4) | kDescKMajor};
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;  // slot s starts (s * kTileBytes) >> 4 further
     const uint32_t s_tmem[2] = {tmem + kTmemS0, tmem + kTmemS1};
     const uint32_t o_tmem[2] = {tmem + kTmemO0, tmem + kTmemO1};
@@ -871,7 +747,6 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
     bool o_started[2] = {false, false};
     uint32_t t = 0;  // ring position (K and V tiles alternate)
     [[maybe_unused]] uint32_t trace_cursor = 0;
-    [[maybe_unused]] uint32_t dbg_phase = 0;
     const uint32_t where = 2u << 16;
 
 #pragma unroll
@@ -886,14 +761,14 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
                        where | (kBarKvFull + slot), (uint32_t)j))
             return;
         tc_fence_after();
-        const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescLoKMajor;
+        const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescKMajor;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
             if (j < n_sub[i] && elect_one()) {
                 issue_qk(s_tmem[i], q_lo[i], k_lo);
-                tc_commit(&ctl->bars[kBarSFull + i]);
+                tc_commit<1>(&ctl->bars[kBarSFull + i]);
             }
-        if (elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + slot]);
+        if (elect_one()) tc_commit<1>(&ctl->bars[kBarKvEmpty + slot]);
         __syncwarp();
     }
     while (j < n_max) {
@@ -912,7 +787,7 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             return;
         QW_TRACE(2, 7, j);
         const uint32_t v_lo = (kv_lo + v_slot * (kTileBytes >> 4)) | kDescLoVMajor;
-        const uint32_t k_lo = (kv_lo + k_slot * (kTileBytes >> 4)) | kDescLoKMajor;
+        const uint32_t k_lo = (kv_lo + k_slot * (kTileBytes >> 4)) | kDescKMajor;
         if (jn < n_max &&
             !mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
                        where | (kBarKvFull + k_slot), (uint32_t)jn))
@@ -938,34 +813,26 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
                 o_started[i] = true;
                 QW_TRACE(2, 4 + i, j);
             }
-            if (i == 1 && elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + v_slot]);
+            if (i == 1 && elect_one()) tc_commit<1>(&ctl->bars[kBarKvEmpty + v_slot]);
             __syncwarp();
             if (jn < n_max && jn < n_sub[i]) {
                 if (elect_one()) {
                     issue_qk(s_tmem[i], q_lo[i], k_lo);
-                    tc_commit(&ctl->bars[kBarSFull + i]);
+                    tc_commit<1>(&ctl->bars[kBarSFull + i]);
                 }
                 __syncwarp();
                 QW_TRACE(2, 2 + i, jn);
-#ifdef QW_ATTN_TRACE_SERIAL
-                // Probe: wait until the group just issued has executed.
-                tc_commit(&ctl->bars[kBarDebug]);
-                if (!mbar_wait_warp(ctl, &ctl->bars[kBarDebug], dbg_phase, p.status, where | kBarDebug, 0))
-                    return;
-                dbg_phase ^= 1u;
-                QW_TRACE(2, 10 + i, jn);
-#endif
             }
         }
         if (jn < n_max) {
-            if (elect_one()) tc_commit(&ctl->bars[kBarKvEmpty + k_slot]);
+            if (elect_one()) tc_commit<1>(&ctl->bars[kBarKvEmpty + k_slot]);
             __syncwarp();
         }
         j = jn;
     }
     if (elect_one()) {
-        tc_commit(&ctl->bars[kBarOFinal + 0]);
-        tc_commit(&ctl->bars[kBarOFinal + 1]);
+        tc_commit<1>(&ctl->bars[kBarOFinal + 0]);
+        tc_commit<1>(&ctl->bars[kBarOFinal + 1]);
     }
 }
 
@@ -981,7 +848,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
     const int la = uniform(ctl->tile_count[0]), lb = uniform(ctl->tile_count[1]);
     if (la <= 0) return;
     const uint32_t tmem = uniform(ctl->tmem_base);
-    const uint32_t q_lo = (smem_u32(smem_q) >> 4) | kDescLoKMajor;
+    const uint32_t q_lo = (smem_u32(smem_q) >> 4) | kDescKMajor;
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;
     const uint32_t s_tmem[2] = {tmem + kTmemS0, tmem + kTmemS1};
     const uint32_t o_tmem[2] = {tmem + kTmemO0, tmem + kTmemO1};
@@ -998,22 +865,22 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
         tc_fence_after();                                                                       \
         out_ = (kv_lo + slot_ * (kTileBytes >> 4)) | (lo_fixed_);                               \
     }
-#define QW_RING_FREE(t_) tc_commit(&ctl->bars[kBarKvEmpty + ((t_) % kStages)])
+#define QW_RING_FREE(t_) tc_commit<1>(&ctl->bars[kBarKvEmpty + ((t_) % kStages)])
 
     if (!mbar_wait_warp(ctl, &ctl->bars[kBarQFull + 0], 0, p.status, where | kBarQFull, 0)) return;
     uint32_t desc;
-    QW_RING_WAIT(pair_a(0, lb), kDescLoKMajor, desc);
+    QW_RING_WAIT(pair_a(0, lb), kDescKMajor, desc);
     if (elect_one()) {
         issue_qk(s_tmem[0], q_lo, desc);
-        tc_commit(&ctl->bars[kBarSFull + 0]);
+        tc_commit<1>(&ctl->bars[kBarSFull + 0]);
         QW_RING_FREE(pair_a(0, lb));
     }
     __syncwarp();
     if (lb > 0) {
-        QW_RING_WAIT(pair_b(0), kDescLoKMajor, desc);
+        QW_RING_WAIT(pair_b(0), kDescKMajor, desc);
         if (elect_one()) {
             issue_qk(s_tmem[1], q_lo, desc);
-            tc_commit(&ctl->bars[kBarSFull + 1]);
+            tc_commit<1>(&ctl->bars[kBarSFull + 1]);
             QW_RING_FREE(pair_b(0));
         }
         __syncwarp();
@@ -1043,10 +910,10 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             __syncwarp();
             if (s + 1 < count) {
                 const uint32_t t_next = i ? pair_b(s + 1) : pair_a(s + 1, lb);
-                QW_RING_WAIT(t_next, kDescLoKMajor, desc);
+                QW_RING_WAIT(t_next, kDescKMajor, desc);
                 if (elect_one()) {
                     issue_qk(s_tmem[i], q_lo, desc);
-                    tc_commit(&ctl->bars[kBarSFull + i]);
+                    tc_commit<1>(&ctl->bars[kBarSFull + i]);
                     QW_RING_FREE(t_next);
                 }
                 __syncwarp();
@@ -1056,8 +923,8 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
 #undef QW_RING_WAIT
 #undef QW_RING_FREE
     if (elect_one()) {
-        tc_commit(&ctl->bars[kBarOFinal + 0]);
-        tc_commit(&ctl->bars[kBarOFinal + 1]);
+        tc_commit<1>(&ctl->bars[kBarOFinal + 0]);
+        tc_commit<1>(&ctl->bars[kBarOFinal + 1]);
     }
 }
 
@@ -1087,7 +954,7 @@ __device__ void tma_role(const KernelParams &p, SharedControl *ctl, uint8_t *sme
             if (!ok) break;
             ++t;
             uint8_t *dst = smem_kv + (size_t)slot * kTileBytes;
-            unsigned long long *bar = &ctl->bars[kBarKvFull + slot];
+            Mbar *bar = &ctl->bars[kBarKvFull + slot];
             mbar_expect_tx(bar, kTileBytes);
             const CUtensorMap *map = which ? map_v : map_k;
             tma_load_3d(dst, map, bar, col, j * kTileN, (int)b);
@@ -1122,7 +989,7 @@ __device__ __forceinline__ void issue_q_loads(const KernelParams &p, SharedContr
     for (int i = 0; i < tiles; ++i) {
         uint32_t r = row0 + (uint32_t)i * kTileM;
         if (r >= p.q_rows) continue;  // inactive sub-tile: n_tiles is 0, nobody waits
-        unsigned long long *bar = &ctl->bars[kBarQFull + i];
+        Mbar *bar = &ctl->bars[kBarQFull + i];
         mbar_expect_tx(bar, kTileBytes);
         uint8_t *dst = smem_q + (size_t)i * kTileBytes;
         tma_load_3d(dst, map_q, bar, (int)(h * kHeadDim), (int)r, (int)b);
@@ -1143,7 +1010,7 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
     SharedControl *ctl = reinterpret_cast<SharedControl *>(smem + kSmemData);
 
     const int tid = threadIdx.x;
-    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be warp-uniform
+    const int warp = warp_index();
     const int lane = tid & 31;
     // CTA -> unit.  Units are numbered batch-major, then head, then query block
     // with the heaviest blocks first (rows late in the joint sequence see the most
@@ -1175,7 +1042,6 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
             mbar_init(&ctl->bars[kBarEpi + i], kTileM / 32);
         }
         mbar_init(&ctl->bars[kBarMerge], kTileM / 32);
-        mbar_init(&ctl->bars[kBarDebug], 1);
         ctl->abort_flag = 0;
         ctl->wait_cycles = p.wait_cycles > 0 ? p.wait_cycles : kWaitCycles;
         int lo = 0, hi = 0;
@@ -1186,19 +1052,15 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         }
         ctl->skip_lo = lo;
         ctl->skip_hi = hi;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_init_fence();
     }
     if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(&ctl->tmem_base)),
-                     "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        tmem_alloc<1>(&ctl->tmem_base, kTmemCols);
     }
     // What stands above may run under the tail of the kernel before this one; all that
     // reads or writes global memory stands below.
-    sm100::grid_launch_dependents();
-    sm100::grid_wait();
+    grid_launch_dependents();
+    grid_wait();
     if (warp == kTmaWarp && lane == 0) {
         const int lo = ctl->skip_lo, hi = ctl->skip_hi;
         issue_q_loads(p, ctl, smem_q, &map_q, b, h, row0, split ? 1 : 2);
@@ -1207,7 +1069,7 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         const int j0 = lo == 0 ? hi : 0;
         for (int which = 0; which < 2; ++which) {
             uint8_t *dst = smem_kv + (size_t)which * kTileBytes;
-            unsigned long long *bar = &ctl->bars[kBarKvFull + which];
+            Mbar *bar = &ctl->bars[kBarKvFull + which];
             mbar_expect_tx(bar, kTileBytes);
             const CUtensorMap *map = which ? &map_v : &map_k;
             const int col = (int)(kvh * kHeadDim);
@@ -1309,43 +1171,16 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
     __syncthreads();
     if (warp == kMmaWarp) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(ctl->tmem_base),
-                     "r"(kTmemCols)
-                     : "memory");
+        tmem_dealloc<1>(ctl->tmem_base, kTmemCols);
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) ==
-                cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(sym);
-    }
-    return fn;
-}
-
-// [batch][rows][heads*128] bf16, boxes of 128 rows x 64 columns, 128B swizzle.
-int make_map(CUtensorMap *map, const void *base, uint32_t batch, uint32_t rows, uint32_t heads) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return (int)cudaErrorNotSupported;
-    cuuint64_t dims[3] = {(cuuint64_t)heads * kHeadDim, rows, batch};
-    cuuint64_t strides[2] = {(cuuint64_t)heads * kHeadDim * 2,
-                             (cuuint64_t)rows * heads * kHeadDim * 2};
-    cuuint32_t box[3] = {64, kTileN, 1};
-    cuuint32_t elem[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(base), dims,
-                    strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+// [batch][rows][heads*128] bf16, boxes of 128 rows x 64 columns.
+int make_map_3d(CUtensorMap *map, const void *base, uint32_t batch, uint32_t rows, uint32_t heads) {
+    const cuuint64_t dims[3] = {(cuuint64_t)heads * kHeadDim, rows, batch};
+    const cuuint64_t strides[2] = {(cuuint64_t)heads * kHeadDim * 2,
+                                   (cuuint64_t)rows * heads * kHeadDim * 2};
+    return make_map(map, base, 3, dims, strides, kTileN);
 }
 
 #ifdef QW_ATTN_TRACE
@@ -1452,9 +1287,9 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
     if (!kernel) return (int)cudaGetLastError();
     CUtensorMap map_q, map_k, map_v;
     int rc;
-    if ((rc = make_map(&map_q, a->q, a->batch, a->q_rows, a->heads))) return rc;
-    if ((rc = make_map(&map_k, a->k, a->batch, a->kv_rows, a->kv_heads))) return rc;
-    if ((rc = make_map(&map_v, a->v, a->batch, a->kv_rows, a->kv_heads))) return rc;
+    if ((rc = make_map_3d(&map_q, a->q, a->batch, a->q_rows, a->heads))) return rc;
+    if ((rc = make_map_3d(&map_k, a->k, a->batch, a->kv_rows, a->kv_heads))) return rc;
+    if ((rc = make_map_3d(&map_v, a->v, a->batch, a->kv_rows, a->kv_heads))) return rc;
     KernelParams p;
     p.out = static_cast<__nv_bfloat16 *>(a->out);
     p.kv_limit = a->kv_limit;
@@ -1500,7 +1335,7 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
     memset(&maps_out, 0, sizeof(maps_out));
     if (!p.head_major_out)
         for (uint32_t d = 0; d < p.n_out; ++d)
-            if ((rc = make_map(&maps_out.m[d], p.out_peers[d], a->batch, a->q_rows, p.out_heads_total)))
+            if ((rc = make_map_3d(&maps_out.m[d], p.out_peers[d], a->batch, a->q_rows, p.out_heads_total)))
                 return rc;
     // One CTA per unit; the units of the last, partly filled wave run split in two
     // (half the rows each, the key tiles divided between the sub-tiles) when the
@@ -1515,7 +1350,7 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
                        : qwcu_attn_sm100_tail_units(p.total_units,
                                                     (uint32_t)sm_count_of_current_device());
     const unsigned grid = p.total_units + p.tail_units;
-    rc = sm100::launch(kernel, grid, kThreads, kSmemBytes, 1, stream, map_q, map_k, map_v, maps_out, p);
+    rc = launch(kernel, grid, kThreads, kSmemBytes, 1, stream, map_q, map_k, map_v, maps_out, p);
 #ifdef QW_ATTN_TRACE
     if (p.trace && !rc) trace_dump(stream);
 #endif

@@ -34,9 +34,9 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- programmatic dependent launch ------------------------------------------
-// Every kernel of the library waits for its predecessor's results before it touches
-// global memory, so a launch may start (barriers, TMEM, descriptors) under the tail
-// of the one before it.
+// A kernel launched with launch() below may start (barriers, TMEM, descriptors) under the
+// tail of the one before it; it waits for that one's results before it touches global
+// memory.
 __device__ __forceinline__ void grid_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -117,21 +117,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, u
             "l"(map), "r"(bar), "r"(c0), "r"(c1)
             : "memory");
 }
-template <int kGroup>
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint32_t bar, int c0,
-                                            int c1, int c2) {
-    if constexpr (kGroup == 2)
-        asm volatile(
-            "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile."
-            "mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-            "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-            : "memory");
-    else
-        asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-            "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-            "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-            : "memory");
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, Mbar *bar, int c0, int c1,
+                                            int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
 }
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, const void *src, int c0, int c1) {
     asm volatile(
@@ -247,23 +239,14 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t 
             : "memory");
 }
 // A from TMEM.
-template <int kGroup>
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc,
                                        uint32_t accumulate) {
-    if constexpr (kGroup == 2)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-            "mov.b64 db, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
-            : "memory");
-    else
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-            "mov.b64 db, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
-            "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
-            : "memory");
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+        "mov.b64 db, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t (&r)[32], uint32_t taddr) {
@@ -277,14 +260,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t (&r)[32], uint32_t taddr) {
           "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
           "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
 }
 // tcgen05.wait::ld that names the registers of an earlier load as read-write operands:
 // no use of them can be scheduled ahead of the wait.
