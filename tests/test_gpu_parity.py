@@ -255,7 +255,7 @@ def test_cfg1_bidirectional_text_reading(gpu):
     gates(out, oracle_layer(w, inputs), "cfg1 bidirectional text")
 
 
-@pytest.fixture(params=["sm100", "sm100-whole", "sm100-row"])
+@pytest.fixture(params=["sm100", "sm100-whole"])
 def tail_form(request, gpu):
     assert gpu.lib.qw_gpu_set_attention_kernel(gpu.handle, request.param.encode())
     yield request.param
@@ -578,6 +578,8 @@ def test_error_conventions(gpu):
     assert lib.h3_gpu_copy_bf16(gpu.handle, t, 128, t, 0, 128) == 1
     gpu.submit()
     assert lib.h3_gpu_submit(gpu.handle) == 0                 # no open chain
+    for name, known in ((b"tensor", 0), (b"sm100-row", 1), (b"sm100", 1)):  # (the latter two are one)
+        assert lib.qw_gpu_set_attention_kernel(gpu.handle, name) == known
     buf = np.zeros(8, np.uint16)
     assert lib.h3_gpu_tensor_read_bf16(t, abi._ptr(buf), 10 ** 9) == 0
     assert lib.h3_gpu_tensor_read_bf16(f, abi._ptr(buf), 4) == 0
@@ -647,7 +649,7 @@ def test_copy_lanes_order_uploads_compute_and_readbacks(gpu):
 
 
 @pytest.mark.parametrize("softmax", ["max", "bounded"])
-@pytest.mark.parametrize("form", ["sm100", "sm100-whole", "sm100-row"])
+@pytest.mark.parametrize("form", ["sm100", "sm100-whole"])
 def test_bounded_waits_run_out_cleanly(gpu, form, softmax):
     """Every device-side wait of the attention kernel has a budget.  With a short
     budget and a producer that leaves out every key tile from the third on, the
