@@ -195,11 +195,18 @@ __device__ __forceinline__ bool mbar_wait(SharedControl *ctl, Mbar *bar,
     return mbar_wait_slow(ctl, bar, parity, status, where, tile);
 }
 
-// The same for all lanes of a warp at once: true when every lane saw the phase complete.
-__device__ __forceinline__ bool mbar_wait_warp(SharedControl *ctl, Mbar *bar,
-                                               uint32_t parity, uint32_t *status, uint32_t where,
-                                               uint32_t tile) {
-    return __all_sync(0xffffffffu, mbar_wait(ctl, bar, parity, status, where, tile)) != 0;
+// The wait of the MMA warp, for all its lanes at once, bounded by a number of probes: at least
+// 150 clocks each where one has to wait, 30 ms together, where a healthy wait is microseconds.
+// The warp issues every MMA of the CTA and each of its clocks is on the chain of both sub-tiles, so
+// the loop holds nothing else: with the clock, the abort flag and the record of the wait above
+// in it, text rows of 412 took 90 us a chain of six instead of 81, six heads 587 instead of
+// 572 us for eight layers, 24 heads of two 1738 instead of 1690 us for four.  When it runs out the
+// warp leaves in silence; the softmax, whose scores then stay away, records and raises the flag.
+constexpr int kMmaProbes = 400000;
+__device__ __forceinline__ bool mbar_wait_warp(Mbar *bar, uint32_t parity) {
+    bool ok = false;
+    for (int i = 0; i < kMmaProbes && !ok; ++i) ok = mbar_try(bar, parity);
+    return __all_sync(0xffffffffu, ok) != 0;
 }
 
 // A value the compiler knows to be the same in all lanes of the (converged) warp.
@@ -760,18 +767,16 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
     bool o_started[2] = {false, false};
     uint32_t t = 0;  // ring position (K and V tiles alternate)
     [[maybe_unused]] uint32_t trace_cursor = 0;
-    const uint32_t where = 2u << 16;
 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
         if (n_sub[i] > 0 &&
-            !mbar_wait_warp(ctl, &ctl->bars[kBarQFull + i], 0, p.status, where | (kBarQFull + i), 0))
+            !mbar_wait_warp(&ctl->bars[kBarQFull + i], 0))
             return;
     {
         uint32_t slot = t % kStages, par = (t / kStages) & 1u;
         ++t;
-        if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + slot], par, p.status,
-                       where | (kBarKvFull + slot), (uint32_t)j))
+        if (!mbar_wait_warp(&ctl->bars[kBarKvFull + slot], par))
             return;
         tc_fence_after();
         const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescKMajor;
@@ -795,29 +800,25 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             ++t;
         }
         QW_TRACE(2, 6, j);
-        if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + v_slot], v_par, p.status,
-                       where | (kBarKvFull + v_slot), (uint32_t)j))
+        if (!mbar_wait_warp(&ctl->bars[kBarKvFull + v_slot], v_par))
             return;
         QW_TRACE(2, 7, j);
         const uint32_t v_lo = (kv_lo + v_slot * (kTileBytes >> 4)) | kDescLoVMajor;
         const uint32_t k_lo = (kv_lo + k_slot * (kTileBytes >> 4)) | kDescKMajor;
         if (jn < n_max &&
-            !mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + k_slot], k_par, p.status,
-                       where | (kBarKvFull + k_slot), (uint32_t)jn))
+            !mbar_wait_warp(&ctl->bars[kBarKvFull + k_slot], k_par))
             return;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (j < n_sub[i]) {
-                if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFirst + i], p_phase[i], p.status,
-                                    where | (kBarPFirst + i), (uint32_t)j))
+                if (!mbar_wait_warp(&ctl->bars[kBarPFirst + i], p_phase[i]))
                     return;
                 tc_fence_after();
                 QW_TRACE(2, i, j);
                 if (elect_one())
                     issue_pv_first(o_tmem[i], s_tmem[i], v_lo, o_started[i], bounded);
                 __syncwarp();
-                if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
-                                    where | (kBarPFull + i), (uint32_t)j))
+                if (!mbar_wait_warp(&ctl->bars[kBarPFull + i], p_phase[i]))
                     return;
                 p_phase[i] ^= 1u;
                 tc_fence_after();
@@ -865,22 +866,20 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;
     const uint32_t s_tmem[2] = {tmem + kTmemS0, tmem + kTmemS1};
     const uint32_t o_tmem[2] = {tmem + kTmemO0, tmem + kTmemO1};
-    const uint32_t where = 2u << 16;
     uint32_t p_phase[2] = {0, 0};
 
     // Waits for ring position t, returns the low descriptor word of its slot.
 #define QW_RING_WAIT(t_, lo_fixed_, out_)                                                       \
     {                                                                                           \
         const uint32_t slot_ = (t_) % kStages, par_ = ((t_) / kStages) & 1u;                    \
-        if (!mbar_wait_warp(ctl, &ctl->bars[kBarKvFull + slot_], par_, p.status,                     \
-                       where | (kBarKvFull + slot_), (uint32_t)(t_)))                           \
+        if (!mbar_wait_warp(&ctl->bars[kBarKvFull + slot_], par_))                           \
             return;                                                                             \
         tc_fence_after();                                                                       \
         out_ = (kv_lo + slot_ * (kTileBytes >> 4)) | (lo_fixed_);                               \
     }
 #define QW_RING_FREE(t_) tc_commit<1>(&ctl->bars[kBarKvEmpty + ((t_) % kStages)])
 
-    if (!mbar_wait_warp(ctl, &ctl->bars[kBarQFull + 0], 0, p.status, where | kBarQFull, 0)) return;
+    if (!mbar_wait_warp(&ctl->bars[kBarQFull + 0], 0)) return;
     uint32_t desc;
     QW_RING_WAIT(pair_a(0, lb), kDescKMajor, desc);
     if (elect_one()) {
@@ -905,14 +904,12 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             if (s >= count) continue;
             const uint32_t t_now = i ? pair_b(s) : pair_a(s, lb);
             QW_RING_WAIT(t_now + 1, kDescLoVMajor, desc);
-            if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFirst + i], p_phase[i], p.status,
-                                where | (kBarPFirst + i), (uint32_t)s))
+            if (!mbar_wait_warp(&ctl->bars[kBarPFirst + i], p_phase[i]))
                 return;
             tc_fence_after();
             if (elect_one()) issue_pv_first(o_tmem[i], s_tmem[i], desc, s > 0, bounded);
             __syncwarp();
-            if (!mbar_wait_warp(ctl, &ctl->bars[kBarPFull + i], p_phase[i], p.status,
-                                where | (kBarPFull + i), (uint32_t)s))
+            if (!mbar_wait_warp(&ctl->bars[kBarPFull + i], p_phase[i]))
                 return;
             p_phase[i] ^= 1u;
             tc_fence_after();
