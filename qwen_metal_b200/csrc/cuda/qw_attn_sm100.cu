@@ -18,8 +18,8 @@
 // Mask: every row has an integer key limit (prefix) and the batch item may have
 // a key-padding window.  Key tiles past the largest limit of a sub-tile are
 // never issued, key tiles that lie completely inside the padding window are
-// skipped by all roles, interior tiles run without a compare, boundary tiles
-// apply the integer compare per element.
+// skipped by all roles, interior tiles run without a compare, the scores of boundary
+// tiles are masked in TMEM first.
 //
 // Epilogue: O / l is rounded to bf16 into the (by then dead) Q tile in shared
 // memory and leaves as TMA stores of the whole 128x128 tile.  When the heads
@@ -46,7 +46,7 @@
 //
 // Every wait is bounded: when one runs out the CTA records where in the status
 // words, raises a shared abort flag that all other waits poll, drains its TMA
-// loads, frees its TMEM and returns.
+// loads, frees its TMEM and returns.  (The MMA warp counts probes and leaves in silence.)
 //
 // Semantics follow the reference prefix kernel (h3_shaders.metal:3061-3272):
 // scale applied to fp32 scores, P rounded to bf16 before P V, fp32 accumulate,
