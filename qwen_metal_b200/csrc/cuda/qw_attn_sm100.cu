@@ -11,7 +11,7 @@
 // warpgroup to the two softmax warpgroups with setmaxnreg):
 //   warps 0-3   softmax + epilogue of sub-tile 0 (TMEM lanes 0..127)
 //   warps 4-7   softmax + epilogue of sub-tile 1
-//   warp  8     MMA issue (one elected lane), TMEM allocation
+//   warp  8     MMA issue (all lanes run the loop, one is elected per issue), TMEM allocation
 //   warp  9     TMA producer (one elected lane)
 //   warps 10-11 idle (they only complete the third warpgroup)
 //
@@ -45,8 +45,9 @@
 // the length fill the idle SMs, and nothing leaves the CTA unmerged.
 //
 // Every wait is bounded: when one runs out the CTA records where in the status
-// words, raises a shared abort flag that all other waits poll, drains its TMA
-// loads, frees its TMEM and returns.  (The MMA warp counts probes and leaves in silence.)
+// words, raises a shared abort flag that the other waits poll, drains its TMA
+// loads, frees its TMEM and returns.  (The MMA warp's waits do not poll it: they count
+// probes, and end within the same budget.)
 //
 // Semantics follow the reference prefix kernel (h3_shaders.metal:3061-3272):
 // scale applied to fp32 scores, P rounded to bf16 before P V, fp32 accumulate,
@@ -109,7 +110,7 @@ struct __align__(16) SharedControl {
     Mbar bars[kBarCount];
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
-    long long wait_cycles;  // budget of every bounded wait of this CTA
+    long long wait_cycles;  // budget of every bounded wait of this CTA but the MMA warp's
     int n_tiles[2];      // key tiles each sub-tile needs (by its largest limit)
     int warp_max[8];     // per softmax warp: largest limit
     int skip_lo, skip_hi;  // key tiles [skip_lo, skip_hi) lie inside the padding window
@@ -162,6 +163,7 @@ struct KernelParams {
     // so that the waits downstream of it run out and the CTA takes its clean exit.
     long long wait_cycles;
     int withhold_from;
+    int mma_probes;  // the same budget for the MMA warp's waits, in probes
 };
 
 // Bounded wait.  Returns false when the budget ran out here (recorded) or another thread
@@ -195,17 +197,17 @@ __device__ __forceinline__ bool mbar_wait(SharedControl *ctl, Mbar *bar,
     return mbar_wait_slow(ctl, bar, parity, status, where, tile);
 }
 
-// The wait of the MMA warp, for all its lanes at once, bounded by a number of probes: at least
-// 150 clocks each where one has to wait, 30 ms together, where a healthy wait is microseconds.
-// The warp issues every MMA of the CTA and each of its clocks is on the chain of both sub-tiles, so
-// the loop holds nothing else: with the clock, the abort flag and the record of the wait above
-// in it, text rows of 412 took 90 us a chain of six instead of 81, six heads 587 instead of
-// 572 us for eight layers, 24 heads of two 1738 instead of 1690 us for four.  When it runs out the
-// warp leaves in silence; the softmax, whose scores then stay away, records and raises the flag.
-constexpr int kMmaProbes = 400000;
-__device__ __forceinline__ bool mbar_wait_warp(Mbar *bar, uint32_t parity) {
+// The wait of the MMA warp, for all its lanes at once, bounded by a number of probes that the host
+// makes of the budget.  The warp issues every MMA of the CTA and each of its clocks is on the chain
+// of both sub-tiles, so the loop holds nothing else: with the clock and the abort flag of the wait
+// above behind 32 probes, in line or called, six heads take 633 to 658 instead of 571 us for eight
+// layers, 24 heads of two 1825 to 1890 instead of 1725 us for four.  A probe that fails suspends
+// the warp for a time that the hardware sets: 400 000 of them took 1.58 s, 7800 clocks each.
+constexpr long long kProbeCycles = 10000;
+__device__ __forceinline__ bool mbar_wait_warp(const KernelParams &p, Mbar *bar, uint32_t parity) {
     bool ok = false;
-    for (int i = 0; i < kMmaProbes && !ok; ++i) ok = mbar_try(bar, parity);
+#pragma unroll 1
+    for (int i = 0; i < p.mma_probes && !ok; ++i) ok = mbar_try(bar, parity);
     return __all_sync(0xffffffffu, ok) != 0;
 }
 
@@ -770,14 +772,11 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-        if (n_sub[i] > 0 &&
-            !mbar_wait_warp(&ctl->bars[kBarQFull + i], 0))
-            return;
+        if (n_sub[i] > 0 && !mbar_wait_warp(p, &ctl->bars[kBarQFull + i], 0)) return;
     {
         uint32_t slot = t % kStages, par = (t / kStages) & 1u;
         ++t;
-        if (!mbar_wait_warp(&ctl->bars[kBarKvFull + slot], par))
-            return;
+        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot], par)) return;
         tc_fence_after();
         const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescKMajor;
 #pragma unroll
@@ -800,26 +799,21 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             ++t;
         }
         QW_TRACE(2, 6, j);
-        if (!mbar_wait_warp(&ctl->bars[kBarKvFull + v_slot], v_par))
-            return;
+        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], v_par)) return;
         QW_TRACE(2, 7, j);
         const uint32_t v_lo = (kv_lo + v_slot * (kTileBytes >> 4)) | kDescLoVMajor;
         const uint32_t k_lo = (kv_lo + k_slot * (kTileBytes >> 4)) | kDescKMajor;
-        if (jn < n_max &&
-            !mbar_wait_warp(&ctl->bars[kBarKvFull + k_slot], k_par))
-            return;
+        if (jn < n_max && !mbar_wait_warp(p, &ctl->bars[kBarKvFull + k_slot], k_par)) return;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (j < n_sub[i]) {
-                if (!mbar_wait_warp(&ctl->bars[kBarPFirst + i], p_phase[i]))
-                    return;
+                if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i])) return;
                 tc_fence_after();
                 QW_TRACE(2, i, j);
                 if (elect_one())
                     issue_pv_first(o_tmem[i], s_tmem[i], v_lo, o_started[i], bounded);
                 __syncwarp();
-                if (!mbar_wait_warp(&ctl->bars[kBarPFull + i], p_phase[i]))
-                    return;
+                if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i])) return;
                 p_phase[i] ^= 1u;
                 tc_fence_after();
                 if (elect_one()) issue_pv_rest(o_tmem[i], s_tmem[i], v_lo, bounded);
@@ -872,14 +866,13 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
 #define QW_RING_WAIT(t_, lo_fixed_, out_)                                                       \
     {                                                                                           \
         const uint32_t slot_ = (t_) % kStages, par_ = ((t_) / kStages) & 1u;                    \
-        if (!mbar_wait_warp(&ctl->bars[kBarKvFull + slot_], par_))                           \
-            return;                                                                             \
+        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot_], par_)) return;                   \
         tc_fence_after();                                                                       \
         out_ = (kv_lo + slot_ * (kTileBytes >> 4)) | (lo_fixed_);                               \
     }
 #define QW_RING_FREE(t_) tc_commit<1>(&ctl->bars[kBarKvEmpty + ((t_) % kStages)])
 
-    if (!mbar_wait_warp(&ctl->bars[kBarQFull + 0], 0)) return;
+    if (!mbar_wait_warp(p, &ctl->bars[kBarQFull + 0], 0)) return;
     uint32_t desc;
     QW_RING_WAIT(pair_a(0, lb), kDescKMajor, desc);
     if (elect_one()) {
@@ -904,13 +897,11 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             if (s >= count) continue;
             const uint32_t t_now = i ? pair_b(s) : pair_a(s, lb);
             QW_RING_WAIT(t_now + 1, kDescLoVMajor, desc);
-            if (!mbar_wait_warp(&ctl->bars[kBarPFirst + i], p_phase[i]))
-                return;
+            if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i])) return;
             tc_fence_after();
             if (elect_one()) issue_pv_first(o_tmem[i], s_tmem[i], desc, s > 0, bounded);
             __syncwarp();
-            if (!mbar_wait_warp(&ctl->bars[kBarPFull + i], p_phase[i]))
-                return;
+            if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i])) return;
             p_phase[i] ^= 1u;
             tc_fence_after();
             if (elect_one()) {
@@ -1336,6 +1327,10 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
         p.out_head_offset = 0;
     }
     p.wait_cycles = a->wait_cycles;
+    // (At least 32 probes, like the other waits.  kProbeCycles is more than a probe takes: this
+    // role, which waits for the cause itself, gives up before those that wait behind it.)
+    const long long budget = p.wait_cycles > 0 ? p.wait_cycles : kWaitCycles;
+    p.mma_probes = 32 + (int)min(budget / kProbeCycles, 1ll << 30);
     p.withhold_from = a->withhold_from > 0 ? a->withhold_from : -1;
     p.slot_use = a->slot_use;
     p.n_freed = a->slot_use ? a->n_freed : 0;

@@ -289,7 +289,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 // ---- bounded waits ------------------------------------------------------------------
 // A wait that runs out records where in the status words and raises the CTA's abort
-// flag, which every other wait of the CTA polls; the roles then leave in order.
+// flag, which the other waits of the CTA poll (the attention's MMA warp counts probes
+// instead); the roles then leave in order.
 constexpr long long kWaitCycles = 400000000LL;  // about 0.2 s; a healthy wait is microseconds
 
 struct Waiter {

@@ -11,6 +11,7 @@ import dataclasses
 import math
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -685,6 +686,44 @@ def test_bounded_waits_run_out_cleanly(gpu, form, softmax):
     gates(gpu.read_bf16(ot, q.size), ref, f"after expired waits ({form}, {softmax})")
     for t in (qt, kt, vt, lt, ot, bt):
         gpu.free(t)
+
+
+@pytest.mark.parametrize("softmax", ["max", "bounded"])
+@pytest.mark.parametrize("form", ["sm100", "sm100-whole"])
+def test_an_expired_wait_ends_the_launch_within_its_budget(gpu, form, softmax):
+    """Every role honours the wait budget: a launch of one wave whose third key tile stays
+    away (2 000 000 cycles, about 1 ms) is over in milliseconds."""
+    lib = gpu.lib
+    S, H = 1024, 3  # 12 units: one wave in either form
+    zeros = np.zeros(S * H * 128, np.uint16)
+    qt, kt, vt, ot = (gpu.bf16(zeros) for _ in range(4))
+    lt, bt = gpu.u32(O.prefix_limits([(100, 0), (S - 100, 1)])), gpu.f32(np.ones(2, np.float32))
+
+    def chain():
+        """Result and duration of one launch; no assertion until the hook is off again."""
+        gpu.begin()
+        if softmax == "bounded":
+            ok = lib.qw_gpu_attn_block_causal_bounded_bf16(gpu.handle, ot, qt, kt, vt, lt, bt, 1, S, H, H,
+                                                           128, None, 0, SCALE)
+        else:
+            ok = lib.qw_gpu_attn_block_causal_bf16(gpu.handle, ot, qt, kt, vt, lt, 1, S, H, H, 128, None, 0,
+                                                   SCALE)
+        start = time.perf_counter()
+        return ok and lib.h3_gpu_submit(gpu.handle), time.perf_counter() - start
+
+    assert lib.qw_gpu_set_attention_kernel(gpu.handle, form.encode())
+    warm, _ = chain()
+    assert lib.qw_gpu_debug_attention_waits(gpu.handle, 2_000_000, 2)
+    expired, seconds = chain()
+    message = gpu.error()
+    assert lib.qw_gpu_debug_attention_waits(gpu.handle, 0, 0)
+    again, _ = chain()
+    for t in (qt, kt, vt, ot, lt, bt):
+        gpu.free(t)
+    assert warm and again and not expired and "wait ran out" in message, message
+    # One budget to expire and one more for what drains behind it are 2 ms; a role that does not
+    # know of the hook waits for the default budget, 0.2 s.
+    assert seconds < 0.05, f"the failing submit took {seconds:.3f} s"
 
 
 def test_scratch_cannot_grow_inside_a_graph_capture(gpu):
