@@ -166,6 +166,19 @@ struct KernelParams {
     int mma_probes;  // the same budget for the MMA warp's waits, in probes
 };
 
+// A wait ran out: the first one of the launch leaves its place in the status words, and the other
+// waits of the CTA end.
+__device__ __forceinline__ void record_expiry(SharedControl *ctl, uint32_t *status, uint32_t where,
+                                              uint32_t tile) {
+    ctl->abort_flag = 1;
+    if (atomicCAS(status, 0u, (uint32_t)QWCU_STATUS_WAIT_TIMEOUT) == 0u) {
+        status[1] = where;
+        status[2] = tile;
+        status[3] = blockIdx.x;
+    }
+    __threadfence();
+}
+
 // Bounded wait.  Returns false when the budget ran out here (recorded) or another thread
 // of the CTA already gave up.  (The GEMM's, out of line after a few probes, is not used
 // here: the softmax waits with its registers full.)
@@ -178,13 +191,7 @@ __device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, Mbar *bar,
             if (mbar_try(bar, parity)) return true;
         if (ctl->abort_flag) return false;
         if (clock64() - start > ctl->wait_cycles) {
-            ctl->abort_flag = 1;
-            if (atomicCAS(status, 0u, (uint32_t)QWCU_STATUS_WAIT_TIMEOUT) == 0u) {
-                status[1] = where;
-                status[2] = tile;
-                status[3] = blockIdx.x;
-            }
-            __threadfence();
+            record_expiry(ctl, status, where, tile);
             return false;
         }
     }
@@ -209,6 +216,14 @@ __device__ __forceinline__ bool mbar_wait_warp(const KernelParams &p, Mbar *bar,
 #pragma unroll 1
     for (int i = 0; i < p.mma_probes && !ok; ++i) ok = mbar_try(bar, parity);
     return __all_sync(0xffffffffu, ok) != 0;
+}
+
+// What the MMA warp does when one ran out, before it leaves.  It waits for what stayed away itself,
+// the softmax only for the scores behind it, so its record is the one that names the ring slot.  Out
+// of line, so that the loop around the waits does not grow.
+__device__ __noinline__ void mma_gave_up(SharedControl *ctl, uint32_t *status, uint32_t bar,
+                                         uint32_t tile) {
+    record_expiry(ctl, status, (2u << 16) | bar, tile);
 }
 
 // A value the compiler knows to be the same in all lanes of the (converged) warp.
@@ -772,11 +787,13 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-        if (n_sub[i] > 0 && !mbar_wait_warp(p, &ctl->bars[kBarQFull + i], 0)) return;
+        if (n_sub[i] > 0 && !mbar_wait_warp(p, &ctl->bars[kBarQFull + i], 0))
+            return mma_gave_up(ctl, p.status, kBarQFull + i, 0);
     {
         uint32_t slot = t % kStages, par = (t / kStages) & 1u;
         ++t;
-        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot], par)) return;
+        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot], par))
+            return mma_gave_up(ctl, p.status, kBarKvFull + slot, (uint32_t)j);
         tc_fence_after();
         const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescKMajor;
 #pragma unroll
@@ -799,21 +816,25 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             ++t;
         }
         QW_TRACE(2, 6, j);
-        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], v_par)) return;
+        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], v_par))
+            return mma_gave_up(ctl, p.status, kBarKvFull + v_slot, (uint32_t)j);
         QW_TRACE(2, 7, j);
         const uint32_t v_lo = (kv_lo + v_slot * (kTileBytes >> 4)) | kDescLoVMajor;
         const uint32_t k_lo = (kv_lo + k_slot * (kTileBytes >> 4)) | kDescKMajor;
-        if (jn < n_max && !mbar_wait_warp(p, &ctl->bars[kBarKvFull + k_slot], k_par)) return;
+        if (jn < n_max && !mbar_wait_warp(p, &ctl->bars[kBarKvFull + k_slot], k_par))
+            return mma_gave_up(ctl, p.status, kBarKvFull + k_slot, (uint32_t)jn);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (j < n_sub[i]) {
-                if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i])) return;
+                if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i]))
+                    return mma_gave_up(ctl, p.status, kBarPFirst + i, (uint32_t)j);
                 tc_fence_after();
                 QW_TRACE(2, i, j);
                 if (elect_one())
                     issue_pv_first(o_tmem[i], s_tmem[i], v_lo, o_started[i], bounded);
                 __syncwarp();
-                if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i])) return;
+                if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i]))
+                    return mma_gave_up(ctl, p.status, kBarPFull + i, (uint32_t)j);
                 p_phase[i] ^= 1u;
                 tc_fence_after();
                 if (elect_one()) issue_pv_rest(o_tmem[i], s_tmem[i], v_lo, bounded);
@@ -866,13 +887,15 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
 #define QW_RING_WAIT(t_, lo_fixed_, out_)                                                       \
     {                                                                                           \
         const uint32_t slot_ = (t_) % kStages, par_ = ((t_) / kStages) & 1u;                    \
-        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot_], par_)) return;                   \
+        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot_], par_))                           \
+            return mma_gave_up(ctl, p.status, kBarKvFull + slot_, (t_));                        \
         tc_fence_after();                                                                       \
         out_ = (kv_lo + slot_ * (kTileBytes >> 4)) | (lo_fixed_);                               \
     }
 #define QW_RING_FREE(t_) tc_commit<1>(&ctl->bars[kBarKvEmpty + ((t_) % kStages)])
 
-    if (!mbar_wait_warp(p, &ctl->bars[kBarQFull + 0], 0)) return;
+    if (!mbar_wait_warp(p, &ctl->bars[kBarQFull + 0], 0))
+        return mma_gave_up(ctl, p.status, kBarQFull + 0, 0);
     uint32_t desc;
     QW_RING_WAIT(pair_a(0, lb), kDescKMajor, desc);
     if (elect_one()) {
@@ -897,11 +920,13 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             if (s >= count) continue;
             const uint32_t t_now = i ? pair_b(s) : pair_a(s, lb);
             QW_RING_WAIT(t_now + 1, kDescLoVMajor, desc);
-            if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i])) return;
+            if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i]))
+                return mma_gave_up(ctl, p.status, kBarPFirst + i, (uint32_t)s);
             tc_fence_after();
             if (elect_one()) issue_pv_first(o_tmem[i], s_tmem[i], desc, s > 0, bounded);
             __syncwarp();
-            if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i])) return;
+            if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i]))
+                return mma_gave_up(ctl, p.status, kBarPFull + i, (uint32_t)s);
             p_phase[i] ^= 1u;
             tc_fence_after();
             if (elect_one()) {

@@ -10,6 +10,7 @@ import ctypes as C
 import dataclasses
 import math
 import os
+import re
 import subprocess
 import time
 
@@ -721,6 +722,10 @@ def test_an_expired_wait_ends_the_launch_within_its_budget(gpu, form, softmax):
     for t in (qt, kt, vt, ot, lt, bt):
         gpu.free(t)
     assert warm and again and not expired and "wait ran out" in message, message
+    # The record is the MMA warp's (role 2): it waits for the tile itself, the others for what
+    # lies behind it.  Barriers 2 to 5 are the four ring slots.
+    where = int(re.search(r"where (0x[0-9a-f]+)", message).group(1), 16)
+    assert where >> 16 == 2 and 2 <= where & 0xffff <= 5, message
     # One budget to expire and one more for what drains behind it are 2 ms; a role that does not
     # know of the hook waits for the default budget, 0.2 s.
     assert seconds < 0.05, f"the failing submit took {seconds:.3f} s"
