@@ -18,8 +18,8 @@
 // Mask: every row has an integer key limit (prefix) and the batch item may have
 // a key-padding window.  Key tiles past the largest limit of a sub-tile are
 // never issued, key tiles that lie completely inside the padding window are
-// skipped by all roles, interior tiles run without a compare, the scores of boundary
-// tiles are masked in TMEM first.
+// skipped by all roles, interior tiles run without a compare, boundary tiles have their
+// scores masked (see mask_scores).
 //
 // Epilogue: O / l is rounded to bf16 into the (by then dead) Q tile in shared
 // memory and leaves as TMA stores of the whole 128x128 tile.  When the heads
@@ -56,6 +56,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+
+#include <type_traits>
 
 #include "qw_sm100.cuh"
 
@@ -393,9 +395,23 @@ __device__ __forceinline__ uint32_t low_bits(int n) {
 // 32 scores of keys key0 .. key0 + 31: those the row does not see become -infinity.  The
 // row's mask is made once for the 32 keys and a score costs a bit test and a select, where
 // comparing its key with the limit and the padding window took three compares and a select.
-// The whole warp pays, on every tile, where text rows, which see few keys, share a block with
-// image rows, and the launch waits for it (six heads, 4352 rows, 64 of them text: 102 -> 78 us
-// with a bound, 115 -> 82 us without; with 256 text rows, a block of their own, 64 and 70 us).
+// (When every 32 keys carried the masks in line, six heads of 4352 rows, 64 of them text, went
+// from 102 to 78 us with a bound and from 115 to 82 us without.)
+//
+// Where text rows, which see few keys, share a block with image rows, their warps mask every tile
+// and the launch waits for them.  Tiles without a mask must not pay for it either: a branch in
+// every 32 keys costs 66 instead of 62 us where the 256 text rows have a block of their own.  Six
+// heads, 4352 rows, 64 / 256 of them text, us a launch:
+//                                        with a bound      without
+//   a branch in every 32 keys              79.5 / 66.4    83.8 / 71.5
+//   every masked tile by mask_tile         85.4 / 62.0    90.8 / 67.2
+//   as now                                 68.5 / 61.8    76.2 / 67.0
+// With a bound a tile's softmax stands twice in the code, with the masks in line and without.
+// Without one the 128 scores are in registers at once: rows that see nothing of a tile take one
+// select per score, and only tiles that some row sees a part of go through mask_tile.  A second
+// copy there is slower where launches are short, since each reads the code anew (six launches of
+// 412 text rows: 68.7 instead of 66.1 us), and so are the bits of all masks in registers (66.5 us,
+// 80 us with 64 text rows).
 __device__ __forceinline__ void mask_scores(uint32_t *s, int key0, int limit, int pad_lo, int pad_hi) {
     const uint32_t visible =
         low_bits(limit - key0) & ~(low_bits(pad_hi - key0) & ~low_bits(pad_lo - key0));
@@ -404,10 +420,7 @@ __device__ __forceinline__ void mask_scores(uint32_t *s, int key0, int limit, in
         s[i] = (visible & (1u << i)) ? s[i] : 0xff800000u;
 }
 
-// The masks of a tile, as a pass of their own over its scores in TMEM.  In line they cost every
-// tile, also the ones without a mask: the softmax of 128 keys beside the other sub-tile's took
-// 1850 clocks with the branch in each 32 keys and takes 1560 without (six heads, 4352 keys, 200
-// and more text rows: 597 -> 584 us for eight layers; 24 heads of two: 1743 -> 1705 us for four).
+// The masks of a tile, as a pass of their own over its scores in TMEM: a small loop.
 __device__ __forceinline__ void mask_tile(uint32_t tmem_s, int key0, int limit, int pad_lo, int pad_hi) {
 #pragma unroll 1
     for (int i = 0; i < kTileN; i += 32) {
@@ -465,32 +478,37 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
             const int key0 = j * kTileN;
             const bool pad_hit = pad_hi > pad_lo && key0 < pad_hi && key0 + kTileN > pad_lo;
             const bool boundary = __any_sync(0xffffffffu, key0 + kTileN > my_limit) || pad_hit;
-            if (boundary) mask_tile(tmem_s, key0, my_limit, pad_lo, pad_hi);
-            uint32_t sa[32], sb[32];
-            QW_TMEM_LD32(tmem_s, sa);
+            const auto softmax_tile = [&](auto masked) __attribute__((always_inline)) {
+                uint32_t sa[32], sb[32];
+                QW_TMEM_LD32(tmem_s, sa);
 #pragma unroll
-            for (int chunk = 0; chunk < 4; ++chunk) {
-                uint32_t(&cur)[32] = (chunk & 1) ? sb : sa;
-                uint32_t(&nxt)[32] = (chunk & 1) ? sa : sb;
-                QW_TMEM_WAIT_LD32(cur);
-                if (chunk == 0 && tid_in_group == 0) QW_TRACE(sub, 1, j);
-                if (chunk < 3) QW_TMEM_LD32(tmem_s + 32 * (chunk + 1), nxt);
-                uint32_t pk[16];
+                for (int chunk = 0; chunk < 4; ++chunk) {
+                    uint32_t(&cur)[32] = (chunk & 1) ? sb : sa;
+                    uint32_t(&nxt)[32] = (chunk & 1) ? sa : sb;
+                    QW_TMEM_WAIT_LD32(cur);
+                    if (chunk == 0 && tid_in_group == 0) QW_TRACE(sub, 1, j);
+                    if (chunk < 3) QW_TMEM_LD32(tmem_s + 32 * (chunk + 1), nxt);
+                    if constexpr (decltype(masked)::value)
+                        mask_scores(cur, key0 + chunk * 32, my_limit, pad_lo, pad_hi);
+                    uint32_t pk[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    float2 x = ffma2(make_float2(__uint_as_float(cur[2 * i]),
-                                                 __uint_as_float(cur[2 * i + 1])),
-                                     cs2, bias2);
-                    const float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                    if (i & 1) sum_b = fadd2(sum_b, pr);
-                    else sum_a = fadd2(sum_a, pr);
-                    pk[i] = pack_bf16(pr.x, pr.y);
+                    for (int i = 0; i < 16; ++i) {
+                        float2 x = ffma2(make_float2(__uint_as_float(cur[2 * i]),
+                                                     __uint_as_float(cur[2 * i + 1])),
+                                         cs2, bias2);
+                        const float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+                        if (i & 1) sum_b = fadd2(sum_b, pr);
+                        else sum_a = fadd2(sum_a, pr);
+                        pk[i] = pack_bf16(pr.x, pr.y);
+                    }
+                    if (chunk == kPartBounded / 2) publish_p_first(bar_p_first, tid_in_group);
+                    // P chunk c lands on columns [16c, 16c+16): scores already consumed.
+                    QW_TMEM_ST16(tmem_s + chunk * 16, pk);
+                    if (chunk == 1 && tid_in_group == 0) QW_TRACE(sub, 2, j);
                 }
-                if (chunk == kPartBounded / 2) publish_p_first(bar_p_first, tid_in_group);
-                // P chunk c lands on columns [16c, 16c+16): scores already consumed.
-                QW_TMEM_ST16(tmem_s + chunk * 16, pk);
-                if (chunk == 1 && tid_in_group == 0) QW_TRACE(sub, 2, j);
-            }
+            };
+            if (boundary) softmax_tile(std::true_type());
+            else softmax_tile(std::false_type());
             if (tid_in_group == 0) QW_TRACE(sub, 3, j);
             tmem_wait_st();
             tc_fence_before();
@@ -513,13 +531,22 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
         const int key0 = j * kTileN;
         const bool pad_hit = pad_hi > pad_lo && key0 < pad_hi && key0 + kTileN > pad_lo;
         const bool boundary = __any_sync(0xffffffffu, key0 + kTileN > my_limit) || pad_hit;
-        if (boundary) mask_tile(tmem_s, key0, my_limit, pad_lo, pad_hi);
+        // A row sees all of the tile, part of it (its limit or the padding window cuts it) or,
+        // like a text row beside image rows, nothing.
+        const bool cut =
+            __any_sync(0xffffffffu, (uint32_t)(my_limit - key0 - 1) < (uint32_t)(kTileN - 1)) || pad_hit;
+        if (cut) mask_tile(tmem_s, key0, my_limit, pad_lo, pad_hi);
         uint32_t s[128];
         QW_TMEM_LD32(tmem_s + 0, s + 0);
         QW_TMEM_LD32(tmem_s + 32, s + 32);
         QW_TMEM_LD32(tmem_s + 64, s + 64);
         QW_TMEM_LD32(tmem_s + 96, s + 96);
         tmem_wait_ld();
+        if (boundary && !cut) {
+            const bool unseen = key0 >= my_limit;
+#pragma unroll
+            for (int i = 0; i < kTileN; ++i) s[i] = unseen ? 0xff800000u : s[i];
+        }
         if (tid_in_group == 0) QW_TRACE(sub, 1, j);
 
         // Row maximum (four independent chains).

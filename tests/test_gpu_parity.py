@@ -510,6 +510,79 @@ def test_ragged_sizes_and_extreme_limits(gpu, kernel, rows):
         assert not out[1].any() and not out[2].any()
 
 
+@pytest.mark.parametrize("softmax", ["max", "bounded"])
+@pytest.mark.parametrize("text,length", [(31, 31), (47, 47), (64, 64), (100, 60), (200, 200)])
+def test_rows_of_a_warp_that_see_different_tiles(gpu, tail_form, text, length, softmax):
+    """Text rows and image rows in the warps of a block: of one key tile some rows of a warp see
+    all, some a part and some nothing.  Keys that a row does not see do not reach it, whatever
+    their scores are."""
+    S, H, lib = 650, 2, gpu.lib
+    rng = np.random.default_rng(text)
+    q, k, v = (randn_bf16(rng, (1, S, H, 128)) for _ in range(3))
+    limits, lens = O.prefix_limits([(text, 0), (S - text, 1)]), np.array([length], np.uint32)
+    pad = text if length < text else 0
+    lens_at = abi._ptr(lens) if pad else None
+
+    def attend(keys):
+        ts = [gpu.new_bf16(q.size), gpu.bf16(q), gpu.bf16(keys), gpu.bf16(v), gpu.u32(limits)]
+        gpu.begin()
+        if softmax == "bounded":
+            ts.append(gpu.f32(np.array([15.0, 15.0], np.float32)))  # N(0,1) rows: norms ~ 11.3 +- 0.7
+            gpu.check(lib.qw_gpu_attn_block_causal_bounded_bf16(gpu.handle, *ts, 1, S, H, H, 128, lens_at,
+                                                                pad, SCALE), "bounded")
+        else:
+            gpu.check(lib.qw_gpu_attn_block_causal_bf16(gpu.handle, *ts, 1, S, H, H, 128, lens_at, pad,
+                                                        SCALE), "block-causal")
+        gpu.submit()
+        out = gpu.read_bf16(ts[0], q.size).reshape(S, H * 128)
+        for t in ts:
+            gpu.free(t)
+        return out
+
+    got = attend(k)
+    ref, _ = O.sdpa(q, k, v, limits, 1, S, S, H, H, SCALE, lens if pad else None, pad)
+    gates(got, ref, f"text {text} of {length}, {softmax}")
+    poisoned = k.copy()
+    poisoned[:, text:text + 300:2] = 0x7F80      # infinity
+    poisoned[:, text + 1:text + 300:2] = 0x7FC0  # NaN
+    assert np.array_equal(attend(poisoned)[:text], got[:text])
+
+
+@pytest.mark.parametrize("softmax", ["max", "bounded"])
+def test_text_rows_in_a_block_with_image_rows_do_not_hold_it_up(gpu, softmax):
+    """A block whose first warps hold text rows masks every key tile.  It took 1.2 times an
+    image block, 1.35 to 1.38 times with the masks as a pass of their own over every such
+    tile, and takes 1.10 (bounded) and 1.15 times; the limit lies between."""
+    S, H, lib = 4352, 6, gpu.lib  # one partly filled wave: the slowest block is the launch
+    q = randn_bf16(np.random.default_rng(0), (1, S, H, 128))
+    ts = [gpu.new_bf16(q.size), gpu.bf16(q), gpu.bf16(q), gpu.bf16(q)]
+    bound = gpu.f32(np.array([15.0, 15.0], np.float32))
+
+    def seconds(text):
+        limits = gpu.u32(O.prefix_limits([(text, 0), (S - text, 1)]))
+        best = math.inf
+        for _ in range(12):
+            before = gpu.stats().gpu_seconds
+            gpu.begin()
+            for _ in range(8):
+                if softmax == "bounded":
+                    ok = lib.qw_gpu_attn_block_causal_bounded_bf16(gpu.handle, *ts, limits, bound, 1, S, H, H,
+                                                                   128, None, 0, SCALE)
+                else:
+                    ok = lib.qw_gpu_attn_block_causal_bf16(gpu.handle, *ts, limits, 1, S, H, H, 128, None, 0,
+                                                           SCALE)
+                gpu.check(ok, "attention")
+            gpu.submit()
+            best = min(best, gpu.stats().gpu_seconds - before)
+        gpu.free(limits)
+        return best
+
+    shared, own = seconds(47), seconds(256)  # 256 text rows are a block of their own
+    for t in [*ts, bound]:
+        gpu.free(t)
+    assert shared < 1.26 * own, f"{shared * 1e6 / 8:.1f} us beside {own * 1e6 / 8:.1f} us"
+
+
 def test_key_padding_extremes(gpu, kernel):
     """text_len = 0 (whole window padded), = text_pad (nothing padded) and a
     window that is not tile aligned."""
