@@ -21,9 +21,18 @@
 // Optional fused epilogue (q and k of the DiT block): a thread owns one row of a head
 // of 128 columns, so the per-head RMSNorm needs no exchange between threads and
 // follows the reference's serial fma order exactly; the interleaved RoPE follows with
-// the row's cos/sin.  The bf16 roundings the reference has between its three kernels
+// the rows' cos/sin.  The bf16 roundings the reference has between its three kernels
 // are reproduced, which makes the result the same as GEMM -> h3_gpu_head_rms_norm_bf16
 // -> qw_gpu_qk_rope_bf16 without the two extra passes over q and k.
+//
+// Where a CTA has one tile, nothing hides its epilogue, and most of that was latency: of
+// cos/sin, which every thread read for its own row (32 lines a load, twice what L1 holds),
+// and of code that each launch reads anew.  So the rotation runs on the staged box, where
+// eight lanes share a row's line and the loads are issued under the main loop, the
+// loops are rolled (a row's columns are read from TMEM twice instead of being held), and the
+// last tile's second box is staged in the ring instead of waiting for the first one's store.
+// 320 rows of 3072, clocks from complete accumulator to stores issued: 12700 -> 3700; chains of
+// four layers, 256^2 301 -> 283 us, 512^2 487 -> 472 us.
 //
 // Every wait is bounded (status words, abort flag).  A CTA leaves nothing in flight, also
 // after a wait has run out: see the end of the kernel.
@@ -61,7 +70,7 @@ struct __align__(16) Control {
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
     uint32_t issued[2];  // of the pair's CTAs: K steps loaded, kGaveUp when a wait ran out
-    float norm_w[2][128];
+    alignas(16) float norm_w[2][128];
 };
 constexpr uint32_t kGaveUp = 0x80000000u;
 
@@ -82,6 +91,7 @@ struct Params {
     uint32_t n_each;             // columns of every output
     uint32_t tiles_per_output;   // ceil(n_each / kN)
     uint32_t m_tiles, n_tiles;   // n_tiles over all outputs
+    uint32_t n_outputs;
     uint32_t band;               // M tiles that run side by side
     uint32_t whole, items;       // items [0, whole) are tiles, the rest half tiles (kN / 2 columns)
     const uint16_t *bias[kMaxOutputs];  // bf16 [n_each] or null
@@ -91,7 +101,7 @@ struct Params {
     // roundings between the stages (GEMM result -> bf16 -> norm -> bf16 -> rotation).
     const uint16_t *norm_weight[2];    // bf16 [128] each, null = plain output
     const float *rope_cos, *rope_sin;  // f32 [table_rows][64]
-    uint32_t table_rows;               // table row = output row % table_rows
+    uint32_t table_rows, table_step;   // table row = output row % table_rows; 4 % table_rows
     float epsilon;
     float *bound_out;  // optional: [0], [1] = bounds of the 2-norm of any q row, k row
     // Bounded-wait exercise (tests only): budget in SM cycles, and the K step (counted over
@@ -135,55 +145,22 @@ __device__ __forceinline__ Item item_at(const Params &p, uint32_t i) {
     return it;
 }
 
-// 64 * kBoxes columns of one row out of the accumulator, as packed bf16 pairs: the GEMM
-// result rounded to bf16 (plus bias), and for a whole head of q / k (kBoxes == 2) the
-// per-head RMSNorm and the rotation on top, each stage rounded to bf16 like the
-// reference's kernels.
-template <int kBoxes>
-__device__ __forceinline__ void row_from_tmem(uint32_t (&pk)[64], uint32_t taddr, const uint16_t *bias,
-                                              uint32_t bias_cols, const float *norm_w,
-                                              const float *cos_row, const float *sin_row,
-                                              float epsilon) {
-    float ss = 0.0f;
+// 32 columns of one row out of the accumulator, as packed bf16 pairs: the GEMM result
+// (plus bias) rounded to bf16.
+__device__ __forceinline__ void row_from_tmem(uint32_t (&pk)[16], uint32_t taddr, const uint16_t *bias,
+                                              uint32_t bias_cols) {
+    uint32_t o[32];
+    tmem_ld32(o, taddr);
+    tmem_wait_ld32(o);
 #pragma unroll
-    for (int c = 0; c < 2 * kBoxes; ++c) {
-        uint32_t o[32];
-        tmem_ld32(o, taddr + (uint32_t)(c * 32));
-        tmem_wait_ld32(o);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float lo = __uint_as_float(o[2 * i]), hi = __uint_as_float(o[2 * i + 1]);
-            if (bias && (uint32_t)(c * 32 + 2 * i) < bias_cols) {  // (column counts are even)
-                const uint32_t b2 = *reinterpret_cast<const uint32_t *>(bias + c * 32 + 2 * i);
-                lo = __fadd_rn(lo, bf16_lo(b2));
-                hi = __fadd_rn(hi, bf16_hi(b2));
-            }
-            const uint32_t w = pack_bf16(lo, hi);
-            pk[c * 16 + i] = w;
-            if (kBoxes == 2 && norm_w) {  // serial fma over the bf16 values, element order 0..127
-                ss = fmaf(bf16_lo(w), bf16_lo(w), ss);
-                ss = fmaf(bf16_hi(w), bf16_hi(w), ss);
-            }
+    for (int i = 0; i < 16; ++i) {
+        float lo = __uint_as_float(o[2 * i]), hi = __uint_as_float(o[2 * i + 1]);
+        if (bias && (uint32_t)(2 * i) < bias_cols) {  // (column counts are even)
+            const uint32_t b2 = *reinterpret_cast<const uint32_t *>(bias + 2 * i);
+            lo = __fadd_rn(lo, bf16_lo(b2));
+            hi = __fadd_rn(hi, bf16_hi(b2));
         }
-    }
-    if (kBoxes != 2 || !norm_w) return;
-    const float inverse = 1.0f / sqrtf(__fadd_rn(ss / 128.0f, epsilon));
-#pragma unroll
-    for (int q4 = 0; q4 < 16; ++q4) {  // four rotation pairs at a time
-        const float4 c4 = *reinterpret_cast<const float4 *>(cos_row + 4 * q4);
-        const float4 s4 = *reinterpret_cast<const float4 *>(sin_row + 4 * q4);
-        const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int pair = 4 * q4 + u;
-            const uint32_t w = pk[pair];
-            // n = bf16(x * inv * w), stored as bf16 between the norm and the rotation
-            const uint32_t n = pack_bf16(__fmul_rn(__fmul_rn(bf16_lo(w), inverse), norm_w[2 * pair]),
-                                         __fmul_rn(__fmul_rn(bf16_hi(w), inverse), norm_w[2 * pair + 1]));
-            const float e = bf16_lo(n), o = bf16_hi(n);
-            pk[pair] = pack_bf16(__fsub_rn(__fmul_rn(e, cc[u]), __fmul_rn(o, sn[u])),
-                                 __fadd_rn(__fmul_rn(e, sn[u]), __fmul_rn(o, cc[u])));
-        }
+        pk[i] = pack_bf16(lo, hi);
     }
 }
 
@@ -212,18 +189,26 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
         }
         ctl->abort_flag = 0;
         mbar_init_fence();
-        tma_prefetch(&maps.a);
     }
-    if (warp == 1) tmem_alloc<kGroup>(&ctl->tmem_base, C::kTmemCols);
-    tc_fence_before();
-    if constexpr (kGroup == 2) {
-        __syncwarp();
-        cluster_sync();  // the peer's barriers exist before anything is reported to them
-    } else {
-        __syncthreads();
+    // (parameters, not memory that a kernel before this one writes)
+    if (warp == 2) {
+        if (lane == 0) tma_prefetch(&maps.a);
+        else if ((uint32_t)lane <= p.n_outputs) tma_prefetch(&maps.w[lane - 1]);
+        else if ((uint32_t)lane <= 2 * p.n_outputs) tma_prefetch(&maps.c[lane - 1 - p.n_outputs]);
     }
-    tc_fence_after();
-    const uint32_t tmem = ctl->tmem_base;
+    // The producer may start as soon as the barriers exist, the peer's too, to which it
+    // reports; the others wait for TMEM as well.
+    __syncwarp();
+    if constexpr (kGroup == 2) cluster_sync();
+    else __syncthreads();
+    uint32_t tmem = 0;
+    if (warp != 0) {
+        if (warp == 1) tmem_alloc<kGroup>(&ctl->tmem_base, C::kTmemCols);
+        tc_fence_before();
+        asm volatile("bar.sync 2, %0;" ::"n"(kThreads - 32) : "memory");
+        tc_fence_after();
+        tmem = ctl->tmem_base;
+    }
     grid_launch_dependents();
     grid_wait();
 
@@ -320,7 +305,6 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
         const uint32_t quarter = (uint32_t)(warp & 3);
         const uint32_t lanes = tmem + ((quarter * 32u) << 16);
         uint8_t *stage = staging + ew * kStoreBytes;
-        uint8_t *line = stage + lane * 128;
         const uint32_t sw = (uint32_t)lane & 7u;
         if (p.norm_weight[0] || p.norm_weight[1]) {
             // norm weights of q and k as floats, shared by all rows
@@ -346,10 +330,6 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
         for (uint32_t i = first; i < p.items; i += step, ++local) {
             const Item it = item_at<kN>(p, i);
             const uint32_t acc = local & 1u;
-            if (!mbar_wait_warp(wait, &ctl->bars[kBarAccFull + acc], (local >> 1) & 1u,
-                                (1u << 16) | (kBarAccFull + acc), i))
-                break;
-            tc_fence_after();
             const bool fused = it.which < 2 && p.norm_weight[it.which] != nullptr;
             // columns of this warp: 128 of a 256-column tile; a narrower one is shared out
             // in boxes of 64, except that a head to be normalised stays in one thread
@@ -357,45 +337,118 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
             const uint32_t off = (uint32_t)group * (wide ? 128u : 64u);
             const uint32_t col0 = it.col0 + off;
             const uint32_t row0 = (it.tm * kGroup + rank) * kRows + quarter * 32u;
-            const bool mine = off < it.cols;
-            uint32_t pk[64];
-            if (mine) {
-                const uint32_t row = row0 + (uint32_t)lane;
-                const uint32_t table_row = (row < p.m ? row : 0u) % p.table_rows;
-                const uint16_t *bias = p.bias[it.which] && col0 < p.n_each ? p.bias[it.which] + col0 : nullptr;
-                const uint32_t src = lanes + acc * kN + off;
-                if (wide)
-                    row_from_tmem<2>(pk, src, bias, p.n_each - col0, fused ? ctl->norm_w[it.which] : nullptr,
-                                     fused ? p.rope_cos + (size_t)table_row * 64 : nullptr,
-                                     fused ? p.rope_sin + (size_t)table_row * 64 : nullptr, p.epsilon);
-                else
-                    row_from_tmem<1>(pk, src, bias, p.n_each - col0, nullptr, nullptr, nullptr, 0.0f);
+            // The second box of a CTA's last tile is staged in the ring, which is done with.
+            uint8_t *const spare = i + step < p.items ? stage : ring + ew * kStoreBytes;
+            const int boxes = off >= it.cols || row0 >= p.m ? 0 : wide ? 2 : 1;
+            // (the last columns of the last tile may lie past the output's)
+            const int live = boxes == 2 && col0 + 64u >= p.n_each ? 1 : col0 >= p.n_each ? 0 : boxes;
+            // The rotation's entries of a box: lane l takes four pairs (16 bytes of cos and of
+            // sin) of rows l / 8, l / 8 + 4, ..., so that a load touches four rows' lines and not
+            // 32.  The first box's are on their way while the accumulator is still filling.
+            float4 cs[8], sn[8];
+            uint32_t table_row = 0;
+            const auto load_table = [&](int i, int box) {
+                const size_t at =
+                    (size_t)(row0 + 4u * i + ((uint32_t)lane >> 3) < p.m ? table_row : 0u) * 64 + box * 32 +
+                    4 * (lane & 7);
+                cs[i] = __ldg(reinterpret_cast<const float4 *>(p.rope_cos + at));
+                sn[i] = __ldg(reinterpret_cast<const float4 *>(p.rope_sin + at));
+                table_row += p.table_step;
+                if (table_row >= p.table_rows) table_row -= p.table_rows;
+            };
+            if (fused && live) {
+                table_row = (row0 + ((uint32_t)lane >> 3)) % p.table_rows;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) load_table(i, 0);
+            }
+            if (!mbar_wait_warp(wait, &ctl->bars[kBarAccFull + acc], (local >> 1) & 1u,
+                                (1u << 16) | (kBarAccFull + acc), i))
+                break;
+            tc_fence_after();
+            const uint32_t src = lanes + acc * kN + off;
+            const uint16_t *bias = p.bias[it.which] ? p.bias[it.which] + col0 : nullptr;
+            float inverse = 0.0f;
+            if (fused && live) {  // serial fma over the bf16 values, element order 0..127
+                float ss = 0.0f;
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t pk[16];
+                    row_from_tmem(pk, src + (uint32_t)(c * 32), bias ? bias + c * 32 : nullptr, 32);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        ss = fmaf(bf16_lo(pk[j]), bf16_lo(pk[j]), ss);
+                        ss = fmaf(bf16_hi(pk[j]), bf16_hi(pk[j]), ss);
+                    }
+                }
+                inverse = 1.0f / sqrtf(__fadd_rn(ss / 128.0f, p.epsilon));
+            }
+#pragma unroll 1
+            for (int box = 0; box < live; ++box) {
+                uint8_t *const staged = box ? spare : stage;
+                if (staged == stage) {
+                    if (lane == 0) tma_store_wait_read<0>();
+                    __syncwarp();
+                }
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    const uint32_t at = (uint32_t)(box * 64 + half * 32);
+                    uint32_t pk[16];
+                    row_from_tmem(pk, src + at, bias ? bias + at : nullptr,
+                                  col0 + at < p.n_each ? p.n_each - col0 - at : 0u);
+                    if (fused) {  // bf16(x * inv * w), stored as bf16 between norm and rotation
+                        const float4 *w4 = reinterpret_cast<const float4 *>(&ctl->norm_w[it.which][at]);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float4 w = w4[j];
+                            pk[2 * j] = pack_bf16(__fmul_rn(__fmul_rn(bf16_lo(pk[2 * j]), inverse), w.x),
+                                                  __fmul_rn(__fmul_rn(bf16_hi(pk[2 * j]), inverse), w.y));
+                            pk[2 * j + 1] =
+                                pack_bf16(__fmul_rn(__fmul_rn(bf16_lo(pk[2 * j + 1]), inverse), w.z),
+                                          __fmul_rn(__fmul_rn(bf16_hi(pk[2 * j + 1]), inverse), w.w));
+                        }
+                    }
+#pragma unroll
+                    for (int c16 = 0; c16 < 4; ++c16)
+                        *reinterpret_cast<uint4 *>(staged + lane * 128 +
+                                                   (((uint32_t)(half * 4 + c16) ^ sw) << 4)) =
+                            make_uint4(pk[4 * c16], pk[4 * c16 + 1], pk[4 * c16 + 2], pk[4 * c16 + 3]);
+                }
+                if (fused) {
+                    // The rotation, in place: a lane has the pairs its table entries are for.
+                    __syncwarp();
+                    if (box == 0 && live == 2) table_row = (row0 + ((uint32_t)lane >> 3)) % p.table_rows;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t r = 4u * i + ((uint32_t)lane >> 3);
+                        uint4 *at = reinterpret_cast<uint4 *>(
+                            staged + r * 128 + ((((uint32_t)lane & 7u) ^ (r & 7u)) << 4));
+                        const uint4 x = *at;
+                        const uint32_t n[4] = {x.x, x.y, x.z, x.w};
+                        const float cc[4] = {cs[i].x, cs[i].y, cs[i].z, cs[i].w};
+                        const float ss[4] = {sn[i].x, sn[i].y, sn[i].z, sn[i].w};
+                        uint32_t y[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float e = bf16_lo(n[j]), o = bf16_hi(n[j]);
+                            y[j] = pack_bf16(__fsub_rn(__fmul_rn(e, cc[j]), __fmul_rn(o, ss[j])),
+                                             __fadd_rn(__fmul_rn(e, ss[j]), __fmul_rn(o, cc[j])));
+                        }
+                        *at = make_uint4(y[0], y[1], y[2], y[3]);
+                        if (box + 1 < live) load_table(i, box + 1);
+                    }
+                }
+                fence_async_shared();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&maps.c[it.which], staged, (int)(col0 + box * 64), (int)row0);
+                    tma_store_commit();
+                }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {  // this warp's part of the accumulator has left TMEM
                 if constexpr (kGroup == 2) mbar_arrive_at(map_to_rank(&ctl->bars[kBarAccEmpty + acc], 0));
                 else mbar_arrive(&ctl->bars[kBarAccEmpty + acc]);
-            }
-            if (!mine || row0 >= p.m) continue;
-#pragma unroll
-            for (int box = 0; box < 2; ++box) {
-                if (box == 1 && !wide) break;
-                if (col0 + (uint32_t)box * 64u >= p.n_each) break;
-                if (lane == 0) tma_store_wait_read<0>();
-                __syncwarp();
-#pragma unroll
-                for (int c16 = 0; c16 < 8; ++c16) {
-                    const int w0 = box * 32 + c16 * 4;
-                    *reinterpret_cast<uint4 *>(line + (((uint32_t)c16 ^ sw) << 4)) =
-                        make_uint4(pk[w0], pk[w0 + 1], pk[w0 + 2], pk[w0 + 3]);
-                }
-                fence_async_shared();
-                __syncwarp();
-                if (lane == 0) {
-                    tma_store_2d(&maps.c[it.which], stage, (int)(col0 + box * 64), (int)row0);
-                    tma_store_commit();
-                }
             }
         }
         if (lane == 0) tma_store_wait_read<0>();
@@ -540,6 +593,7 @@ extern "C" int qwcu_linear_sm100_launch(const qwcu_linear_args *a, int sm_count,
     p.m = a->m;
     p.k = a->k;
     p.n_each = a->n;
+    p.n_outputs = a->n_outputs;
     p.tiles_per_output = choice.tiles_per_output;
     p.m_tiles = choice.m_tiles;
     p.n_tiles = choice.n_tiles;
@@ -552,6 +606,7 @@ extern "C" int qwcu_linear_sm100_launch(const qwcu_linear_args *a, int sm_count,
     p.rope_cos = a->rope_cos;
     p.rope_sin = a->rope_sin;
     p.table_rows = a->table_rows ? a->table_rows : 1;
+    p.table_step = 4u % p.table_rows;
     p.epsilon = a->epsilon;
     p.bound_out = a->bound_out;
     p.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kWaitCycles;

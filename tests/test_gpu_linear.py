@@ -125,3 +125,33 @@ def test_qkv_and_fused_norm_rope_epilogue(gpu, batch, seq, dim):
     assert np.sqrt((bf16_to_f32(fk).astype(np.float64) ** 2).sum(-1)).max() <= bound[1]
     for t in [xt, wqt, wkt, ct, st, bt] + wts + plain + fused:
         gpu.free(t)
+
+
+@pytest.mark.parametrize("batch,seq,dim", [(301, 1, 256), (67, 3, 256), (29, 5, 384), (5, 33, 128)])
+def test_fused_epilogue_where_the_table_repeats_inside_a_tile(gpu, batch, seq, dim):
+    """Rows take the rotation's entries modulo the table, which here is shorter than the 4 rows
+    a load covers, or than the 32 of a staged box: bit for bit, ragged last boxes included."""
+    rng = np.random.default_rng(batch)
+    lib = gpu.lib
+    rows, heads = batch * seq, dim // 128
+    x = workloads.normal_bf16(rng, (rows, dim))
+    ws = [weights(rng, dim, dim) for _ in range(3)]
+    wq, wk = workloads.normal_bf16(rng, (128,), 1.0, 0.1), workloads.normal_bf16(rng, (128,), 1.0, 0.1)
+    angle = rng.uniform(-3, 3, (seq, 64))
+    cos, sin = np.cos(angle).astype(np.float32), np.sin(angle).astype(np.float32)
+    ins = [gpu.bf16(x)] + [gpu.bf16(w) for w in ws]
+    plain, fused = ([gpu.new_bf16(rows * dim) for _ in range(3)] for _ in range(2))
+    rest = [gpu.bf16(wq), gpu.bf16(wk), gpu.f32(cos), gpu.f32(sin), gpu.new_f32(2)]
+    gpu.begin()
+    gpu.check(lib.qw_gpu_qkv_bf16(gpu.handle, *plain, *ins, rows, dim), "qkv")
+    gpu.check(lib.qw_gpu_qkv_norm_rope_bf16(gpu.handle, *fused, *ins, *rest, batch, seq, dim, 1e-6),
+              "qkv norm rope")
+    gpu.submit()
+    got = [gpu.read_bf16(t, rows * dim) for t in plain]
+    qn = O.head_rms_norm(got[0].reshape(rows, heads, 128), wq, rows, heads, 1e-6)
+    kn = O.head_rms_norm(got[1].reshape(rows, heads, 128), wk, rows, heads, 1e-6)
+    want_q, want_k = O.qk_rope(qn, kn, np.tile(cos, (batch, 1)), np.tile(sin, (batch, 1)), rows, heads)
+    for t, want in zip(fused, (want_q, want_k, got[2].reshape(rows, heads, 128))):
+        assert np.array_equal(gpu.read_bf16(t, rows * dim).reshape(rows, heads, 128), want)
+    for t in ins + plain + fused + rest:
+        gpu.free(t)
