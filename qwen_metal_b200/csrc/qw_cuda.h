@@ -71,7 +71,7 @@ typedef struct {
     uint32_t n_out_peers;
     uint32_t out_heads_total;
     uint32_t out_head_offset;
-    uint32_t *status; /* QWCU_STATUS_WORDS device words, zero when healthy */
+    uint32_t *status; /* QWCU_STATUS_WORDS words, zero when healthy */
     /* Sharded heads with the gather as a separate push (cuda/qw_push.cu): at its
      * start the kernel increments *slot_use and stores the new epoch into
      * freed_peer[0..n_freed) (peer-mapped flag words): the peers may now store

@@ -24,8 +24,8 @@ struct h3_gpu {
     uint64_t kernel_launches;
     cudaEvent_t chain_start, chain_stop;
     double chain_start_wall;
-    uint32_t *status_dev;  /* QWCU_STATUS_WORDS words, zero when healthy */
-    uint32_t *status_host; /* pinned mirror */
+    uint32_t *status_host; /* QWCU_STATUS_WORDS words in pinned host memory, zero when healthy */
+    uint32_t *status_dev;  /* the same words as the device addresses them */
     int attn_kernel;
     long long attn_wait_cycles; /* tests: budget of the attention kernel's waits (0 = default) */
     int attn_withhold_tile;     /* tests: first key tile the producer leaves out (0 = none) */
