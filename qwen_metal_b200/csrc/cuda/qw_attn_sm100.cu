@@ -82,10 +82,9 @@ static_assert(2 * 128 * kSoftmaxRegs + 128 * kOtherRegs <= kThreads * kLaunchReg
               "setmaxnreg budget exceeds the launch allocation");
 // P of a tile is published in two parts, the first kPart * 16 keys and the rest: P V of
 // the first part runs under the softmax of the rest, which takes it out of the chain
-// S -> softmax -> P V -> next S that bounds the kernel.  With the fixed exponent the later
-// cut is the better one (six heads, 4352 keys: 622 us with 4, 601 us with 6), with the
-// running maximum the earlier (8188 x 8211 keys: 1018 us with 4, 1079 us with 6).
-constexpr int kPartRunning = 4, kPartBounded = 6;
+// S -> softmax -> P V -> next S that bounds the kernel (six heads, 4352 keys, with a bound:
+// 622 us with 4, 601 us with 6; 8188 x 8211 keys without one: 980 us with 4, 955 us with 6).
+constexpr int kPart = 6;
 constexpr int kSoftmaxThreads = 256;
 constexpr int kMmaWarp = 8;
 constexpr int kTmaWarp = 9;
@@ -501,7 +500,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
                         else sum_a = fadd2(sum_a, pr);
                         pk[i] = pack_bf16(pr.x, pr.y);
                     }
-                    if (chunk == kPartBounded / 2) publish_p_first(bar_p_first, tid_in_group);
+                    if (chunk == kPart / 2) publish_p_first(bar_p_first, tid_in_group);
                     // P chunk c lands on columns [16c, 16c+16): scores already consumed.
                     QW_TMEM_ST16(tmem_s + chunk * 16, pk);
                     if (chunk == 1 && tid_in_group == 0) QW_TRACE(sub, 2, j);
@@ -605,7 +604,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
                 else sum_a = fadd2(sum_a, pr);
                 pk[i] = pack_bf16(pr.x, pr.y);
             }
-            if (chunk == kPartRunning / 2) publish_p_first(bar_p_first, tid_in_group);
+            if (chunk == kPart / 2) publish_p_first(bar_p_first, tid_in_group);
             QW_TMEM_ST16(tmem_s + chunk * 16, pk);
         }
         if (tid_in_group == 0) QW_TRACE(sub, 3, j);
@@ -780,20 +779,8 @@ __device__ __forceinline__ void issue_pv_keys(uint32_t d_tmem, uint32_t p_tmem, 
     }
 }
 
-// The two parts P V is issued in, as the softmax publishes them.
-__device__ __forceinline__ void issue_pv_first(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo,
-                                               bool accumulate, bool bounded) {
-    if (bounded) issue_pv_keys<0, kPartBounded>(d_tmem, p_tmem, v_lo, accumulate);
-    else issue_pv_keys<0, kPartRunning>(d_tmem, p_tmem, v_lo, accumulate);
-}
-__device__ __forceinline__ void issue_pv_rest(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo,
-                                              bool bounded) {
-    if (bounded) issue_pv_keys<kPartBounded, 8>(d_tmem, p_tmem, v_lo, true);
-    else issue_pv_keys<kPartRunning, 8>(d_tmem, p_tmem, v_lo, true);
-}
-
 __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *ctl,
-                                         uint8_t *smem_q, uint8_t *smem_kv, bool bounded) {
+                                         uint8_t *smem_q, uint8_t *smem_kv) {
     // Whole form: both sub-tiles walk the visited tiles from 0; u counts them.
     const int n0 = uniform(ctl->tile_count[0]), n1 = uniform(ctl->tile_count[1]);
     const int n_max = max(n0, n1);
@@ -801,94 +788,100 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
     if (j >= n_max) return;
     const uint32_t tmem = uniform(ctl->tmem_base);
     // Low descriptor words: start address in 16-byte units plus the fixed LBO field.
-    const uint32_t q_lo[2] = {(smem_u32(smem_q) >> 4) | kDescKMajor,
-                              (smem_u32(smem_q + kTileBytes) >> 4) | kDescKMajor};
+    const uint32_t q_lo = (smem_u32(smem_q) >> 4) | kDescKMajor;  // sub-tile 1's is one tile further
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;  // slot s starts (s * kTileBytes) >> 4 further
-    const uint32_t s_tmem[2] = {tmem + kTmemS0, tmem + kTmemS1};
-    const uint32_t o_tmem[2] = {tmem + kTmemO0, tmem + kTmemO1};
-    const int n_sub[2] = {n0, n1};
-    uint32_t p_phase[2] = {0, 0};
-    bool o_started[2] = {false, false};
     uint32_t t = 0;  // ring position (K and V tiles alternate)
     [[maybe_unused]] uint32_t trace_cursor = 0;
 
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-        if (n_sub[i] > 0 && !mbar_wait_warp(p, &ctl->bars[kBarQFull + i], 0))
-            return mma_gave_up(ctl, p.status, kBarQFull + i, 0);
     {
-        uint32_t slot = t % kStages, par = (t / kStages) & 1u;
-        ++t;
-        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot], par))
+        const uint32_t slot = t++ % kStages;
+        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot], 0))
             return mma_gave_up(ctl, p.status, kBarKvFull + slot, (uint32_t)j);
-        tc_fence_after();
         const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescKMajor;
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (j < n_sub[i] && elect_one()) {
-                issue_qk(s_tmem[i], q_lo[i], k_lo);
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) {
+            if (j >= (i ? n1 : n0)) continue;
+            if (!mbar_wait_warp(p, &ctl->bars[kBarQFull + i], 0))
+                return mma_gave_up(ctl, p.status, kBarQFull + i, 0);
+            tc_fence_after();
+            if (elect_one()) {
+                issue_qk(tmem + kTmemS0 + (uint32_t)i * kTileN,
+                         q_lo + (uint32_t)i * (kTileBytes >> 4), k_lo);
                 tc_commit<1>(&ctl->bars[kBarSFull + i]);
             }
+            __syncwarp();
+        }
         if (elect_one()) tc_commit<1>(&ctl->bars[kBarKvEmpty + slot]);
         __syncwarp();
     }
+    uint32_t v_slot = t++ % kStages;
+    if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], 0))
+        return mma_gave_up(ctl, p.status, kBarKvFull + v_slot, (uint32_t)j);
+    // The tensor cores take four MMAs ahead, about 150 clocks of work, and a wait costs this warp 60
+    // to 110 even where nothing is left to wait for.  So the next tiles of K and of V are waited
+    // for behind the first parts of P V, where the warp waits for the rest of P anyway, and not both
+    // in front of the step; and the two sub-tiles take turns in one loop, whose code is half as long.
+    // Eight layers of six heads, 4352 keys: 560 us before, 552 us.
     while (j < n_max) {
         const int jn = j + 1;
-        uint32_t v_slot = t % kStages, v_par = (t / kStages) & 1u;
-        ++t;
-        uint32_t k_slot = 0, k_par = 0;
-        if (jn < n_max) {
-            k_slot = t % kStages;
-            k_par = (t / kStages) & 1u;
-            ++t;
-        }
-        QW_TRACE(2, 6, j);
-        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], v_par))
-            return mma_gave_up(ctl, p.status, kBarKvFull + v_slot, (uint32_t)j);
-        QW_TRACE(2, 7, j);
+        const bool more = jn < n_max;
+        const uint32_t k_slot = t % kStages, k_par = (t / kStages) & 1u;
         const uint32_t v_lo = (kv_lo + v_slot * (kTileBytes >> 4)) | kDescLoVMajor;
         const uint32_t k_lo = (kv_lo + k_slot * (kTileBytes >> 4)) | kDescKMajor;
-        if (jn < n_max && !mbar_wait_warp(p, &ctl->bars[kBarKvFull + k_slot], k_par))
-            return mma_gave_up(ctl, p.status, kBarKvFull + k_slot, (uint32_t)jn);
-#pragma unroll
+        bool have_k = !more;
+#pragma unroll 1
         for (int i = 0; i < 2; ++i) {
-            if (j < n_sub[i]) {
-                if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i]))
+            const int n_i = i ? n1 : n0;
+            const uint32_t s_i = tmem + kTmemS0 + (uint32_t)i * kTileN;
+            const uint32_t o_i = tmem + kTmemO0 + (uint32_t)i * kTileN;
+            if (j < n_i) {
+                if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], (uint32_t)j & 1u))
                     return mma_gave_up(ctl, p.status, kBarPFirst + i, (uint32_t)j);
                 tc_fence_after();
                 QW_TRACE(2, i, j);
                 if (elect_one())
-                    issue_pv_first(o_tmem[i], s_tmem[i], v_lo, o_started[i], bounded);
+                    issue_pv_keys<0, kPart>(o_i, s_i, v_lo, j > 0);
                 __syncwarp();
-                if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i]))
+                if (i == 1 && more) {
+                    const uint32_t tv = t + 1;
+                    if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + tv % kStages], (tv / kStages) & 1u))
+                        return mma_gave_up(ctl, p.status, kBarKvFull + tv % kStages, (uint32_t)jn);
+                }
+                if (!have_k) {
+                    if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + k_slot], k_par))
+                        return mma_gave_up(ctl, p.status, kBarKvFull + k_slot, (uint32_t)jn);
+                    have_k = true;
+                }
+                if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], (uint32_t)j & 1u))
                     return mma_gave_up(ctl, p.status, kBarPFull + i, (uint32_t)j);
-                p_phase[i] ^= 1u;
                 tc_fence_after();
-                if (elect_one()) issue_pv_rest(o_tmem[i], s_tmem[i], v_lo, bounded);
-                __syncwarp();
-                o_started[i] = true;
-                QW_TRACE(2, 4 + i, j);
-            }
-            if (i == 1 && elect_one()) tc_commit<1>(&ctl->bars[kBarKvEmpty + v_slot]);
-            __syncwarp();
-            if (jn < n_max && jn < n_sub[i]) {
                 if (elect_one()) {
-                    issue_qk(s_tmem[i], q_lo[i], k_lo);
-                    tc_commit<1>(&ctl->bars[kBarSFull + i]);
+                    issue_pv_keys<kPart, 8>(o_i, s_i, v_lo, true);
+                    if (i == 1 && more) tc_commit<1>(&ctl->bars[kBarKvEmpty + v_slot]);
+                    if (jn < n_i) {
+                        issue_qk(s_i, q_lo + (uint32_t)i * (kTileBytes >> 4), k_lo);
+                        tc_commit<1>(&ctl->bars[kBarSFull + i]);
+                    } else {
+                        tc_commit<1>(&ctl->bars[kBarOFinal + i]);
+                    }
                 }
                 __syncwarp();
                 QW_TRACE(2, 2 + i, jn);
             }
         }
-        if (jn < n_max) {
-            if (elect_one()) tc_commit<1>(&ctl->bars[kBarKvEmpty + k_slot]);
+        if (more) {
+            if (elect_one()) {
+                if (j >= n1) tc_commit<1>(&ctl->bars[kBarKvEmpty + v_slot]);
+                tc_commit<1>(&ctl->bars[kBarKvEmpty + k_slot]);
+            }
             __syncwarp();
+            ++t;
+            v_slot = t % kStages;
+            if (j >= n1 && !mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], (t / kStages) & 1u))
+                return mma_gave_up(ctl, p.status, kBarKvFull + v_slot, (uint32_t)jn);
+            ++t;
         }
         j = jn;
-    }
-    if (elect_one()) {
-        tc_commit<1>(&ctl->bars[kBarOFinal + 0]);
-        tc_commit<1>(&ctl->bars[kBarOFinal + 1]);
     }
 }
 
@@ -900,7 +893,7 @@ __device__ __forceinline__ uint32_t pair_a(int s, int lb) { return 2u * (uint32_
 __device__ __forceinline__ uint32_t pair_b(int s) { return 2u * (uint32_t)(2 * s + 1); }
 
 __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedControl *ctl,
-                                               uint8_t *smem_q, uint8_t *smem_kv, bool bounded) {
+                                               uint8_t *smem_q, uint8_t *smem_kv) {
     const int la = uniform(ctl->tile_count[0]), lb = uniform(ctl->tile_count[1]);
     if (la <= 0) return;
     const uint32_t tmem = uniform(ctl->tmem_base);
@@ -950,14 +943,14 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i]))
                 return mma_gave_up(ctl, p.status, kBarPFirst + i, (uint32_t)s);
             tc_fence_after();
-            if (elect_one()) issue_pv_first(o_tmem[i], s_tmem[i], desc, s > 0, bounded);
+            if (elect_one()) issue_pv_keys<0, kPart>(o_tmem[i], s_tmem[i], desc, s > 0);
             __syncwarp();
             if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i]))
                 return mma_gave_up(ctl, p.status, kBarPFull + i, (uint32_t)s);
             p_phase[i] ^= 1u;
             tc_fence_after();
             if (elect_one()) {
-                issue_pv_rest(o_tmem[i], s_tmem[i], desc, bounded);
+                issue_pv_keys<kPart, 8>(o_tmem[i], s_tmem[i], desc, true);
                 QW_RING_FREE(t_now + 1);
             }
             __syncwarp();
@@ -1207,8 +1200,8 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
     }
     if (tid < kSoftmaxThreads) {
     } else if (warp == kMmaWarp) {
-        if (split) mma_role_split(p, ctl, smem_q, smem_kv, bound >= 0.0f);
-        else mma_role(p, ctl, smem_q, smem_kv, bound >= 0.0f);
+        if (split) mma_role_split(p, ctl, smem_q, smem_kv);
+        else mma_role(p, ctl, smem_q, smem_kv);
     } else if (warp == kTmaWarp && lane == 0) {
         tma_role(p, ctl, smem_kv, &map_k, &map_v, b, kvh, split);
         // Q loads of active sub-tiles must have landed as well.
