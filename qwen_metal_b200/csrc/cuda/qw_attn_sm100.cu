@@ -21,9 +21,9 @@
 // skipped by all roles, interior tiles run without a compare, boundary tiles have their
 // scores masked (see mask_scores).
 //
-// Epilogue: O / l is rounded to bf16 into the (by then dead) Q tile in shared
-// memory and leaves as TMA stores of the whole 128x128 tile.  When the heads
-// are sharded over several GPUs the tile goes to this rank's head columns of a
+// Epilogue: O / l is rounded to bf16 and goes through the (by then dead) Q tile in shared
+// memory to global memory, every warp its own 32 rows (write_rows).  When the heads
+// are sharded over several GPUs the rows go to this rank's head columns of a
 // full-width output (the kernel can address several such destinations, peer-
 // mapped ones included); the multi-GPU group writes the rank's own buffer here
 // and carries the columns to the peers with a push kernel under the next layer,
@@ -102,8 +102,7 @@ enum Barrier : int {
     kBarPFirst = kBarSFull + 2,           // 2: first part of P_i written (one arrival per warp)
     kBarPFull = kBarPFirst + 2,           // 2: the rest of P_i written
     kBarOFinal = kBarPFull + 2,           // 2: last P V of sub-tile i complete
-    kBarEpi = kBarOFinal + 2,             // 2: output tile of sub-tile i staged in shared memory
-    kBarMerge = kBarEpi + 2,              // split form: sub-tile 1 published its exponent and row sum
+    kBarMerge = kBarOFinal + 2,           // split form: sub-tile 1 published its exponent and row sum
     kBarCount = kBarMerge + 1
 };
 
@@ -169,7 +168,7 @@ struct KernelParams {
 
 // A wait ran out: the first one of the launch leaves its place in the status words, and the other
 // waits of the CTA end.
-__device__ __forceinline__ void record_expiry(SharedControl *ctl, uint32_t *status, uint32_t where,
+__device__ __noinline__ void record_expiry(SharedControl *ctl, uint32_t *status, uint32_t where,
                                               uint32_t tile) {
     ctl->abort_flag = 1;
     if (atomicCAS(status, 0u, (uint32_t)QWCU_STATUS_WAIT_TIMEOUT) == 0u) {
@@ -232,12 +231,6 @@ template <typename T>
 __device__ __forceinline__ T uniform(T v) {
     return __shfl_sync(0xffffffffu, v, 0);
 }
-// Output tensor maps, one per destination (one on a single GPU, one per rank
-// when the heads are sharded and every rank receives the rows).
-struct OutMaps {
-    CUtensorMap m[8];
-};
-
 // Instruction descriptors, M = 128, N = 128.
 constexpr uint32_t kIdescQK = instr_desc(kTileM, kTileN, false);
 constexpr uint32_t kIdescPV = instr_desc(kTileM, kTileN, true);
@@ -432,14 +425,79 @@ __device__ __forceinline__ void mask_tile(uint32_t tmem_s, int key0, int limit, 
     tmem_wait_st();
 }
 
+// 32 output rows of a warp, one destination: out = (w_own * O_own + w_other * O_other) * inv,
+// rounded to bf16.  A thread has a row in TMEM; 64 columns at a time go through a box of 32 rows
+// x 128 bytes in shared memory (16-byte pieces XOR-swizzled by the row) and from there to global
+// memory with eight lanes per row.  (tmem_own, tmem_other: kNoTmem where there is none.  Every
+// lane takes part in the warp-collective TMEM loads.)
+//
+// Plain stores end with the instruction; a TMA store of the tile had to be waited for until it
+// had read shared memory, 1100 clocks at the end of every CTA.  And a function of its own: its
+// registers in one allocation with the softmax loop's cost that loop more than all of this (in
+// line, 8188 x 8211 keys took 1020 us instead of 955).  Six layers of 33 to 412 text rows took 45.2 to
+// 65.8 us and take 42.3 to 64.7; eight layers of six heads, 4352 keys, 555 -> 540 us.
+constexpr uint32_t kNoTmem = 0xffffffffu;
+__device__ __noinline__ void write_rows(uint32_t tmem_own, uint32_t tmem_other, float w_own,
+                                        float w_other, float inv, uint32_t box, __nv_bfloat16 *out,
+                                        uint32_t row_stride, uint32_t rows) {
+    const uint32_t lane = threadIdx.x & 31u, first = lane >> 3, piece = lane & 7u;
+    out += (size_t)first * row_stride + piece * 8u;
+#pragma unroll 1
+    for (uint32_t half = 0; half < 2; ++half, out += 64) {
+        uint32_t o[64];
+        if (tmem_own != kNoTmem) {
+            QW_TMEM_LD32(tmem_own + half * 64, o);
+            QW_TMEM_LD32(tmem_own + half * 64 + 32, o + 32);
+            QW_TMEM_WAIT_LD32(o);
+            QW_TMEM_WAIT_LD32(o + 32);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 64; ++i) o[i] = 0u;
+        }
+        if (tmem_other != kNoTmem) {
+#pragma unroll
+            for (int part = 0; part < 64; part += 32) {
+                uint32_t x[32];
+                QW_TMEM_LD32(tmem_other + half * 64 + part, x);
+                QW_TMEM_WAIT_LD32(x);
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    o[part + i] = __float_as_uint(fmaf(__uint_as_float(x[i]), w_other,
+                                                       __uint_as_float(o[part + i]) * w_own));
+            }
+        } else if (w_own != 1.0f) {
+#pragma unroll
+            for (int i = 0; i < 64; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * w_own);
+        }
+        __syncwarp();  // (the half before has been read)
+#pragma unroll
+        for (uint32_t c16 = 0; c16 < 8; ++c16) {
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                w[i] = pack_bf16(__uint_as_float(o[8 * c16 + 2 * i]) * inv,
+                                 __uint_as_float(o[8 * c16 + 2 * i + 1]) * inv);
+            st_shared16(box + lane * 128u + ((c16 ^ piece) << 4), w[0], w[1], w[2], w[3]);
+        }
+        __syncwarp();
+        __nv_bfloat16 *to = out;
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i, to += 4 * (size_t)row_stride) {
+            const uint32_t r = 4u * i + first;
+            const uint4 x = ld_shared16(box + r * 128u + ((piece ^ (r & 7u)) << 4));
+            if (r < rows) *reinterpret_cast<uint4 *>(to) = x;
+        }
+    }
+}
+
 // kBounded: the caller promised |score * scale * log2(e)| <= bound (see
 // KernelParams::score_bound), so P = exp2(score*c - bound) needs no row maximum:
 // the scores stream out of TMEM 32 columns at a time, each chunk's exponentials
 // run under the next chunk's load, and O is never rescaled.
 template <bool kBounded>
 __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedControl *ctl,
-                                             const OutMaps &maps_out, uint8_t *stage, int sub,
-                                             int tid_in_group, int my_limit, uint32_t b, uint32_t h,
+                                             uint8_t *stage, int sub, int tid_in_group,
+                                             int my_limit, uint32_t b, uint32_t h,
                                              uint32_t row, uint32_t tile_row0, bool split,
                                              float bound) {
     const int warp_in_group = tid_in_group >> 5;
@@ -617,13 +675,8 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
         ++processed;
     }
 
-    // Epilogue: O / l -> bf16.  Token-major output goes through shared memory (the
-    // dead Q tile of this sub-tile, same swizzled box layout) and leaves as TMA
-    // stores of the whole 128x128 tile, one pair per destination: on a single
-    // GPU that is one coalesced write, with sharded heads the same tile also
-    // goes to every peer's output over NVLink in bulk instead of 64-byte pieces.
+    // Epilogue: O / l -> bf16.
     if (!ok || tile_row0 >= p.q_rows) return;  // gave up, or this sub-tile holds no rows
-    const bool has_row = row < p.q_rows;
     if (processed > 0) {
         ok = mbar_wait(ctl, &ctl->bars[kBarOFinal + sub], 0, p.status,
                        (1u << 16) | (uint32_t)(kBarOFinal + sub), 0xffffu);
@@ -667,82 +720,33 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
         inv = l_all > 0.0f ? 1.0f / l_all : 0.0f;
         w_own = a_own;
         w_other = a_other;
-    } else if (processed == 0 && !p.head_major_out) {
+    } else if (processed == 0) {
         // Nothing was computed for this sub-tile (zeros go out), but its Q load may
         // still be in flight into the staging area: let it land first.
         ok = mbar_wait(ctl, &ctl->bars[kBarQFull + sub], 0, p.status,
                        (1u << 16) | (uint32_t)(kBarQFull + sub), 0xfffdu);
         if (!ok) return;
     }
-    if (split && !p.head_major_out && !use_own) {
+    if (split && !use_own) {
         // (same reason: the shared Q tile is the staging area)
         ok = mbar_wait(ctl, &ctl->bars[kBarQFull + 0], 0, p.status,
                        (1u << 16) | (uint32_t)(kBarQFull + 0), 0xfffdu);
         if (!ok) return;
     }
-    const uint32_t tmem_other = tmem + lane_base + kTmemO1;
-    // Row r of the tile in the staging area: two 128-byte lines (columns 0..63 and
-    // 64..127, one half tile apart), 16-byte chunks XOR-swizzled by the row like TMA
-    // does.  Head-major output is written directly.  (Every lane takes part in the
-    // warp-collective TMEM loads; only the stores depend on the row being real.)
-    uint8_t *line = stage + tid_in_group * 128;
-    const int sw = tid_in_group & 7;
-    __nv_bfloat16 *direct =
-        p.out + (((size_t)b * p.heads + h) * p.q_rows + (has_row ? row : 0u)) * kHeadDim;
+    const uint32_t warp_row0 = tile_row0 + (uint32_t)warp_in_group * 32u;
+    if (warp_row0 >= p.q_rows) return;
+    const uint32_t row_stride = (p.head_major_out ? 1u : p.out_heads_total) * kHeadDim;
+    const size_t first = p.head_major_out
+                             ? (((size_t)b * p.heads + h) * p.q_rows + warp_row0) * kHeadDim
+                             : ((size_t)b * p.q_rows + warp_row0) * row_stride +
+                                   (size_t)(p.out_head_offset + h) * kHeadDim;
+    const uint32_t tmem_own = use_own ? tmem_o : kNoTmem;
+    const uint32_t tmem_other = use_other ? tmem + lane_base + kTmemO1 : kNoTmem;
 #pragma unroll 1
-    for (int chunk = 0; chunk < 4; ++chunk) {
-        float v[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = 0.0f;
-        if (use_own) {
-            uint32_t o[32];
-            QW_TMEM_LD32(tmem_o + chunk * 32, o);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * w_own;
-        }
-        if (use_other) {
-            uint32_t o[32];
-            QW_TMEM_LD32(tmem_other + chunk * 32, o);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = fmaf(__uint_as_float(o[i]), w_other, v[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < 32; i += 8) {
-            uint4 packed;
-            packed.x = pack_bf16(v[i] * inv, v[i + 1] * inv);
-            packed.y = pack_bf16(v[i + 2] * inv, v[i + 3] * inv);
-            packed.z = pack_bf16(v[i + 4] * inv, v[i + 5] * inv);
-            packed.w = pack_bf16(v[i + 6] * inv, v[i + 7] * inv);
-            if (p.head_major_out) {
-                if (has_row) reinterpret_cast<uint4 *>(direct + chunk * 32)[i >> 3] = packed;
-            } else {
-                const int c16 = chunk * 4 + (i >> 3);  // 16-byte chunk of the 256-byte row
-                *reinterpret_cast<uint4 *>(line + (c16 >> 3) * kHalfTileBytes +
-                                           (((c16 & 7) ^ sw) << 4)) = packed;
-            }
-        }
-    }
-    if (p.head_major_out) return;
-    fence_async_shared();
-    __syncwarp();
-    if ((tid_in_group & 31) == 0) mbar_arrive(&ctl->bars[kBarEpi + sub]);
-    if (tid_in_group == 0) {
-        if (!mbar_wait(ctl, &ctl->bars[kBarEpi + sub], 0, p.status,
-                       (1u << 16) | (uint32_t)(kBarEpi + sub), 0xfffcu))
-            return;
-        const int col = (int)((p.out_head_offset + h) * kHeadDim);
-        for (uint32_t d = 0; d < p.n_out; ++d) {
-            tma_store_3d(&maps_out.m[d], stage, col, (int)tile_row0, (int)b);
-            tma_store_3d(&maps_out.m[d], stage + kHalfTileBytes, col + 64, (int)tile_row0, (int)b);
-        }
-        tma_store_commit();
-        // Shared memory may be released once the stores have read it; the
-        // writes themselves are complete when the grid completes, which is
-        // what the barrier behind a sharded launch waits for.
-        tma_store_wait_read<0>();
-    }
+    for (uint32_t d = 0; d < p.n_out; ++d)
+        write_rows(tmem_own, tmem_other, w_own, w_other, inv,
+                   smem_u32(stage + warp_in_group * (32 * 128)), p.out_peers[d] + first, row_stride,
+                   min(32u, p.q_rows - warp_row0));
 }
 
 // ---------------------------------------------------------------------------
@@ -821,7 +825,8 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
     // to 110 even where nothing is left to wait for.  So the next tiles of K and of V are waited
     // for behind the first parts of P V, where the warp waits for the rest of P anyway, and not both
     // in front of the step; and the two sub-tiles take turns in one loop, whose code is half as long.
-    // Eight layers of six heads, 4352 keys: 560 us before, 552 us.
+    // Eight layers of six heads, 4352 keys: 560 us before, 552 us, 537 us with the epilogue's
+    // registers out of the softmax's way as well (see write_rows).
     while (j < n_max) {
         const int jn = j + 1;
         const bool more = jn < n_max;
@@ -899,9 +904,6 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
     const uint32_t tmem = uniform(ctl->tmem_base);
     const uint32_t q_lo = (smem_u32(smem_q) >> 4) | kDescKMajor;
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;
-    const uint32_t s_tmem[2] = {tmem + kTmemS0, tmem + kTmemS1};
-    const uint32_t o_tmem[2] = {tmem + kTmemO0, tmem + kTmemO1};
-    uint32_t p_phase[2] = {0, 0};
 
     // Waits for ring position t, returns the low descriptor word of its slot.
 #define QW_RING_WAIT(t_, lo_fixed_, out_)                                                       \
@@ -919,7 +921,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
     uint32_t desc;
     QW_RING_WAIT(pair_a(0, lb), kDescKMajor, desc);
     if (elect_one()) {
-        issue_qk(s_tmem[0], q_lo, desc);
+        issue_qk(tmem + kTmemS0, q_lo, desc);
         tc_commit<1>(&ctl->bars[kBarSFull + 0]);
         QW_RING_FREE(pair_a(0, lb));
     }
@@ -927,30 +929,31 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
     if (lb > 0) {
         QW_RING_WAIT(pair_b(0), kDescKMajor, desc);
         if (elect_one()) {
-            issue_qk(s_tmem[1], q_lo, desc);
+            issue_qk(tmem + kTmemS1, q_lo, desc);
             tc_commit<1>(&ctl->bars[kBarSFull + 1]);
             QW_RING_FREE(pair_b(0));
         }
         __syncwarp();
     }
     for (int s = 0; s < la; ++s) {
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < 2; ++i) {
+            const uint32_t s_i = tmem + kTmemS0 + (uint32_t)i * kTileN;
+            const uint32_t o_i = tmem + kTmemO0 + (uint32_t)i * kTileN;
             const int count = i ? lb : la;
             if (s >= count) continue;
             const uint32_t t_now = i ? pair_b(s) : pair_a(s, lb);
             QW_RING_WAIT(t_now + 1, kDescLoVMajor, desc);
-            if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], p_phase[i]))
+            if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], (uint32_t)s & 1u))
                 return mma_gave_up(ctl, p.status, kBarPFirst + i, (uint32_t)s);
             tc_fence_after();
-            if (elect_one()) issue_pv_keys<0, kPart>(o_tmem[i], s_tmem[i], desc, s > 0);
+            if (elect_one()) issue_pv_keys<0, kPart>(o_i, s_i, desc, s > 0);
             __syncwarp();
-            if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], p_phase[i]))
+            if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], (uint32_t)s & 1u))
                 return mma_gave_up(ctl, p.status, kBarPFull + i, (uint32_t)s);
-            p_phase[i] ^= 1u;
             tc_fence_after();
             if (elect_one()) {
-                issue_pv_keys<kPart, 8>(o_tmem[i], s_tmem[i], desc, true);
+                issue_pv_keys<kPart, 8>(o_i, s_i, desc, true);
                 QW_RING_FREE(t_now + 1);
             }
             __syncwarp();
@@ -958,7 +961,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
                 const uint32_t t_next = i ? pair_b(s + 1) : pair_a(s + 1, lb);
                 QW_RING_WAIT(t_next, kDescKMajor, desc);
                 if (elect_one()) {
-                    issue_qk(s_tmem[i], q_lo, desc);
+                    issue_qk(s_i, q_lo, desc);
                     tc_commit<1>(&ctl->bars[kBarSFull + i]);
                     QW_RING_FREE(t_next);
                 }
@@ -1047,8 +1050,7 @@ template <bool kMayBound>
 __global__ void __launch_bounds__(kThreads, 1)
 qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
                      const __grid_constant__ CUtensorMap map_k,
-                     const __grid_constant__ CUtensorMap map_v,
-                     const __grid_constant__ OutMaps maps_out, const KernelParams p) {
+                     const __grid_constant__ CUtensorMap map_v, const KernelParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *smem_q = smem;
@@ -1085,7 +1087,6 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
             mbar_init(&ctl->bars[kBarPFirst + i], kTileM / 32);
             mbar_init(&ctl->bars[kBarPFull + i], kTileM / 32);
             mbar_init(&ctl->bars[kBarOFinal + i], 1);
-            mbar_init(&ctl->bars[kBarEpi + i], kTileM / 32);
         }
         mbar_init(&ctl->bars[kBarMerge], kTileM / 32);
         ctl->abort_flag = 0;
@@ -1190,10 +1191,10 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         uint8_t *stage = smem_q + (size_t)sub * kTileBytes;
         const uint32_t tile_row0 = split ? row0 : row0 + (uint32_t)sub * kTileM;
         if (kMayBound && bound >= 0.0f)
-            softmax_role<kMayBound>(p, ctl, maps_out, stage, sub, tid_in_group, my_limit, b, h,
+            softmax_role<kMayBound>(p, ctl, stage, sub, tid_in_group, my_limit, b, h,
                                     my_row, tile_row0, split, bound);
         else
-            softmax_role<false>(p, ctl, maps_out, stage, sub, tid_in_group, my_limit, b, h, my_row,
+            softmax_role<false>(p, ctl, stage, sub, tid_in_group, my_limit, b, h, my_row,
                                 tile_row0, split, 0.0f);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
@@ -1267,7 +1268,7 @@ void trace_dump(cudaStream_t stream) {
 }
 #endif
 
-typedef void (*AttnKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const OutMaps,
+typedef void (*AttnKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap,
                            const KernelParams);
 
 int sm_count_of_current_device() {
@@ -1381,12 +1382,6 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
     p.n_freed = a->slot_use ? a->n_freed : 0;
     if (p.n_freed > 8) return (int)cudaErrorInvalidValue;
     for (uint32_t d = 0; d < 8; ++d) p.freed_peer[d] = d < p.n_freed ? a->freed_peer[d] : nullptr;
-    OutMaps maps_out;
-    memset(&maps_out, 0, sizeof(maps_out));
-    if (!p.head_major_out)
-        for (uint32_t d = 0; d < p.n_out; ++d)
-            if ((rc = make_map_3d(&maps_out.m[d], p.out_peers[d], a->batch, a->q_rows, p.out_heads_total)))
-                return rc;
     // One CTA per unit; the units of the last, partly filled wave run split in two
     // (half the rows each, the key tiles divided between the sub-tiles) when the
     // doubled CTAs still fit the idle SMs, give or take a few light units.
@@ -1400,7 +1395,7 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
                        : qwcu_attn_sm100_tail_units(p.total_units,
                                                     (uint32_t)sm_count_of_current_device());
     const unsigned grid = p.total_units + p.tail_units;
-    rc = launch(kernel, grid, kThreads, kSmemBytes, 1, stream, map_q, map_k, map_v, maps_out, p);
+    rc = launch(kernel, grid, kThreads, kSmemBytes, 1, stream, map_q, map_k, map_v, p);
 #ifdef QW_ATTN_TRACE
     if (p.trace && !rc) trace_dump(stream);
 #endif
