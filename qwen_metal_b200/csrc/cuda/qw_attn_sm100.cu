@@ -166,6 +166,13 @@ struct KernelParams {
     int mma_probes;  // the same budget for the MMA warp's waits, in probes
 };
 
+// Shared address of a barrier.  (The roles keep the first one's and add: with a conversion from a
+// pointer at every wait and commit, six heads, eight layers took 535 instead of 529 us, 24 heads of
+// two, four layers 1687 instead of 1650.)
+__device__ __forceinline__ uint32_t bar_at(uint32_t bars, uint32_t which) {
+    return bars + which * (uint32_t)sizeof(Mbar);
+}
+
 // A wait ran out: the first one of the launch leaves its place in the status words, and the other
 // waits of the CTA end.
 __device__ __noinline__ void record_expiry(SharedControl *ctl, uint32_t *status, uint32_t where,
@@ -182,7 +189,7 @@ __device__ __noinline__ void record_expiry(SharedControl *ctl, uint32_t *status,
 // Bounded wait.  Returns false when the budget ran out here (recorded) or another thread
 // of the CTA already gave up.  (The GEMM's, out of line after a few probes, is not used
 // here: the softmax waits with its registers full.)
-__device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, Mbar *bar,
+__device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, uint32_t bar,
                                             uint32_t parity, uint32_t *status, uint32_t where,
                                             uint32_t tile) {
     long long start = clock64();
@@ -197,7 +204,7 @@ __device__ __forceinline__ bool mbar_wait_slow(SharedControl *ctl, Mbar *bar,
     }
 }
 
-__device__ __forceinline__ bool mbar_wait(SharedControl *ctl, Mbar *bar,
+__device__ __forceinline__ bool mbar_wait(SharedControl *ctl, uint32_t bar,
                                           uint32_t parity, uint32_t *status, uint32_t where,
                                           uint32_t tile) {
     if (mbar_try(bar, parity)) return true;
@@ -211,7 +218,7 @@ __device__ __forceinline__ bool mbar_wait(SharedControl *ctl, Mbar *bar,
 // layers, 24 heads of two 1825 to 1890 instead of 1725 us for four.  A probe that fails suspends
 // the warp for a time that the hardware sets: 400 000 of them took 1.58 s, 7800 clocks each.
 constexpr long long kProbeCycles = 10000;
-__device__ __forceinline__ bool mbar_wait_warp(const KernelParams &p, Mbar *bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_warp(const KernelParams &p, uint32_t bar, uint32_t parity) {
     bool ok = false;
 #pragma unroll 1
     for (int i = 0; i < p.mma_probes && !ok; ++i) ok = mbar_try(bar, parity);
@@ -370,9 +377,9 @@ __device__ __forceinline__ int visited_tiles(int tiles, int lo, int hi) {
 // ---------------------------------------------------------------------------
 // Softmax + epilogue role: 128 threads per sub-tile, one query row each.
 // ---------------------------------------------------------------------------
-// The first part of P is complete once its stores, issued a chunk of exponentials ago,
-// have landed: P V of these keys starts under the softmax of the others.
-__device__ __forceinline__ void publish_p_first(Mbar *bar, int tid_in_group) {
+// The first part of P: published before the exponentials of the rest are begun, so that its P V
+// runs under them.
+__device__ __forceinline__ void publish_p_first(uint32_t bar, int tid_in_group) {
     tmem_wait_st();
     tc_fence_before();
     if ((tid_in_group & 31) == 0) mbar_arrive(bar);
@@ -505,9 +512,9 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
     const uint32_t tmem = ctl->tmem_base;
     const uint32_t tmem_s = tmem + lane_base + (sub ? kTmemS1 : kTmemS0);
     const uint32_t tmem_o = tmem + lane_base + (sub ? kTmemO1 : kTmemO0);
-    Mbar *bar_s = &ctl->bars[kBarSFull + sub];
-    Mbar *bar_p_first = &ctl->bars[kBarPFirst + sub];
-    Mbar *bar_p = &ctl->bars[kBarPFull + sub];
+    const uint32_t bars = smem_u32(ctl->bars) + (uint32_t)sub * (uint32_t)sizeof(Mbar);
+    const uint32_t bar_s = bar_at(bars, kBarSFull), bar_p = bar_at(bars, kBarPFull);
+    const uint32_t bar_p_first = bar_at(bars, kBarPFirst);
     const int pad_lo = p.text_pad ? (int)p.text_len[b] : 0;
     const int pad_hi = (int)p.text_pad;
     const float c = p.scale_log2;  // positive (the host sends other scales elsewhere)
@@ -542,6 +549,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
                 for (int chunk = 0; chunk < 4; ++chunk) {
                     uint32_t(&cur)[32] = (chunk & 1) ? sb : sa;
                     uint32_t(&nxt)[32] = (chunk & 1) ? sa : sb;
+                    if (chunk == kPart / 2) publish_p_first(bar_p_first, tid_in_group);
                     QW_TMEM_WAIT_LD32(cur);
                     if (chunk == 0 && tid_in_group == 0) QW_TRACE(sub, 1, j);
                     if (chunk < 3) QW_TMEM_LD32(tmem_s + 32 * (chunk + 1), nxt);
@@ -558,7 +566,6 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
                         else sum_a = fadd2(sum_a, pr);
                         pk[i] = pack_bf16(pr.x, pr.y);
                     }
-                    if (chunk == kPart / 2) publish_p_first(bar_p_first, tid_in_group);
                     // P chunk c lands on columns [16c, 16c+16): scores already consumed.
                     QW_TMEM_ST16(tmem_s + chunk * 16, pk);
                     if (chunk == 1 && tid_in_group == 0) QW_TRACE(sub, 2, j);
@@ -652,6 +659,10 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
 #pragma unroll
         for (int chunk = 0; chunk < 4; ++chunk) {
             uint32_t pk[16];
+            if (chunk == kPart / 2) {
+                publish_p_first(bar_p_first, tid_in_group);
+                QW_TMEM_WAIT_LD32(s + 32 * (kPart / 2));  // (nothing is loading: the rest stays behind)
+            }
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int e = chunk * 32 + 2 * i;
@@ -662,7 +673,6 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
                 else sum_a = fadd2(sum_a, pr);
                 pk[i] = pack_bf16(pr.x, pr.y);
             }
-            if (chunk == kPart / 2) publish_p_first(bar_p_first, tid_in_group);
             QW_TMEM_ST16(tmem_s + chunk * 16, pk);
         }
         if (tid_in_group == 0) QW_TRACE(sub, 3, j);
@@ -678,7 +688,7 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
     // Epilogue: O / l -> bf16.
     if (!ok || tile_row0 >= p.q_rows) return;  // gave up, or this sub-tile holds no rows
     if (processed > 0) {
-        ok = mbar_wait(ctl, &ctl->bars[kBarOFinal + sub], 0, p.status,
+        ok = mbar_wait(ctl, bar_at(bars, kBarOFinal), 0, p.status,
                        (1u << 16) | (uint32_t)(kBarOFinal + sub), 0xffffu);
         if (!ok) return;
         tc_fence_after();
@@ -702,12 +712,12 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
             if ((tid_in_group & 31) == 0) mbar_arrive(&ctl->bars[kBarMerge]);
             return;
         }
-        ok = mbar_wait(ctl, &ctl->bars[kBarMerge], 0, p.status, (1u << 16) | (uint32_t)kBarMerge,
+        ok = mbar_wait(ctl, bar_at(bars, kBarMerge), 0, p.status, (1u << 16) | (uint32_t)kBarMerge,
                        0xfffbu);
         if (!ok) return;
         use_other = ctl->tile_count[1] > 0;
         if (use_other) {
-            ok = mbar_wait(ctl, &ctl->bars[kBarOFinal + 1], 0, p.status,
+            ok = mbar_wait(ctl, bar_at(bars, kBarOFinal + 1), 0, p.status,
                            (1u << 16) | (uint32_t)(kBarOFinal + 1), 0xfffeu);
             if (!ok) return;
             tc_fence_after();
@@ -723,13 +733,13 @@ __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedContro
     } else if (processed == 0) {
         // Nothing was computed for this sub-tile (zeros go out), but its Q load may
         // still be in flight into the staging area: let it land first.
-        ok = mbar_wait(ctl, &ctl->bars[kBarQFull + sub], 0, p.status,
+        ok = mbar_wait(ctl, bar_at(bars, kBarQFull), 0, p.status,
                        (1u << 16) | (uint32_t)(kBarQFull + sub), 0xfffdu);
         if (!ok) return;
     }
     if (split && !use_own) {
         // (same reason: the shared Q tile is the staging area)
-        ok = mbar_wait(ctl, &ctl->bars[kBarQFull + 0], 0, p.status,
+        ok = mbar_wait(ctl, bar_at(bars, kBarQFull), 0, p.status,
                        (1u << 16) | (uint32_t)(kBarQFull + 0), 0xfffdu);
         if (!ok) return;
     }
@@ -790,7 +800,7 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
     const int n_max = max(n0, n1);
     int j = 0;
     if (j >= n_max) return;
-    const uint32_t tmem = uniform(ctl->tmem_base);
+    const uint32_t tmem = uniform(ctl->tmem_base), bars = uniform(smem_u32(ctl->bars));
     // Low descriptor words: start address in 16-byte units plus the fixed LBO field.
     const uint32_t q_lo = (smem_u32(smem_q) >> 4) | kDescKMajor;  // sub-tile 1's is one tile further
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;  // slot s starts (s * kTileBytes) >> 4 further
@@ -799,27 +809,27 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
 
     {
         const uint32_t slot = t++ % kStages;
-        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot], 0))
+        if (!mbar_wait_warp(p, bar_at(bars, kBarKvFull + slot), 0))
             return mma_gave_up(ctl, p.status, kBarKvFull + slot, (uint32_t)j);
         const uint32_t k_lo = (kv_lo + slot * (kTileBytes >> 4)) | kDescKMajor;
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
             if (j >= (i ? n1 : n0)) continue;
-            if (!mbar_wait_warp(p, &ctl->bars[kBarQFull + i], 0))
+            if (!mbar_wait_warp(p, bar_at(bars, kBarQFull + i), 0))
                 return mma_gave_up(ctl, p.status, kBarQFull + i, 0);
             tc_fence_after();
             if (elect_one()) {
                 issue_qk(tmem + kTmemS0 + (uint32_t)i * kTileN,
                          q_lo + (uint32_t)i * (kTileBytes >> 4), k_lo);
-                tc_commit<1>(&ctl->bars[kBarSFull + i]);
+                tc_commit<1>(bar_at(bars, kBarSFull + i));
             }
             __syncwarp();
         }
-        if (elect_one()) tc_commit<1>(&ctl->bars[kBarKvEmpty + slot]);
+        if (elect_one()) tc_commit<1>(bar_at(bars, kBarKvEmpty + slot));
         __syncwarp();
     }
     uint32_t v_slot = t++ % kStages;
-    if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], 0))
+    if (!mbar_wait_warp(p, bar_at(bars, kBarKvFull + v_slot), 0))
         return mma_gave_up(ctl, p.status, kBarKvFull + v_slot, (uint32_t)j);
     // The tensor cores take four MMAs ahead, about 150 clocks of work, and a wait costs this warp 60
     // to 110 even where nothing is left to wait for.  So the next tiles of K and of V are waited
@@ -840,7 +850,7 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
             const uint32_t s_i = tmem + kTmemS0 + (uint32_t)i * kTileN;
             const uint32_t o_i = tmem + kTmemO0 + (uint32_t)i * kTileN;
             if (j < n_i) {
-                if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], (uint32_t)j & 1u))
+                if (!mbar_wait_warp(p, bar_at(bars, kBarPFirst + i), (uint32_t)j & 1u))
                     return mma_gave_up(ctl, p.status, kBarPFirst + i, (uint32_t)j);
                 tc_fence_after();
                 QW_TRACE(2, i, j);
@@ -849,25 +859,25 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
                 __syncwarp();
                 if (i == 1 && more) {
                     const uint32_t tv = t + 1;
-                    if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + tv % kStages], (tv / kStages) & 1u))
+                    if (!mbar_wait_warp(p, bar_at(bars, kBarKvFull + tv % kStages), (tv / kStages) & 1u))
                         return mma_gave_up(ctl, p.status, kBarKvFull + tv % kStages, (uint32_t)jn);
                 }
                 if (!have_k) {
-                    if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + k_slot], k_par))
+                    if (!mbar_wait_warp(p, bar_at(bars, kBarKvFull + k_slot), k_par))
                         return mma_gave_up(ctl, p.status, kBarKvFull + k_slot, (uint32_t)jn);
                     have_k = true;
                 }
-                if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], (uint32_t)j & 1u))
+                if (!mbar_wait_warp(p, bar_at(bars, kBarPFull + i), (uint32_t)j & 1u))
                     return mma_gave_up(ctl, p.status, kBarPFull + i, (uint32_t)j);
                 tc_fence_after();
                 if (elect_one()) {
                     issue_pv_keys<kPart, 8>(o_i, s_i, v_lo, true);
-                    if (i == 1 && more) tc_commit<1>(&ctl->bars[kBarKvEmpty + v_slot]);
+                    if (i == 1 && more) tc_commit<1>(bar_at(bars, kBarKvEmpty + v_slot));
                     if (jn < n_i) {
                         issue_qk(s_i, q_lo + (uint32_t)i * (kTileBytes >> 4), k_lo);
-                        tc_commit<1>(&ctl->bars[kBarSFull + i]);
+                        tc_commit<1>(bar_at(bars, kBarSFull + i));
                     } else {
-                        tc_commit<1>(&ctl->bars[kBarOFinal + i]);
+                        tc_commit<1>(bar_at(bars, kBarOFinal + i));
                     }
                 }
                 __syncwarp();
@@ -876,13 +886,13 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
         }
         if (more) {
             if (elect_one()) {
-                if (j >= n1) tc_commit<1>(&ctl->bars[kBarKvEmpty + v_slot]);
-                tc_commit<1>(&ctl->bars[kBarKvEmpty + k_slot]);
+                if (j >= n1) tc_commit<1>(bar_at(bars, kBarKvEmpty + v_slot));
+                tc_commit<1>(bar_at(bars, kBarKvEmpty + k_slot));
             }
             __syncwarp();
             ++t;
             v_slot = t % kStages;
-            if (j >= n1 && !mbar_wait_warp(p, &ctl->bars[kBarKvFull + v_slot], (t / kStages) & 1u))
+            if (j >= n1 && !mbar_wait_warp(p, bar_at(bars, kBarKvFull + v_slot), (t / kStages) & 1u))
                 return mma_gave_up(ctl, p.status, kBarKvFull + v_slot, (uint32_t)jn);
             ++t;
         }
@@ -901,7 +911,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
                                                uint8_t *smem_q, uint8_t *smem_kv) {
     const int la = uniform(ctl->tile_count[0]), lb = uniform(ctl->tile_count[1]);
     if (la <= 0) return;
-    const uint32_t tmem = uniform(ctl->tmem_base);
+    const uint32_t tmem = uniform(ctl->tmem_base), bars = uniform(smem_u32(ctl->bars));
     const uint32_t q_lo = (smem_u32(smem_q) >> 4) | kDescKMajor;
     const uint32_t kv_lo = smem_u32(smem_kv) >> 4;
 
@@ -909,20 +919,20 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
 #define QW_RING_WAIT(t_, lo_fixed_, out_)                                                       \
     {                                                                                           \
         const uint32_t slot_ = (t_) % kStages, par_ = ((t_) / kStages) & 1u;                    \
-        if (!mbar_wait_warp(p, &ctl->bars[kBarKvFull + slot_], par_))                           \
+        if (!mbar_wait_warp(p, bar_at(bars, kBarKvFull + slot_), par_))                           \
             return mma_gave_up(ctl, p.status, kBarKvFull + slot_, (t_));                        \
         tc_fence_after();                                                                       \
         out_ = (kv_lo + slot_ * (kTileBytes >> 4)) | (lo_fixed_);                               \
     }
-#define QW_RING_FREE(t_) tc_commit<1>(&ctl->bars[kBarKvEmpty + ((t_) % kStages)])
+#define QW_RING_FREE(t_) tc_commit<1>(bar_at(bars, kBarKvEmpty + ((t_) % kStages)))
 
-    if (!mbar_wait_warp(p, &ctl->bars[kBarQFull + 0], 0))
+    if (!mbar_wait_warp(p, bar_at(bars, kBarQFull + 0), 0))
         return mma_gave_up(ctl, p.status, kBarQFull + 0, 0);
     uint32_t desc;
     QW_RING_WAIT(pair_a(0, lb), kDescKMajor, desc);
     if (elect_one()) {
         issue_qk(tmem + kTmemS0, q_lo, desc);
-        tc_commit<1>(&ctl->bars[kBarSFull + 0]);
+        tc_commit<1>(bar_at(bars, kBarSFull + 0));
         QW_RING_FREE(pair_a(0, lb));
     }
     __syncwarp();
@@ -930,7 +940,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
         QW_RING_WAIT(pair_b(0), kDescKMajor, desc);
         if (elect_one()) {
             issue_qk(tmem + kTmemS1, q_lo, desc);
-            tc_commit<1>(&ctl->bars[kBarSFull + 1]);
+            tc_commit<1>(bar_at(bars, kBarSFull + 1));
             QW_RING_FREE(pair_b(0));
         }
         __syncwarp();
@@ -944,12 +954,12 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
             if (s >= count) continue;
             const uint32_t t_now = i ? pair_b(s) : pair_a(s, lb);
             QW_RING_WAIT(t_now + 1, kDescLoVMajor, desc);
-            if (!mbar_wait_warp(p, &ctl->bars[kBarPFirst + i], (uint32_t)s & 1u))
+            if (!mbar_wait_warp(p, bar_at(bars, kBarPFirst + i), (uint32_t)s & 1u))
                 return mma_gave_up(ctl, p.status, kBarPFirst + i, (uint32_t)s);
             tc_fence_after();
             if (elect_one()) issue_pv_keys<0, kPart>(o_i, s_i, desc, s > 0);
             __syncwarp();
-            if (!mbar_wait_warp(p, &ctl->bars[kBarPFull + i], (uint32_t)s & 1u))
+            if (!mbar_wait_warp(p, bar_at(bars, kBarPFull + i), (uint32_t)s & 1u))
                 return mma_gave_up(ctl, p.status, kBarPFull + i, (uint32_t)s);
             tc_fence_after();
             if (elect_one()) {
@@ -962,7 +972,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
                 QW_RING_WAIT(t_next, kDescKMajor, desc);
                 if (elect_one()) {
                     issue_qk(s_i, q_lo, desc);
-                    tc_commit<1>(&ctl->bars[kBarSFull + i]);
+                    tc_commit<1>(bar_at(bars, kBarSFull + i));
                     QW_RING_FREE(t_next);
                 }
                 __syncwarp();
@@ -972,8 +982,8 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
 #undef QW_RING_WAIT
 #undef QW_RING_FREE
     if (elect_one()) {
-        tc_commit<1>(&ctl->bars[kBarOFinal + 0]);
-        tc_commit<1>(&ctl->bars[kBarOFinal + 1]);
+        tc_commit<1>(bar_at(bars, kBarOFinal + 0));
+        tc_commit<1>(bar_at(bars, kBarOFinal + 1));
     }
 }
 
@@ -998,7 +1008,7 @@ __device__ void tma_role(const KernelParams &p, SharedControl *ctl, uint8_t *sme
         const int j = phys_tile(ctl, u);
         for (int which = 0; which < 2 && ok; ++which) {
             uint32_t slot = t % kStages, par = ((t / kStages) & 1u) ^ 1u;
-            ok = mbar_wait(ctl, &ctl->bars[kBarKvEmpty + slot], par, p.status,
+            ok = mbar_wait(ctl, smem_u32(&ctl->bars[kBarKvEmpty + slot]), par, p.status,
                            where | (kBarKvEmpty + slot), (uint32_t)j);
             if (!ok) break;
             ++t;

@@ -53,9 +53,12 @@ __device__ __forceinline__ void mbar_init(Mbar *bar, uint32_t count) {
 __device__ __forceinline__ void mbar_init_fence() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive(Mbar *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+// (By pointer or by shared address: a loop that keeps the address of its barriers as one word
+// saves the conversion at each of them.)
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(Mbar *bar) { mbar_arrive(smem_u32(bar)); }
 __device__ __forceinline__ void mbar_expect_tx(Mbar *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
                  "r"(bytes)
@@ -63,16 +66,19 @@ __device__ __forceinline__ void mbar_expect_tx(Mbar *bar, uint32_t bytes) {
 }
 // (The arrivals may come from the peer CTA: what they order is TMEM and TMA traffic,
 // which carries fences of its own.)
-__device__ __forceinline__ bool mbar_try(Mbar *bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return done != 0;
+}
+__device__ __forceinline__ bool mbar_try(Mbar *bar, uint32_t parity) {
+    return mbar_try(smem_u32(bar), parity);
 }
 
 // ---- cluster --------------------------------------------------------------------
@@ -193,18 +199,21 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t cols) {
 // The barrier is signalled when every MMA issued so far by this thread is done; for a
 // pair the same barrier of both CTAs.
 template <int kGroup>
-__device__ __forceinline__ void tc_commit(Mbar *bar) {
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
     if constexpr (kGroup == 2)
         asm volatile(
             "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
-            "[%0], %1;" ::"r"(smem_u32(bar)),
+            "[%0], %1;" ::"r"(bar),
             "h"((unsigned short)3)
             : "memory");
     else
         asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(bar))
+            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
             : "memory");
+}
+template <int kGroup>
+__device__ __forceinline__ void tc_commit(Mbar *bar) {
+    tc_commit<kGroup>(smem_u32(bar));
 }
 
 // Shared-memory matrix descriptor as two words: start address >> 4 in bits 0-13,
