@@ -51,6 +51,7 @@ struct Params {
     uint32_t rows, table_rows, heads;
     float eps;
     int double_round;
+    uint32_t groups, group_heads;  // few strips: a row's heads in groups
     uint32_t strips;  // rows * tensors: one half-warp walks the heads of one (row, tensor)
     int tensors;
     float *bound_out;  // optional: [0], [1] = upper bounds of the 2-norm of any q row, k row
@@ -67,6 +68,64 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // Heads a half-warp has in flight at once (independent 16-byte loads; the
 // kernel is HBM-bound once the instruction count is small enough).
 constexpr int kHeadsPerTrip = 4;
+
+// One head: lane l of a half-warp holds elements [8l, 8l+8) = RoPE pairs 4l..4l+3.
+__device__ __forceinline__ uint4 finish_head(const Params &p, const uint4 &x, bool norm, bool rotate,
+                                             const float (&wf)[8], const float (&cc)[4],
+                                             const float (&sn)[4], uint32_t half_mask) {
+                    float v[8] = {bf16_lo(x.x), bf16_hi(x.x), bf16_lo(x.y), bf16_hi(x.y),
+                                  bf16_lo(x.z), bf16_hi(x.z), bf16_lo(x.w), bf16_hi(x.w)};
+                    uint32_t y[4] = {x.x, x.y, x.z, x.w};
+                    if (norm) {
+                        float ss = 0.0f;
+    #pragma unroll
+                        for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
+    #pragma unroll
+                        for (int off = 8; off > 0; off >>= 1)
+                            ss += __shfl_xor_sync(half_mask, ss, off, 16);
+                        // mean = ss / 128 exactly; 1/sqrt to within 2 ulp of the reference's rsqrt
+                        const float inv = rsqrtf(__fadd_rn(ss * 0.0078125f, p.eps));
+    #pragma unroll
+                        for (int i = 0; i < 8; i += 2) {
+                            float n0 = __fmul_rn(v[i], inv), n1 = __fmul_rn(v[i + 1], inv);
+                            if (p.double_round) {
+                                const uint32_t r = pack_bf16x2(n0, n1);
+                                n0 = bf16_lo(r);
+                                n1 = bf16_hi(r);
+                            }
+                            y[i >> 1] = pack_bf16x2(__fmul_rn(n0, wf[i]), __fmul_rn(n1, wf[i + 1]));
+                        }
+                        if (rotate) {
+    #pragma unroll
+                            for (int i = 0; i < 4; ++i) {  // the bf16 store between norm and rotation
+                                v[2 * i] = bf16_lo(y[i]);
+                                v[2 * i + 1] = bf16_hi(y[i]);
+                            }
+                        }
+                    }
+                    if (rotate) {
+    #pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float e = v[2 * i], o = v[2 * i + 1];
+                            y[i] = pack_bf16x2(__fsub_rn(__fmul_rn(e, cc[i]), __fmul_rn(o, sn[i])),
+                                               __fadd_rn(__fmul_rn(e, sn[i]), __fmul_rn(o, cc[i])));
+                        }
+                    }
+    return make_uint4(y[0], y[1], y[2], y[3]);
+}
+
+// The bound of a normalised head's 2-norm (the first strips are row 0 of q and of k): sum
+// (x*inv)^2 <= 128, so after the weight it is at most sqrt(128) * max|w|; the two bf16 roundings
+// (norm, rotation) and the f32 tables add well under 1 %.  The rotation itself preserves it.
+__device__ __forceinline__ void write_bound(const Params &p, uint32_t which, const float (&wf)[8],
+                                            uint32_t half_mask, int lane16) {
+    float wmax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wmax = fmaxf(wmax, fabsf(wf[i]));
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(half_mask, wmax, off, 16));
+    if (lane16 == 0) p.bound_out[which] = 11.313708499f * 1.01f * wmax;
+}
 
 // A half-warp owns one (row, tensor) strip: it keeps its 8-element slice of the
 // norm weight and of the row's cos/sin in registers and walks the heads, four at
@@ -98,19 +157,7 @@ __global__ void __launch_bounds__(256) qw_prologue_kernel(const Params p) {
             wf[0] = bf16_lo(wv.x); wf[1] = bf16_hi(wv.x); wf[2] = bf16_lo(wv.y); wf[3] = bf16_hi(wv.y);
             wf[4] = bf16_lo(wv.z); wf[5] = bf16_hi(wv.z); wf[6] = bf16_lo(wv.w); wf[7] = bf16_hi(wv.w);
         }
-        if (p.bound_out && strip < 2u && w) {
-            // The first two strips are row 0 of q and of k.  A normalised head has
-            // sum (x*inv)^2 <= 128, so after the weight its 2-norm is at most
-            // sqrt(128) * max|w|; the two bf16 roundings (norm, rotation) and the
-            // f32 tables add well under 1 %.  The rotation itself preserves it.
-            float wmax = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) wmax = fmaxf(wmax, fabsf(wf[i]));
-#pragma unroll
-            for (int off = 8; off > 0; off >>= 1)
-                wmax = fmaxf(wmax, __shfl_xor_sync(half_mask, wmax, off, 16));
-            if (lane16 == 0) p.bound_out[which] = 11.313708499f * 1.01f * wmax;
-        }
+        if (p.bound_out && strip < 2u && w) write_bound(p, which, wf, half_mask, lane16);
         if (rotate) {
             const size_t t = (size_t)((live ? row : 0u) % p.table_rows) * 16 + lane16;
             const float4 c = p.cos_t[t], s4 = p.sin_t[t];
@@ -125,49 +172,66 @@ __global__ void __launch_bounds__(256) qw_prologue_kernel(const Params p) {
                                                      : make_uint4(0, 0, 0, 0);
 #pragma unroll
             for (int u = 0; u < kHeadsPerTrip; ++u) {
-                float v[8] = {bf16_lo(x[u].x), bf16_hi(x[u].x), bf16_lo(x[u].y), bf16_hi(x[u].y),
-                              bf16_lo(x[u].z), bf16_hi(x[u].z), bf16_lo(x[u].w), bf16_hi(x[u].w)};
-                uint32_t y[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-                if (w) {
-                    float ss = 0.0f;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
-#pragma unroll
-                    for (int off = 8; off > 0; off >>= 1)
-                        ss += __shfl_xor_sync(half_mask, ss, off, 16);
-                    // mean = ss / 128 exactly; 1/sqrt to within 2 ulp of the reference's rsqrt
-                    const float inv = rsqrtf(__fadd_rn(ss * 0.0078125f, p.eps));
-#pragma unroll
-                    for (int i = 0; i < 8; i += 2) {
-                        float n0 = __fmul_rn(v[i], inv), n1 = __fmul_rn(v[i + 1], inv);
-                        if (p.double_round) {
-                            const uint32_t r = pack_bf16x2(n0, n1);
-                            n0 = bf16_lo(r);
-                            n1 = bf16_hi(r);
-                        }
-                        y[i >> 1] = pack_bf16x2(__fmul_rn(n0, wf[i]), __fmul_rn(n1, wf[i + 1]));
-                    }
-                    if (rotate) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {  // the bf16 store between norm and rotation
-                            v[2 * i] = bf16_lo(y[i]);
-                            v[2 * i + 1] = bf16_hi(y[i]);
-                        }
-                    }
-                }
-                if (rotate) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float e = v[2 * i], o = v[2 * i + 1];
-                        y[i] = pack_bf16x2(__fsub_rn(__fmul_rn(e, cc[i]), __fmul_rn(o, sn[i])),
-                                           __fadd_rn(__fmul_rn(e, sn[i]), __fmul_rn(o, cc[i])));
-                    }
-                }
+                const uint4 y = finish_head(p, x[u], w != nullptr, rotate, wf, cc, sn, half_mask);
                 if (live && head0 + u < p.heads)
-                    dst[(size_t)(head0 + u) * 16] = make_uint4(y[0], y[1], y[2], y[3]);
+                    dst[(size_t)(head0 + u) * 16] = y;
             }
         }
     }
+}
+
+// The same for few strips, where a strip's time is a chain of memory round trips and not
+// bandwidth: its first loads all leave together, a trip's loads run under the trip before, and
+// the heads of a row are dealt out to p.groups half-warps of p.group_heads each, as long as that
+// finds SMs with room.  77 registers: three CTAs per SM, where the form above has four, so it is
+// for grids of up to three per SM.  us a launch of q and k, the form above and this one: 24 heads, 320
+// rows 9.7 and 5.2, 1152 rows 12.3 and 7.6; 32 heads, 2351 rows 18.2 and 15.5; beyond, with one group, 6
+// heads of 4352 rows 8.2 and 9.8, 24 heads 21.1 and 22.9.
+__global__ void __launch_bounds__(256) qw_prologue_few_kernel(const Params p) {
+    sm100::grid_launch_dependents();
+    sm100::grid_wait();
+    const int lane16 = threadIdx.x & 15;
+    const uint32_t half_mask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
+    const uint32_t strip = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    const uint32_t per_row = (uint32_t)p.tensors * p.groups;
+    const uint32_t row = strip / per_row, rest = strip - row * per_row;
+    if (row >= p.rows) return;  // (the reductions name their own 16 lanes)
+    const uint32_t group = rest / (uint32_t)p.tensors;
+    const uint32_t which = rest - group * (uint32_t)p.tensors;  // 0 query, 1 key, 2 value
+    const uint4 *src = (which == 0 ? p.q_in : which == 1 ? p.k_in : p.v_in) + (size_t)row * p.heads * 16 + lane16;
+    uint4 *dst = (which == 0 ? p.q_out : which == 1 ? p.k_out : p.v_out) + (size_t)row * p.heads * 16 + lane16;
+    const uint4 *w = which == 0 ? p.wq : which == 1 ? p.wk : nullptr;
+    const bool rotate = p.cos_t && which < 2;
+    const uint32_t begin = group * p.group_heads, end = min(p.heads, begin + p.group_heads);
+    const auto load_trip = [&](uint4 (&x)[kHeadsPerTrip], uint32_t head0) {
+#pragma unroll
+        for (int u = 0; u < kHeadsPerTrip; ++u)
+            x[u] = head0 + u < end ? src[(size_t)(head0 + u) * 16] : make_uint4(0, 0, 0, 0);
+    };
+    uint4 x[kHeadsPerTrip];
+    load_trip(x, begin);
+    float4 c4 = make_float4(0, 0, 0, 0), s4 = c4;
+    if (rotate) {
+        const size_t t = (size_t)(row % p.table_rows) * 16 + lane16;
+        c4 = p.cos_t[t];
+        s4 = p.sin_t[t];
+    }
+    const uint4 wv = w ? w[lane16] : make_uint4(0, 0, 0, 0);
+    const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+    const float wf[8] = {bf16_lo(wv.x), bf16_hi(wv.x), bf16_lo(wv.y), bf16_hi(wv.y),
+                         bf16_lo(wv.z), bf16_hi(wv.z), bf16_lo(wv.w), bf16_hi(wv.w)};
+    for (uint32_t head0 = begin; head0 < end; head0 += kHeadsPerTrip) {
+        uint4 next[kHeadsPerTrip];
+        load_trip(next, head0 + kHeadsPerTrip);
+#pragma unroll
+        for (int u = 0; u < kHeadsPerTrip; ++u) {
+            const uint4 y = finish_head(p, x[u], w != nullptr, rotate, wf, cc, sn, half_mask);
+            if (head0 + u < end) dst[(size_t)(head0 + u) * 16] = y;
+        }
+#pragma unroll
+        for (int u = 0; u < kHeadsPerTrip; ++u) x[u] = next[u];
+    }
+    if (p.bound_out && row == 0 && group == 0 && w) write_bound(p, which, wf, half_mask, lane16);
 }
 
 __global__ void qw_scale_bf16_kernel(__nv_bfloat16 *out, const __nv_bfloat16 *in, size_t n,
@@ -207,6 +271,8 @@ bool spread_ready() {
     const bool tracked = dev >= 0 && dev < 64;
     if (tracked && ready[dev]) return true;
     if (cudaFuncSetAttribute(qw_prologue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)spread_smem(1)) != cudaSuccess ||
+        cudaFuncSetAttribute(qw_prologue_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)spread_smem(1)) != cudaSuccess)
         return false;
     if (tracked) ready[dev] = true;
@@ -244,6 +310,20 @@ extern "C" int qwcu_prologue_launch(const qwcu_prologue_args *a, qwcu_stream str
     if (strips > 0xffffffffull) return (int)cudaErrorInvalidValue;
     p.strips = (uint32_t)strips;
     const int threads = 256;
+    const unsigned sms = (unsigned)sm_count_cached();
+    if (!spread_ready()) return (int)cudaGetLastError();
+    const unsigned long long room = 3ull * sms * (threads / 16);  // half-warps of three CTAs per SM
+    const unsigned long long plain = (unsigned long long)a->rows * p.tensors;
+    const bool few = plain <= room;
+    if (few) {
+        const uint32_t trips = (a->heads + kHeadsPerTrip - 1) / kHeadsPerTrip;
+        unsigned long long groups = room / plain;
+        if (groups > trips) groups = trips;
+        p.group_heads = (uint32_t)((trips + groups - 1) / groups) * kHeadsPerTrip;
+        p.groups = (a->heads + p.group_heads - 1) / p.group_heads;
+        strips = plain * p.groups;
+        p.strips = (uint32_t)strips;
+    }
     unsigned long long want = (strips * 16 + threads - 1) / threads;
     // Grid: at most 8 resident CTAs per SM, a multiple of the SM count when capped.
     unsigned long long cap = (unsigned long long)sm_count_cached() * 8ull;
@@ -254,11 +334,9 @@ extern "C" int qwcu_prologue_launch(const qwcu_prologue_args *a, qwcu_stream str
     // nobody uses holds every SM to its even share (24 heads, 1152 rows: 15.3 -> 8.9 us, 10.3 us
     // without the early start; 2351 rows: 12.5 -> 10.9 us).  A smaller grid finds an SM for every
     // CTA, a larger one fills all of them (8.9 us at 320 rows, 20.1 us at 4352, either way).
-    if (!spread_ready()) return (int)cudaGetLastError();
-    const unsigned sms = (unsigned)sm_count_cached();
     const bool spread = 2 * blocks > sms && blocks <= 3 * sms;
     const size_t smem = spread ? spread_smem((blocks + sms - 1) / sms) : 0;
-    return sm100::launch(qw_prologue_kernel, blocks, threads, smem, 1, stream, p);
+    return sm100::launch(few ? qw_prologue_few_kernel : qw_prologue_kernel, blocks, threads, smem, 1, stream, p);
 }
 
 extern "C" int qwcu_scale_bf16_launch(void *out, const void *in, size_t elements, float scale,
