@@ -405,6 +405,7 @@ __device__ __forceinline__ uint32_t low_bits(int n) {
 //   a branch in every 32 keys              79.5 / 66.4    83.8 / 71.5
 //   every masked tile by mask_tile         85.4 / 62.0    90.8 / 67.2
 //   as now                                 68.5 / 61.8    76.2 / 67.0
+//   (since the rest has changed            65.3 / 59.2    71.4 / 62.1)
 // With a bound a tile's softmax stands twice in the code, with the masks in line and without.
 // Without one the 128 scores are in registers at once: rows that see nothing of a tile take one
 // select per score, and only tiles that some row sees a part of go through mask_tile.  A second
