@@ -434,65 +434,61 @@ __device__ __forceinline__ void mask_tile(uint32_t tmem_s, int key0, int limit, 
 }
 
 // 32 output rows of a warp, one destination: out = (w_own * O_own + w_other * O_other) * inv,
-// rounded to bf16.  A thread has a row in TMEM; 64 columns at a time go through a box of 32 rows
-// x 128 bytes in shared memory (16-byte pieces XOR-swizzled by the row) and from there to global
-// memory with eight lanes per row.  (tmem_own, tmem_other: kNoTmem where there is none.  Every
+// rounded to bf16.  A thread has a row in TMEM; 32 columns at a time go through a box of 32 rows
+// x 64 bytes in shared memory (16-byte pieces XOR-swizzled by the row, two boxes in turn) and from
+// there to global memory with four lanes per row.  (tmem_own, tmem_other: kNoTmem where there is none.  Every
 // lane takes part in the warp-collective TMEM loads.)
 //
 // Plain stores end with the instruction; a TMA store of the tile had to be waited for until it
 // had read shared memory, 1100 clocks at the end of every CTA.  And a function of its own: its
 // registers in one allocation with the softmax loop's cost that loop more than all of this (in
 // line, 8188 x 8211 keys took 1020 us instead of 955).  Six layers of 33 to 412 text rows took 45.2 to
-// 65.8 us and take 42.3 to 64.7; eight layers of six heads, 4352 keys, 555 -> 540 us.
+// 65.8 us and take 42.3 to 64.7; eight layers of six heads, 4352 keys, 555 -> 540 us.  (A function's
+// registers beyond some 60 are saved on the stack at its call: all 128 columns at once cost half a
+// microsecond a launch more; with 64 at a time six layers of 1500 text rows took 205.1 us, now 202.6.)
 constexpr uint32_t kNoTmem = 0xffffffffu;
 __device__ __noinline__ void write_rows(uint32_t tmem_own, uint32_t tmem_other, float w_own,
                                         float w_other, float inv, uint32_t box, __nv_bfloat16 *out,
                                         uint32_t row_stride, uint32_t rows) {
-    const uint32_t lane = threadIdx.x & 31u, first = lane >> 3, piece = lane & 7u;
+    const uint32_t lane = threadIdx.x & 31u, first = lane >> 2, piece = lane & 3u;
     out += (size_t)first * row_stride + piece * 8u;
 #pragma unroll 1
-    for (uint32_t half = 0; half < 2; ++half, out += 64) {
-        uint32_t o[64];
+    for (uint32_t c = 0; c < (uint32_t)kHeadDim; c += 32, out += 32, box ^= 2048u) {
+        uint32_t o[32];
         if (tmem_own != kNoTmem) {
-            QW_TMEM_LD32(tmem_own + half * 64, o);
-            QW_TMEM_LD32(tmem_own + half * 64 + 32, o + 32);
+            QW_TMEM_LD32(tmem_own + c, o);
             QW_TMEM_WAIT_LD32(o);
-            QW_TMEM_WAIT_LD32(o + 32);
         } else {
 #pragma unroll
-            for (int i = 0; i < 64; ++i) o[i] = 0u;
+            for (int i = 0; i < 32; ++i) o[i] = 0u;
         }
         if (tmem_other != kNoTmem) {
+            uint32_t x[32];
+            QW_TMEM_LD32(tmem_other + c, x);
+            QW_TMEM_WAIT_LD32(x);
 #pragma unroll
-            for (int part = 0; part < 64; part += 32) {
-                uint32_t x[32];
-                QW_TMEM_LD32(tmem_other + half * 64 + part, x);
-                QW_TMEM_WAIT_LD32(x);
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    o[part + i] = __float_as_uint(fmaf(__uint_as_float(x[i]), w_other,
-                                                       __uint_as_float(o[part + i]) * w_own));
-            }
+            for (int i = 0; i < 32; ++i)
+                o[i] = __float_as_uint(
+                    fmaf(__uint_as_float(x[i]), w_other, __uint_as_float(o[i]) * w_own));
         } else if (w_own != 1.0f) {
 #pragma unroll
-            for (int i = 0; i < 64; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * w_own);
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * w_own);
         }
-        __syncwarp();  // (the half before has been read)
 #pragma unroll
-        for (uint32_t c16 = 0; c16 < 8; ++c16) {
+        for (uint32_t c16 = 0; c16 < 4; ++c16) {
             uint32_t w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 w[i] = pack_bf16(__uint_as_float(o[8 * c16 + 2 * i]) * inv,
                                  __uint_as_float(o[8 * c16 + 2 * i + 1]) * inv);
-            st_shared16(box + lane * 128u + ((c16 ^ piece) << 4), w[0], w[1], w[2], w[3]);
+            st_shared16(box + lane * 64u + ((c16 ^ ((lane >> 1) & 3u)) << 4), w[0], w[1], w[2], w[3]);
         }
-        __syncwarp();
+        __syncwarp();  // (the box before is read while this one is written: one barrier is enough)
         __nv_bfloat16 *to = out;
 #pragma unroll
-        for (uint32_t i = 0; i < 8; ++i, to += 4 * (size_t)row_stride) {
-            const uint32_t r = 4u * i + first;
-            const uint4 x = ld_shared16(box + r * 128u + ((piece ^ (r & 7u)) << 4));
+        for (uint32_t i = 0; i < 4; ++i, to += 8 * (size_t)row_stride) {
+            const uint32_t r = 8u * i + first;
+            const uint4 x = ld_shared16(box + r * 64u + ((piece ^ ((r >> 1) & 3u)) << 4));
             if (r < rows) *reinterpret_cast<uint4 *>(to) = x;
         }
     }

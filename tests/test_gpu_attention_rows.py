@@ -1,4 +1,4 @@
-"""The attention kernel writes its output 32 rows per warp, eight lanes to a row: row counts
+"""The attention kernel writes its output 32 rows per warp, several lanes to a row: row counts
 around a warp's, a sub-tile's and a block's rows, in both forms, token- and head-major, against
 the CPU oracle, with rows that see nothing and with what lies behind the output left as it was.
 Tolerances as for the attention elsewhere."""
