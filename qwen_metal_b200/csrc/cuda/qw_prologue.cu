@@ -183,11 +183,15 @@ __global__ void __launch_bounds__(256) qw_prologue_kernel(const Params p) {
 // The same for few strips, where a strip's time is a chain of memory round trips and not
 // bandwidth: its first loads all leave together, a trip's loads run under the trip before, and
 // the heads of a row are dealt out to p.groups half-warps of p.group_heads each, as long as that
-// finds SMs with room.  77 registers: three CTAs per SM, where the form above has four, so it is
-// for grids of up to three per SM.  us a launch of q and k, the form above and this one: 24 heads, 320
-// rows 9.7 and 5.2, 1152 rows 12.3 and 7.6; 32 heads, 2351 rows 18.2 and 15.5; beyond, with one group, 6
-// heads of 4352 rows 8.2 and 9.8, 24 heads 21.1 and 22.9.
-__global__ void __launch_bounds__(256) qw_prologue_few_kernel(const Params p) {
+// finds SMs with room.  Two heads a trip (and the next two in flight) fit the registers of four CTAs
+// per SM, which is the largest grid it is for; four heads a trip fit three.  us a launch of q and k: the form
+// above, this one with trips of four, with trips of two: 24 heads, 320 rows 9.7, 4.9, 5.1; 1152 rows
+// 12.3, 7.5, 7.0; 32 heads, 2351 rows 18.2, 15.5, 13.6; 6 heads, 4352 rows 8.2, 9.8, 6.9; 24 heads, 3500 rows
+// -, 15.8, 16.2, 4352 rows 21.0, 22.9, 20.6.  Two waves of it are no better than the form above
+// (24 heads, 8704 rows 39.4 and 39.4, 16896 rows 72.1 and 73.5).
+constexpr int kFewTrip = 2, kFewPerSm = 4;
+constexpr uint32_t kFewGroup = 4;  // heads are dealt out by the four
+__global__ void __launch_bounds__(256, kFewPerSm) qw_prologue_few_kernel(const Params p) {
     sm100::grid_launch_dependents();
     sm100::grid_wait();
     const int lane16 = threadIdx.x & 15;
@@ -203,12 +207,12 @@ __global__ void __launch_bounds__(256) qw_prologue_few_kernel(const Params p) {
     const uint4 *w = which == 0 ? p.wq : which == 1 ? p.wk : nullptr;
     const bool rotate = p.cos_t && which < 2;
     const uint32_t begin = group * p.group_heads, end = min(p.heads, begin + p.group_heads);
-    const auto load_trip = [&](uint4 (&x)[kHeadsPerTrip], uint32_t head0) {
+    const auto load_trip = [&](uint4 (&x)[kFewTrip], uint32_t head0) {
 #pragma unroll
-        for (int u = 0; u < kHeadsPerTrip; ++u)
+        for (int u = 0; u < kFewTrip; ++u)
             x[u] = head0 + u < end ? src[(size_t)(head0 + u) * 16] : make_uint4(0, 0, 0, 0);
     };
-    uint4 x[kHeadsPerTrip];
+    uint4 x[kFewTrip];
     load_trip(x, begin);
     float4 c4 = make_float4(0, 0, 0, 0), s4 = c4;
     if (rotate) {
@@ -220,16 +224,16 @@ __global__ void __launch_bounds__(256) qw_prologue_few_kernel(const Params p) {
     const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
     const float wf[8] = {bf16_lo(wv.x), bf16_hi(wv.x), bf16_lo(wv.y), bf16_hi(wv.y),
                          bf16_lo(wv.z), bf16_hi(wv.z), bf16_lo(wv.w), bf16_hi(wv.w)};
-    for (uint32_t head0 = begin; head0 < end; head0 += kHeadsPerTrip) {
-        uint4 next[kHeadsPerTrip];
-        load_trip(next, head0 + kHeadsPerTrip);
+    for (uint32_t head0 = begin; head0 < end; head0 += kFewTrip) {
+        uint4 next[kFewTrip];
+        load_trip(next, head0 + kFewTrip);
 #pragma unroll
-        for (int u = 0; u < kHeadsPerTrip; ++u) {
+        for (int u = 0; u < kFewTrip; ++u) {
             const uint4 y = finish_head(p, x[u], w != nullptr, rotate, wf, cc, sn, half_mask);
             if (head0 + u < end) dst[(size_t)(head0 + u) * 16] = y;
         }
 #pragma unroll
-        for (int u = 0; u < kHeadsPerTrip; ++u) x[u] = next[u];
+        for (int u = 0; u < kFewTrip; ++u) x[u] = next[u];
     }
     if (p.bound_out && row == 0 && group == 0 && w) write_bound(p, which, wf, half_mask, lane16);
 }
@@ -312,14 +316,14 @@ extern "C" int qwcu_prologue_launch(const qwcu_prologue_args *a, qwcu_stream str
     const int threads = 256;
     const unsigned sms = (unsigned)sm_count_cached();
     if (!spread_ready()) return (int)cudaGetLastError();
-    const unsigned long long room = 3ull * sms * (threads / 16);  // half-warps of three CTAs per SM
+    const unsigned long long room = (unsigned long long)kFewPerSm * sms * (threads / 16);  // half-warps
     const unsigned long long plain = (unsigned long long)a->rows * p.tensors;
     const bool few = plain <= room;
     if (few) {
-        const uint32_t trips = (a->heads + kHeadsPerTrip - 1) / kHeadsPerTrip;
+        const uint32_t parts = (a->heads + kFewGroup - 1) / kFewGroup;
         unsigned long long groups = room / plain;
-        if (groups > trips) groups = trips;
-        p.group_heads = (uint32_t)((trips + groups - 1) / groups) * kHeadsPerTrip;
+        if (groups > parts) groups = parts;
+        p.group_heads = (uint32_t)((parts + groups - 1) / groups) * kFewGroup;
         p.groups = (a->heads + p.group_heads - 1) / p.group_heads;
         strips = plain * p.groups;
         p.strips = (uint32_t)strips;

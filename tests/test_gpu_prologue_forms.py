@@ -7,7 +7,7 @@ import pytest
 from qwen_metal_b200 import workloads
 
 pytestmark = pytest.mark.gpu
-MANY = 7200  # rows: more strips than three CTAs per SM hold (148 SMs of 48 strips)
+MANY = 9600  # rows: more strips than four CTAs per SM hold (148 SMs of 64 strips)
 
 
 @pytest.mark.parametrize("rows", [1, 5, 33, 320, 2351])
