@@ -453,7 +453,8 @@ __device__ __noinline__ void write_rows(uint32_t tmem_own, uint32_t tmem_other, 
     const uint32_t lane = threadIdx.x & 31u, first = lane >> 2, piece = lane & 3u;
     out += (size_t)first * row_stride + piece * 8u;
 #pragma unroll 1
-    for (uint32_t c = 0; c < (uint32_t)kHeadDim; c += 32, out += 32, box ^= 2048u) {
+    for (uint32_t c = 0; c < (uint32_t)kHeadDim; c += 32, out += 32) {
+        const uint32_t at = box + (c & 32u) * 64u;  // (the second box 2 KB behind the first)
         uint32_t o[32];
         if (tmem_own != kNoTmem) {
             QW_TMEM_LD32(tmem_own + c, o);
@@ -481,14 +482,14 @@ __device__ __noinline__ void write_rows(uint32_t tmem_own, uint32_t tmem_other, 
             for (int i = 0; i < 4; ++i)
                 w[i] = pack_bf16(__uint_as_float(o[8 * c16 + 2 * i]) * inv,
                                  __uint_as_float(o[8 * c16 + 2 * i + 1]) * inv);
-            st_shared16(box + lane * 64u + ((c16 ^ ((lane >> 1) & 3u)) << 4), w[0], w[1], w[2], w[3]);
+            st_shared16(at + lane * 64u + ((c16 ^ ((lane >> 1) & 3u)) << 4), w[0], w[1], w[2], w[3]);
         }
         __syncwarp();  // (the box before is read while this one is written: one barrier is enough)
         __nv_bfloat16 *to = out;
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i, to += 8 * (size_t)row_stride) {
             const uint32_t r = 8u * i + first;
-            const uint4 x = ld_shared16(box + r * 64u + ((piece ^ ((r >> 1) & 3u)) << 4));
+            const uint4 x = ld_shared16(at + r * 64u + ((piece ^ ((r >> 1) & 3u)) << 4));
             if (r < rows) *reinterpret_cast<uint4 *>(to) = x;
         }
     }
