@@ -7,7 +7,7 @@
 //   gate           : out = bf16(residual + branch * gate[row_map[row]])
 //                    (reference h3_shaders.metal:3583-3599)
 //
-// The norm keeps a row in registers (of four warps or of one, 16-byte loads, all of
+// The norm keeps a row in registers (one warp per row, 16-byte loads, all of
 // them in flight before the first use), so every input byte is read once and
 // every output byte written once; mean and variance are the reference's two
 // passes, done on the register copy.  Rows wider than the register budget, or
@@ -22,8 +22,10 @@
 
 namespace {
 
+// (128-thread CTAs: the row copy plus the prefetched modulation vectors take up to
+// about 150 registers per thread, and three to four such CTAs fit on an SM)
 constexpr int kWarpsPerBlock = 4;
-constexpr uint32_t kMaxWidth = 4096;  // four 16-byte vectors per lane of four warps
+constexpr int kMaxVecs = 16;  // 16-byte vectors per lane: rows up to 32 * 16 * 8 = 4096 columns
 
 __device__ __forceinline__ float bf16_lo(uint32_t pair) { return __uint_as_float(pair << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
@@ -88,8 +90,10 @@ __device__ __forceinline__ float row_sum(float v, float (&part)[kWarpsPerBlock])
 // width % 8 == 0 and width <= 32 * kRowWarps * kVecs * 8.
 // kRowWarps == 1: a warp walks rows (stride = warps in the grid); the grid holds a few
 // resident CTAs per SM, so no time goes into launching a CTA per handful of rows.
-// kRowWarps == kWarpsPerBlock: a CTA per row (320 rows of 3072: a 256^2 chain of four layers 340 ->
-// 317 us, 1152 rows: 512^2 523 -> 509 us; many rows: see the launch).
+// kRowWarps == kWarpsPerBlock: a CTA per row, for so few rows that a warp of the first
+// form would have one row at most: its time is then the latency of one row, and four
+// warps get through it sooner (320 rows of 3072: a 256^2 chain of four layers 340 -> 317 us,
+// 1152 rows: 512^2 523 -> 509 us).
 template <int kVecs, int kRowWarps>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 qw_layer_norm_mod_kernel(const NormArgs a) {
@@ -268,33 +272,42 @@ extern "C" int qwcu_layer_norm_mod_launch(const qwcu_rowwise_args *a, int sm_cou
     k.status = a->status;
     if (!a->maps) return (int)cudaErrorInvalidValue;
     const unsigned blocks = (a->rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    const bool vector = a->width % 8 == 0 && a->width <= kMaxWidth &&
+    const bool vector = a->width % 8 == 0 && a->width <= 32u * kMaxVecs * 8u &&
                         aligned16(k.in) && aligned16(k.out) && aligned16(k.modulation);
     constexpr unsigned threads = kWarpsPerBlock * 32;
     if (!vector)
         return sm100::launch(qw_layer_norm_mod_generic_kernel, blocks, threads, 0, 1, stream, k);
-    // A CTA per row, unless rows are both many (more than the warps of four CTAs per SM) and
-    // narrow: then a warp per row, walking rows in as many CTAs as are resident (a smaller grid,
-    // started under the tail of the kernel before it, would pile up on the SMs that are free first).
-    // A quarter of a row per warp takes a quarter of the registers, so that four times the rows are
-    // in flight: us a launch, a warp per row and a CTA per row, 8704 rows of 1024 8.4 and 11.2, of
-    // 1536 13.1 and 13.2, of 2048 15.5 and 14.8, of 3072 24.5 and 19.8, of 4096 34.1 and 24.1; 4096
-    // rows of 3072 13.9 and 11.0; 20000 rows of 3072 46.2 and 40.5.
-    // (The four warps' sums are added in another order than one warp takes them in; the error against
-    // 64 bits is the same: 1.659298e-3 either way on 4096 rows of 3072, 126 and 119 outputs that are
-    // not the nearest bf16, at mean 3 on 3000 rows 1732 and 1723.)
+    // With fewer rows than the warps of four CTAs per SM a CTA takes one row.  More rows:
+    // warps that walk rows, in as many CTAs as the registers let be resident.  Started under
+    // the tail of the kernel before it, a smaller grid would pile up on the SMs that are free
+    // first (8704 rows of 1024: 10.9 us with 4 per SM, 6.6 us with 8; of 2048: 14.1 us with 4,
+    // 10.6 us with 5), and a larger one has a second wave (of 4096: 39.5 us with 4, 31.5 us
+    // with 3).
+    // A CTA per row would be quicker for many wide rows too (8704 rows of 3072 24.5 -> 19.8 us, of
+    // 4096 34.1 -> 24.2 us), but its four warps add a row's sums in another order, and two layers on
+    // the other roundings of one bf16 value are 3e-3 of the result.  With the order kept it is
+    // slower: partial sums handed from warp to warp 39.3 and 45.2 us, a warp per row held
+    // to 80 registers for six CTAs per SM 27.2 us (3072 columns).
     const unsigned sms = (unsigned)(sm_count > 0 ? sm_count : 148);
+    const bool few = blocks <= sms * 4u;
     const uint32_t vecs_per_lane = (a->width / 8 + 31) / 32;
-    if (vecs_per_lane <= 4 && blocks > sms * 4u) {
-        const unsigned resident = sms * 8u;
-        return sm100::launch(qw_layer_norm_mod_kernel<4, 1>, blocks < resident ? blocks : resident,
-                             threads, 0, 1, stream, k);
+    void (*kernel)(const NormArgs);
+    unsigned resident;
+    if (vecs_per_lane <= 4) {
+        kernel = few ? qw_layer_norm_mod_kernel<1, 4> : qw_layer_norm_mod_kernel<4, 1>;
+        resident = 8;
+    } else if (vecs_per_lane <= 8) {
+        kernel = few ? qw_layer_norm_mod_kernel<2, 4> : qw_layer_norm_mod_kernel<8, 1>;
+        resident = 5;
+    } else if (vecs_per_lane <= 12) {
+        kernel = few ? qw_layer_norm_mod_kernel<3, 4> : qw_layer_norm_mod_kernel<12, 1>;
+        resident = 4;
+    } else {
+        kernel = few ? qw_layer_norm_mod_kernel<4, 4> : qw_layer_norm_mod_kernel<kMaxVecs, 1>;
+        resident = 3;
     }
-    return sm100::launch(vecs_per_lane <= 4    ? qw_layer_norm_mod_kernel<1, 4>
-                         : vecs_per_lane <= 8  ? qw_layer_norm_mod_kernel<2, 4>
-                         : vecs_per_lane <= 12 ? qw_layer_norm_mod_kernel<3, 4>
-                                               : qw_layer_norm_mod_kernel<4, 4>,
-                         a->rows, threads, 0, 1, stream, k);
+    const unsigned grid = few ? a->rows : blocks < sms * resident ? blocks : sms * resident;
+    return sm100::launch(kernel, grid, threads, 0, 1, stream, k);
 }
 
 extern "C" int qwcu_gate_launch(const qwcu_rowwise_args *a, int sm_count, qwcu_stream stream_) {

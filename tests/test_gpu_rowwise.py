@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import oracle_lib as O
-from qwen_metal_b200 import workloads
+from qwen_metal_b200 import abi, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -176,3 +176,59 @@ def test_norm_mod_forms_match_oracle(gpu, rows, width):
     row_map = rng.integers(0, 2, rows).astype(np.uint32)
     got = run_norm(gpu, x, mod, row_map, rows, width, 3, 1)
     check_norm(got, O.layer_norm_mod(x, mod, row_map, rows, width, 3, 1, 1e-6))
+
+
+def sums_in_order(x, lanes):
+    """A row's two sums in float32, in the order of the kernel's form with `lanes` lanes to a row:
+    a lane takes every lanes-th vector of 8, the lanes of a warp meet in a butterfly, four warps
+    are added one behind the other.  Returns mean and variance.  (A product of two floats is exact
+    in 64 bits, so the fma is one rounding there and one back.)"""
+    rows, width = x.shape
+    vecs = width // 8
+    steps = -(-vecs // lanes)
+    held = np.zeros((rows, steps * lanes, 8), np.float32)
+    held[:, :vecs] = x.reshape(rows, vecs, 8)
+    held = held.reshape(rows, steps, lanes, 8)
+    real = (np.arange(steps * lanes) < vecs).reshape(steps, lanes)
+
+    def meet(v):
+        v = v.reshape(rows, -1, 32)
+        for off in (16, 8, 4, 2, 1):
+            v = v + v[:, :, np.arange(32) ^ off]
+        total = v[:, 0, 0]
+        for warp in range(1, v.shape[1]):
+            total = total + v[:, warp, 0]
+        return (total / np.float32(width)).astype(np.float32)
+
+    acc = np.zeros((rows, lanes), np.float32)
+    for i in range(steps):
+        for k in range(0, 8, 2):
+            acc = acc + (held[:, i, :, k] + held[:, i, :, k + 1])
+    mean = meet(acc)
+    acc = np.zeros((rows, lanes), np.float32)
+    for i in range(steps):
+        for k in range(8):
+            c = (held[:, i, :, k] - mean[:, None]).astype(np.float64)
+            acc = np.where(real[i], (c * c + acc).astype(np.float32), acc)
+    return mean, meet(acc)
+
+
+@pytest.mark.parametrize("rows,width", [
+    (2368, 3072), (64, 1032),                # a CTA per row: the last row count on 148 SMs
+    (2369, 1024), (2369, 1032), (2961, 2048), (4096, 3072), (2369, 3080), (2369, 4096),  # a warp per row
+])
+def test_norm_sums_keep_their_order(gpu, rows, width):
+    """Bit for bit: the order of a row's sums is part of the result.  Another one flips the
+    rounding of one output in a hundred thousand, which the oracle's comparison allows and two
+    layers turn into 3e-3 of theirs."""
+    import torch
+
+    rng = np.random.default_rng(rows + width)
+    x = workloads.normal_bf16(rng, (rows, width), 0.3, 1.7)
+    mod = workloads.normal_bf16(rng, (1, 1, width), 0.0, 0.5)
+    got = run_norm(gpu, x, mod, np.zeros(rows, np.uint32), rows, width, 1, 0)
+    xf, scale = O.bf16_to_f32(x), np.float32(1.0) + O.bf16_to_f32(mod).reshape(1, width)
+    mean, var = sums_in_order(xf, 128 if rows <= 2368 else 32)
+    inverse = torch.rsqrt(torch.from_numpy(var + np.float32(1e-6)).cuda()).cpu().numpy()
+    want = abi.f32_to_bf16((xf - mean[:, None]) * inverse[:, None] * scale)
+    assert np.array_equal(got, want), int((got != want).sum())
