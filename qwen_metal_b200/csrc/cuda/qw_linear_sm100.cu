@@ -145,6 +145,17 @@ __device__ __forceinline__ Item item_at(const Params &p, uint32_t i) {
     return it;
 }
 
+// How many of a warp's `boxes` (64 columns each, the first from column col0 on) hold columns of
+// an output of n: the last tile may reach past it, with a box or with both.
+__host__ __device__ constexpr int boxes_inside(int boxes, uint32_t col0, uint32_t n) {
+    return col0 >= n ? 0 : boxes == 2 && col0 + 64u >= n ? 1 : boxes;
+}
+static_assert(boxes_inside(2, 2688, 2688) == 0 && boxes_inside(2, 2752, 2688) == 0 &&
+                  boxes_inside(2, 2624, 2688) == 1 && boxes_inside(2, 2560, 2688) == 2 &&
+                  boxes_inside(2, 2560, 2632) == 2 && boxes_inside(1, 2624, 2688) == 1 &&
+                  boxes_inside(1, 2688, 2688) == 0 && boxes_inside(0, 0, 2688) == 0,
+              "a warp's boxes at the end of an output");
+
 // 32 columns of one row out of the accumulator, as packed bf16 pairs: the GEMM result
 // (plus bias) rounded to bf16.
 __device__ __forceinline__ void row_from_tmem(uint32_t (&pk)[16], uint32_t taddr, const uint16_t *bias,
@@ -340,8 +351,7 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
             // The second box of a CTA's last tile is staged in the ring, which is done with.
             uint8_t *const spare = i + step < p.items ? stage : ring + ew * kStoreBytes;
             const int boxes = off >= it.cols || row0 >= p.m ? 0 : wide ? 2 : 1;
-            // (the last columns of the last tile may lie past the output's)
-            const int live = boxes == 2 && col0 + 64u >= p.n_each ? 1 : col0 >= p.n_each ? 0 : boxes;
+            const int live = boxes_inside(boxes, col0, p.n_each);
             // The rotation's entries of a box: lane l takes four pairs (16 bytes of cos and of
             // sin) of rows l / 8, l / 8 + 4, ..., so that a load touches four rows' lines and not
             // 32.  The first box's are on their way while the accumulator is still filling.
@@ -366,7 +376,7 @@ qw_linear_sm100_kernel(const __grid_constant__ Maps maps, const Params p) {
                 break;
             tc_fence_after();
             const uint32_t src = lanes + acc * kN + off;
-            const uint16_t *bias = p.bias[it.which] ? p.bias[it.which] + col0 : nullptr;
+            const uint16_t *bias = live && p.bias[it.which] ? p.bias[it.which] + col0 : nullptr;
             float inverse = 0.0f;
             if (fused && live) {  // serial fma over the bf16 values, element order 0..127
                 float ss = 0.0f;

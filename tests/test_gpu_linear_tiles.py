@@ -4,6 +4,8 @@ pair, the half tiles of a partly filled last wave), against the CPU oracle on th
 around the tile borders.  Tolerance as for the GEMM elsewhere: fp32 sums in another
 order, one rounding to bf16.  linear_plans.py holds what each size is dispatched to on
 148 SMs; the tests fail where it is something else."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -82,6 +84,53 @@ def test_fused_epilogue_on_every_tile_shape(gpu, seq, dim):
     assert np.array_equal(fk, want_k.reshape(fk.shape)), float((fk != want_k.reshape(fk.shape)).mean())
     assert np.array_equal(fv.reshape(seq, dim), got[2])
     for t in [xt, wqt, wkt, ct, st, bt] + wts + plain + fused:
+        gpu.free(t)
+
+
+class LinearArgs(C.Structure):
+    """qwcu_linear_args."""
+    _fields_ = [("a", C.c_void_p), ("w", C.c_void_p * 3), ("c", C.c_void_p * 3), ("bias", C.c_void_p * 3),
+                ("n_outputs", C.c_uint32), ("m", C.c_uint32), ("k", C.c_uint32), ("n", C.c_uint32),
+                ("norm_weight", C.c_void_p * 2), ("rope_cos", C.c_void_p), ("rope_sin", C.c_void_p),
+                ("table_rows", C.c_uint32), ("epsilon", C.c_float), ("bound_out", C.c_void_p),
+                ("status", C.c_void_p), ("wait_cycles", C.c_longlong), ("withhold_from", C.c_uint32 * 2)]
+
+
+@pytest.mark.parametrize("rows,dim", [(200, 512), (513, 2688)])  # (21 heads: half a tile past each output)
+def test_fused_epilogue_takes_a_bias(gpu, rows, dim):
+    """The launch takes a bias together with the norm and the rotation, which no op asks for: bit
+    for bit the projection with a bias, then the oracle's norm and rotation."""
+    P.check(gpu, rows, dim, 3)
+    rng = np.random.default_rng(rows)
+    lib, heads, k = gpu.lib, dim // 128, 72
+    ptr = lib.qw_gpu_tensor_device_ptr
+    x = gpu.bf16(workloads.normal_bf16(rng, (rows, k)))
+    ws = [gpu.bf16(weights(rng, dim, k)) for _ in range(3)]
+    bs = [gpu.bf16(workloads.normal_bf16(rng, (dim,))) for _ in range(3)]
+    norms = [workloads.normal_bf16(rng, (128,), 1.0, 0.1) for _ in range(2)]
+    angle = rng.uniform(-3, 3, (rows, 64))
+    cos, sin = np.cos(angle).astype(np.float32), np.sin(angle).astype(np.float32)
+    rest = [gpu.bf16(norms[0]), gpu.bf16(norms[1]), gpu.f32(cos), gpu.f32(sin), gpu.u32(np.zeros(16, np.uint32))]
+    plain, fused = ([gpu.new_bf16(rows * dim) for _ in range(3)] for _ in range(2))
+    args = LinearArgs(a=ptr(x), n_outputs=3, m=rows, k=k, n=dim, rope_cos=ptr(rest[2]), rope_sin=ptr(rest[3]),
+                      table_rows=rows, epsilon=1e-6, status=ptr(rest[4]))
+    for i in range(3):
+        args.w[i], args.c[i], args.bias[i] = ptr(ws[i]), ptr(fused[i]), ptr(bs[i])
+    for i in range(2):
+        args.norm_weight[i] = ptr(rest[i])
+    launch = lib.qwcu_linear_sm100_launch
+    launch.restype, launch.argtypes = C.c_int, [C.POINTER(LinearArgs), C.c_int, C.c_void_p]
+    gpu.begin()
+    for i in range(3):
+        gpu.check(lib.h3_gpu_linear_bf16(gpu.handle, plain[i], x, ws[i], bs[i], rows, k, dim), "linear")
+    assert launch(C.byref(args), lib.qwcu_device_sm_count(0), lib.qw_gpu_stream(gpu.handle)) == 0
+    gpu.submit()
+    got = [gpu.read_bf16(t, rows * dim).reshape(rows, heads, 128) for t in plain]
+    normed = [O.head_rms_norm(g, w, rows, heads, 1e-6) for g, w in zip(got, norms)]
+    want = [*O.qk_rope(*normed, cos, sin, rows, heads), got[2]]
+    for t, w in zip(fused, want):
+        assert np.array_equal(gpu.read_bf16(t, rows * dim).reshape(w.shape), w)
+    for t in [x] + ws + bs + rest + plain + fused:
         gpu.free(t)
 
 
