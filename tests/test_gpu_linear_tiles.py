@@ -47,30 +47,38 @@ def test_every_tile_shape_matches_oracle(gpu, rows, k, n, bias):
         gpu.free(t)
 
 
-@pytest.mark.parametrize("seq,dim", [
-    (200, 512),    # 128-column pair tiles: a head per tile
-    (300, 4096),   # single CTAs: two heads per tile, the second by the second warp group
-    (1152, 3072),  # pairs: two whole tiles on either accumulator, then halves of one head
-    (513, 2688),   # 21 heads: the last tile of every output holds one
+@pytest.mark.parametrize("batch,table,dim", [
+    (1, 200, 512),    # 128-column pair tiles: a head per tile
+    (1, 300, 4096),   # single CTAs: two heads per tile, the second by the second warp group
+    (1, 1152, 3072),  # pairs: two whole tiles on either accumulator, then halves of one head
+    (1, 513, 2688),   # 21 heads: the last tile of every output holds one
+    # the same with a rotation table that begins again between, inside and many times in the boxes
+    # of 32 rows, in 256-column tiles and halves, on a first and a last tile of a CTA
+    (100, 2, 512), (60, 5, 4096), (4, 75, 4096), (9, 128, 3072), (384, 3, 3072), (12, 96, 3072), (19, 27, 2688),
 ])
-def test_fused_epilogue_on_every_tile_shape(gpu, seq, dim):
+def test_fused_epilogue_on_every_tile_shape(gpu, batch, table, dim):
     """q/k/v with the norm and the rotation in the epilogue: the plain projection against
     the oracle on a row sample, the fused one bit for bit against the oracle's norm and
     rotation of the plain one's bf16 output, v equal to the plain one's."""
+    seq = batch * table
     P.check(gpu, seq, dim, 3)
     rng = np.random.default_rng(seq + dim)
     lib, heads = gpu.lib, dim // 128
     x = workloads.normal_bf16(rng, (seq, dim))
     ws = [weights(rng, dim, dim) for _ in range(3)]
     wq, wk = (workloads.normal_bf16(rng, (128,), 1.0, 0.1) for _ in range(2))
-    cos, sin = abi.rope_tables(seq - 144, 12, 12)
+    if batch == 1:
+        cos, sin = abi.rope_tables(seq - 144, 12, 12)
+    else:
+        angle = rng.uniform(-3, 3, (table, 64))
+        cos, sin = np.cos(angle).astype(np.float32), np.sin(angle).astype(np.float32)
     xt, wts = gpu.bf16(x), [gpu.bf16(w) for w in ws]
     plain, fused = ([gpu.new_bf16(seq * dim) for _ in range(3)] for _ in range(2))
     wqt, wkt, ct, st, bt = gpu.bf16(wq), gpu.bf16(wk), gpu.f32(cos), gpu.f32(sin), gpu.new_f32(2)
     gpu.begin()
     gpu.check(lib.qw_gpu_qkv_bf16(gpu.handle, *plain, xt, *wts, seq, dim), "qkv")
-    gpu.check(lib.qw_gpu_qkv_norm_rope_bf16(gpu.handle, *fused, xt, *wts, wqt, wkt, ct, st, bt, 1, seq,
-                                            dim, 1e-6), "qkv norm rope")
+    gpu.check(lib.qw_gpu_qkv_norm_rope_bf16(gpu.handle, *fused, xt, *wts, wqt, wkt, ct, st, bt, batch,
+                                            table, dim, 1e-6), "qkv norm rope")
     gpu.submit()
     got = [gpu.read_bf16(t, seq * dim).reshape(seq, dim) for t in plain]
     sample = np.array([0, 31, 32, 127, 128, seq // 2, seq - 1], np.uint32)
@@ -78,7 +86,7 @@ def test_fused_epilogue_on_every_tile_shape(gpu, seq, dim):
         check_gemm(g[sample], O.linear(x, w, None, seq, dim, dim, sample)[sample], f"{name} {seq}x{dim}")
     normed = [O.head_rms_norm(g.reshape(seq, heads, 128), w, seq, heads, 1e-6)
               for g, w in zip(got, (wq, wk))]
-    want_q, want_k = O.qk_rope(*normed, cos, sin, seq, heads)
+    want_q, want_k = O.qk_rope(*normed, np.tile(cos, (batch, 1)), np.tile(sin, (batch, 1)), seq, heads)
     fq, fk, fv = (gpu.read_bf16(t, seq * dim).reshape(seq, heads, 128) for t in fused)
     assert np.array_equal(fq, want_q.reshape(fq.shape)), float((fq != want_q.reshape(fq.shape)).mean())
     assert np.array_equal(fk, want_k.reshape(fk.shape)), float((fk != want_k.reshape(fk.shape)).mean())
