@@ -73,44 +73,44 @@ constexpr int kHeadsPerTrip = 4;
 __device__ __forceinline__ uint4 finish_head(const Params &p, const uint4 &x, bool norm, bool rotate,
                                              const float (&wf)[8], const float (&cc)[4],
                                              const float (&sn)[4], uint32_t half_mask) {
-                    float v[8] = {bf16_lo(x.x), bf16_hi(x.x), bf16_lo(x.y), bf16_hi(x.y),
-                                  bf16_lo(x.z), bf16_hi(x.z), bf16_lo(x.w), bf16_hi(x.w)};
-                    uint32_t y[4] = {x.x, x.y, x.z, x.w};
-                    if (norm) {
-                        float ss = 0.0f;
-    #pragma unroll
-                        for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
-    #pragma unroll
-                        for (int off = 8; off > 0; off >>= 1)
-                            ss += __shfl_xor_sync(half_mask, ss, off, 16);
-                        // mean = ss / 128 exactly; 1/sqrt to within 2 ulp of the reference's rsqrt
-                        const float inv = rsqrtf(__fadd_rn(ss * 0.0078125f, p.eps));
-    #pragma unroll
-                        for (int i = 0; i < 8; i += 2) {
-                            float n0 = __fmul_rn(v[i], inv), n1 = __fmul_rn(v[i + 1], inv);
-                            if (p.double_round) {
-                                const uint32_t r = pack_bf16x2(n0, n1);
-                                n0 = bf16_lo(r);
-                                n1 = bf16_hi(r);
-                            }
-                            y[i >> 1] = pack_bf16x2(__fmul_rn(n0, wf[i]), __fmul_rn(n1, wf[i + 1]));
-                        }
-                        if (rotate) {
-    #pragma unroll
-                            for (int i = 0; i < 4; ++i) {  // the bf16 store between norm and rotation
-                                v[2 * i] = bf16_lo(y[i]);
-                                v[2 * i + 1] = bf16_hi(y[i]);
-                            }
-                        }
-                    }
-                    if (rotate) {
-    #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float e = v[2 * i], o = v[2 * i + 1];
-                            y[i] = pack_bf16x2(__fsub_rn(__fmul_rn(e, cc[i]), __fmul_rn(o, sn[i])),
-                                               __fadd_rn(__fmul_rn(e, sn[i]), __fmul_rn(o, cc[i])));
-                        }
-                    }
+    float v[8] = {bf16_lo(x.x), bf16_hi(x.x), bf16_lo(x.y), bf16_hi(x.y),
+                  bf16_lo(x.z), bf16_hi(x.z), bf16_lo(x.w), bf16_hi(x.w)};
+    uint32_t y[4] = {x.x, x.y, x.z, x.w};
+    if (norm) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1)
+            ss += __shfl_xor_sync(half_mask, ss, off, 16);
+        // mean = ss / 128 exactly; 1/sqrt to within 2 ulp of the reference's rsqrt
+        const float inv = rsqrtf(__fadd_rn(ss * 0.0078125f, p.eps));
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            float n0 = __fmul_rn(v[i], inv), n1 = __fmul_rn(v[i + 1], inv);
+            if (p.double_round) {
+                const uint32_t r = pack_bf16x2(n0, n1);
+                n0 = bf16_lo(r);
+                n1 = bf16_hi(r);
+            }
+            y[i >> 1] = pack_bf16x2(__fmul_rn(n0, wf[i]), __fmul_rn(n1, wf[i + 1]));
+        }
+        if (rotate) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {  // the bf16 store between norm and rotation
+                v[2 * i] = bf16_lo(y[i]);
+                v[2 * i + 1] = bf16_hi(y[i]);
+            }
+        }
+    }
+    if (rotate) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float e = v[2 * i], o = v[2 * i + 1];
+            y[i] = pack_bf16x2(__fsub_rn(__fmul_rn(e, cc[i]), __fmul_rn(o, sn[i])),
+                               __fadd_rn(__fmul_rn(e, sn[i]), __fmul_rn(o, cc[i])));
+        }
+    }
     return make_uint4(y[0], y[1], y[2], y[3]);
 }
 
@@ -183,12 +183,18 @@ __global__ void __launch_bounds__(256) qw_prologue_kernel(const Params p) {
 // The same for few strips, where a strip's time is a chain of memory round trips and not
 // bandwidth: its first loads all leave together, a trip's loads run under the trip before, and
 // the heads of a row are dealt out to p.groups half-warps of p.group_heads each, as long as that
-// finds SMs with room.  Two heads a trip (and the next two in flight) fit the registers of four CTAs
-// per SM, which is the largest grid it is for; four heads a trip fit three.  us a launch of q and k: the form
-// above, this one with trips of four, with trips of two: 24 heads, 320 rows 9.7, 4.9, 5.1; 1152 rows
-// 12.3, 7.5, 7.0; 32 heads, 2351 rows 18.2, 15.5, 13.6; 6 heads, 4352 rows 8.2, 9.8, 6.9; 24 heads, 3500 rows
-// -, 15.8, 16.2, 4352 rows 21.0, 22.9, 20.6.  Two waves of it are no better than the form above
-// (24 heads, 8704 rows 39.4 and 39.4, 16896 rows 72.1 and 73.5).
+// finds SMs with room.  Two heads a trip (and the next two in flight) fit the registers of four
+// CTAs per SM, which is the largest grid it is for; four heads a trip fit three.  us a launch of
+// q and k:
+//                         form above   trips of four   trips of two
+//   24 heads,  320 rows       9.7            4.9            5.1
+//   24 heads, 1152 rows      12.2            7.5            7.0
+//   32 heads, 2351 rows      18.2           15.5           13.7
+//   24 heads, 3500 rows      17.0           15.8           16.3
+//    6 heads, 4352 rows       8.1            9.8            6.9
+//   24 heads, 4352 rows      21.0           22.9           20.7
+// Two waves of it are no better than the form above (24 heads, 8704 rows 39.4 and 39.4, 16896
+// rows 72.1 and 73.5).
 constexpr int kFewTrip = 2, kFewPerSm = 4;
 constexpr uint32_t kFewGroup = 4;  // heads are dealt out by the four
 __global__ void __launch_bounds__(256, kFewPerSm) qw_prologue_few_kernel(const Params p) {
@@ -202,8 +208,9 @@ __global__ void __launch_bounds__(256, kFewPerSm) qw_prologue_few_kernel(const P
     if (row >= p.rows) return;  // (the reductions name their own 16 lanes)
     const uint32_t group = rest / (uint32_t)p.tensors;
     const uint32_t which = rest - group * (uint32_t)p.tensors;  // 0 query, 1 key, 2 value
-    const uint4 *src = (which == 0 ? p.q_in : which == 1 ? p.k_in : p.v_in) + (size_t)row * p.heads * 16 + lane16;
-    uint4 *dst = (which == 0 ? p.q_out : which == 1 ? p.k_out : p.v_out) + (size_t)row * p.heads * 16 + lane16;
+    const size_t at = (size_t)row * p.heads * 16 + lane16;
+    const uint4 *src = (which == 0 ? p.q_in : which == 1 ? p.k_in : p.v_in) + at;
+    uint4 *dst = (which == 0 ? p.q_out : which == 1 ? p.k_out : p.v_out) + at;
     const uint4 *w = which == 0 ? p.wq : which == 1 ? p.wk : nullptr;
     const bool rotate = p.cos_t && which < 2;
     const uint32_t begin = group * p.group_heads, end = min(p.heads, begin + p.group_heads);
@@ -274,9 +281,7 @@ bool spread_ready() {
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     const bool tracked = dev >= 0 && dev < 64;
     if (tracked && ready[dev]) return true;
-    if (cudaFuncSetAttribute(qw_prologue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)spread_smem(1)) != cudaSuccess ||
-        cudaFuncSetAttribute(qw_prologue_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(qw_prologue_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)spread_smem(1)) != cudaSuccess)
         return false;
     if (tracked) ready[dev] = true;
@@ -313,34 +318,31 @@ extern "C" int qwcu_prologue_launch(const qwcu_prologue_args *a, qwcu_stream str
     strips = (strips + 1ull) & ~1ull;  // whole warps iterate together
     if (strips > 0xffffffffull) return (int)cudaErrorInvalidValue;
     p.strips = (uint32_t)strips;
-    const int threads = 256;
-    const unsigned sms = (unsigned)sm_count_cached();
+    const unsigned threads = 256, sms = (unsigned)sm_count_cached();
     if (!spread_ready()) return (int)cudaGetLastError();
     const unsigned long long room = (unsigned long long)kFewPerSm * sms * (threads / 16);  // half-warps
     const unsigned long long plain = (unsigned long long)a->rows * p.tensors;
-    const bool few = plain <= room;
-    if (few) {
+    if (plain <= room) {
         const uint32_t parts = (a->heads + kFewGroup - 1) / kFewGroup;
         unsigned long long groups = room / plain;
         if (groups > parts) groups = parts;
         p.group_heads = (uint32_t)((parts + groups - 1) / groups) * kFewGroup;
         p.groups = (a->heads + p.group_heads - 1) / p.group_heads;
-        strips = plain * p.groups;
-        p.strips = (uint32_t)strips;
+        const unsigned blocks = (unsigned)((plain * p.groups * 16 + threads - 1) / threads);
+        // Started under the tail of the kernel before it (sm100::launch), a grid of half a CTA to
+        // three CTAs per SM would pile up on the SMs that are free first.  Shared memory that
+        // nobody uses holds every SM to its even share (32 heads, 700 rows 7.8 -> 6.8 us; 24 heads,
+        // 1152 rows 7.9 -> 7.0, 3500 rows 18.3 -> 16.3; 2351 rows of 32 heads 13.7, 320 of 24 heads
+        // 5.1 either way).  A smaller grid finds an SM for every CTA, a larger one fills all of them.
+        const bool spread = 2 * blocks > sms && blocks <= 3 * sms;
+        const size_t smem = spread ? spread_smem((blocks + sms - 1) / sms) : 0;
+        return sm100::launch(qw_prologue_few_kernel, blocks, threads, smem, 1, stream, p);
     }
-    unsigned long long want = (strips * 16 + threads - 1) / threads;
+    const unsigned long long want = (strips * 16 + threads - 1) / threads;
     // Grid: at most 8 resident CTAs per SM, a multiple of the SM count when capped.
-    unsigned long long cap = (unsigned long long)sm_count_cached() * 8ull;
-    unsigned int blocks = (unsigned int)(want < cap ? want : cap);
-    if (!blocks) blocks = 1;
-    // Started under the tail of the kernel before it (sm100::launch), a grid of half a CTA to
-    // three CTAs per SM would pile up on the SMs that are free first.  Shared memory that
-    // nobody uses holds every SM to its even share (24 heads, 1152 rows: 15.3 -> 8.9 us, 10.3 us
-    // without the early start; 2351 rows: 12.5 -> 10.9 us).  A smaller grid finds an SM for every
-    // CTA, a larger one fills all of them (8.9 us at 320 rows, 20.1 us at 4352, either way).
-    const bool spread = 2 * blocks > sms && blocks <= 3 * sms;
-    const size_t smem = spread ? spread_smem((blocks + sms - 1) / sms) : 0;
-    return sm100::launch(few ? qw_prologue_few_kernel : qw_prologue_kernel, blocks, threads, smem, 1, stream, p);
+    const unsigned long long cap = sms * 8ull;
+    const unsigned blocks = (unsigned)(want < cap ? want : cap);
+    return sm100::launch(qw_prologue_kernel, blocks, threads, 0, 1, stream, p);
 }
 
 extern "C" int qwcu_scale_bf16_launch(void *out, const void *in, size_t elements, float scale,
