@@ -126,7 +126,6 @@ constexpr size_t kSmemData = (size_t)(2 + kStages) * kTileBytes;
 constexpr size_t kSmemBytes = kSmemData + sizeof(SharedControl) + 1024;  // +1024: manual alignment
 
 struct KernelParams {
-    __nv_bfloat16 *out;
     const int32_t *kv_limit;
     uint32_t *status;
 #ifdef QW_ATTN_TRACE
@@ -176,7 +175,7 @@ __device__ __forceinline__ uint32_t bar_at(uint32_t bars, uint32_t which) {
 // A wait ran out: the first one of the launch leaves its place in the status words, and the other
 // waits of the CTA end.
 __device__ __noinline__ void record_expiry(SharedControl *ctl, uint32_t *status, uint32_t where,
-                                              uint32_t tile) {
+                                           uint32_t tile) {
     ctl->abort_flag = 1;
     if (atomicCAS(status, 0u, (uint32_t)QWCU_STATUS_WAIT_TIMEOUT) == 0u) {
         status[1] = where;
@@ -503,8 +502,7 @@ template <bool kBounded>
 __device__ __forceinline__ void softmax_role(const KernelParams &p, SharedControl *ctl,
                                              uint8_t *stage, int sub, int tid_in_group,
                                              int my_limit, uint32_t b, uint32_t h,
-                                             uint32_t row, uint32_t tile_row0, bool split,
-                                             float bound) {
+                                             uint32_t tile_row0, bool split, float bound) {
     const int warp_in_group = tid_in_group >> 5;
     const uint32_t lane_base = (uint32_t)(warp_in_group * 32) << 16;
     const uint32_t tmem = ctl->tmem_base;
@@ -917,7 +915,7 @@ __device__ __forceinline__ void mma_role_split(const KernelParams &p, SharedCont
 #define QW_RING_WAIT(t_, lo_fixed_, out_)                                                       \
     {                                                                                           \
         const uint32_t slot_ = (t_) % kStages, par_ = ((t_) / kStages) & 1u;                    \
-        if (!mbar_wait_warp(p, bar_at(bars, kBarKvFull + slot_), par_))                           \
+        if (!mbar_wait_warp(p, bar_at(bars, kBarKvFull + slot_), par_))                         \
             return mma_gave_up(ctl, p.status, kBarKvFull + slot_, (t_));                        \
         tc_fence_after();                                                                       \
         out_ = (kv_lo + slot_ * (kTileBytes >> 4)) | (lo_fixed_);                               \
@@ -1146,7 +1144,6 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
     // Row limits: each softmax thread owns one row; the largest limit of a
     // sub-tile bounds its key-tile loop.
     int my_limit = 0;
-    uint32_t my_row = 0;
     int sub = 0, tid_in_group = 0;
     // Fixed reference exponent (log2 units, an integer so that P is the exact
     // power-of-two multiple of what any other reference would give), or < 0 for
@@ -1161,7 +1158,7 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         sub = tid >> 7;
         tid_in_group = tid & 127;
         // (split form: both warpgroups work on the same 128 rows)
-        my_row = row0 + (split ? 0u : (uint32_t)sub * kTileM) + (uint32_t)tid_in_group;
+        const uint32_t my_row = row0 + (split ? 0u : (uint32_t)sub * kTileM) + (uint32_t)tid_in_group;
         my_limit = row_limit(p, b, my_row);
         int warp_max = my_limit;
         // A row past the end is computed like its neighbours and never stored: with a
@@ -1199,11 +1196,10 @@ qw_attn_sm100_kernel(const __grid_constant__ CUtensorMap map_q,
         uint8_t *stage = smem_q + (size_t)sub * kTileBytes;
         const uint32_t tile_row0 = split ? row0 : row0 + (uint32_t)sub * kTileM;
         if (kMayBound && bound >= 0.0f)
-            softmax_role<kMayBound>(p, ctl, stage, sub, tid_in_group, my_limit, b, h,
-                                    my_row, tile_row0, split, bound);
+            softmax_role<kMayBound>(p, ctl, stage, sub, tid_in_group, my_limit, b, h, tile_row0, split,
+                                    bound);
         else
-            softmax_role<false>(p, ctl, stage, sub, tid_in_group, my_limit, b, h, my_row,
-                                tile_row0, split, 0.0f);
+            softmax_role<false>(p, ctl, stage, sub, tid_in_group, my_limit, b, h, tile_row0, split, 0.0f);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
     }
@@ -1346,7 +1342,6 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
     if ((rc = make_map_3d(&map_k, a->k, a->batch, a->kv_rows, a->kv_heads))) return rc;
     if ((rc = make_map_3d(&map_v, a->v, a->batch, a->kv_rows, a->kv_heads))) return rc;
     KernelParams p;
-    p.out = static_cast<__nv_bfloat16 *>(a->out);
     p.kv_limit = a->kv_limit;
     p.status = a->status;
 #ifdef QW_ATTN_TRACE
@@ -1376,7 +1371,7 @@ extern "C" int qwcu_attn_sm100_launch(const qwcu_attn_args *a, qwcu_stream strea
         p.out_head_offset = a->out_head_offset;
     } else {
         p.n_out = 1;
-        p.out_peers[0] = p.out;
+        p.out_peers[0] = static_cast<__nv_bfloat16 *>(a->out);
         p.out_heads_total = a->heads;
         p.out_head_offset = 0;
     }
