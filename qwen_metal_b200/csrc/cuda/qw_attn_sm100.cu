@@ -82,8 +82,8 @@ static_assert(2 * 128 * kSoftmaxRegs + 128 * kOtherRegs <= kThreads * kLaunchReg
               "setmaxnreg budget exceeds the launch allocation");
 // P of a tile is published in two parts, the first kPart * 16 keys and the rest: P V of
 // the first part runs under the softmax of the rest, which takes it out of the chain
-// S -> softmax -> P V -> next S that bounds the kernel (six heads, 4352 keys, with a bound:
-// 622 us with 4, 601 us with 6; 8188 x 8211 keys without one: 980 us with 4, 955 us with 6).
+// S -> softmax -> P V -> next S that bounds the kernel (eight layers of six heads, 4352 keys, with
+// a bound: 528 us with 4, 513 us with 6; 8188 x 8211 keys without one: 966 and 945 us).
 constexpr int kPart = 6;
 constexpr int kSoftmaxThreads = 256;
 constexpr int kMmaWarp = 8;
@@ -165,9 +165,8 @@ struct KernelParams {
     int mma_probes;  // the same budget for the MMA warp's waits, in probes
 };
 
-// Shared address of a barrier.  (The roles keep the first one's and add: with a conversion from a
-// pointer at every wait and commit, six heads, eight layers took 535 instead of 529 us, 24 heads of
-// two, four layers 1687 instead of 1650.)
+// Shared address of a barrier.  (The roles keep the first one's and add: a conversion from a pointer
+// at every wait and commit cost 1 % with six heads and 4352 keys, 2 % with 24 heads of two.)
 __device__ __forceinline__ uint32_t bar_at(uint32_t bars, uint32_t which) {
     return bars + which * (uint32_t)sizeof(Mbar);
 }
@@ -213,9 +212,8 @@ __device__ __forceinline__ bool mbar_wait(SharedControl *ctl, uint32_t bar,
 // The wait of the MMA warp, for all its lanes at once, bounded by a number of probes that the host
 // makes of the budget.  The warp issues every MMA of the CTA and each of its clocks is on the chain
 // of both sub-tiles, so the loop holds nothing else: with the clock and the abort flag of the wait
-// above behind 32 probes, in line or called, six heads take 633 to 658 instead of 571 us for eight
-// layers, 24 heads of two 1825 to 1890 instead of 1725 us for four.  A probe that fails suspends
-// the warp for a time that the hardware sets: 400 000 of them took 1.58 s, 7800 clocks each.
+// above behind 32 probes, in line or called, layers of six heads, 4352 keys, took 11 to 15 % longer,
+// of 24 heads of two 6 to 10 %.  A probe that fails suspends the warp for a time that the hardware sets: 400 000 of them took 1.58 s, 7800 clocks each.
 constexpr long long kProbeCycles = 10000;
 __device__ __forceinline__ bool mbar_wait_warp(const KernelParams &p, uint32_t bar, uint32_t parity) {
     bool ok = false;
@@ -393,24 +391,22 @@ __device__ __forceinline__ uint32_t low_bits(int n) {
 // 32 scores of keys key0 .. key0 + 31: those the row does not see become -infinity.  The
 // row's mask is made once for the 32 keys and a score costs a bit test and a select, where
 // comparing its key with the limit and the padding window took three compares and a select.
-// (When every 32 keys carried the masks in line, six heads of 4352 rows, 64 of them text, went
-// from 102 to 78 us with a bound and from 115 to 82 us without.)
+// (When every 32 keys carried the masks in line, that took a quarter off a launch of six heads
+// and 4352 rows, 64 of them text.)
 //
 // Where text rows, which see few keys, share a block with image rows, their warps mask every tile
-// and the launch waits for them.  Tiles without a mask must not pay for it either: a branch in
-// every 32 keys costs 66 instead of 62 us where the 256 text rows have a block of their own.  Six
-// heads, 4352 rows, 64 / 256 of them text, us a launch:
+// and the launch waits for them.  Tiles without a mask must not pay for it either: 256 text rows
+// have a block of their own.  Six heads, 4352 rows, 64 / 256 of them text, a launch's time over
+// that of the present form, and the present form's us:
 //                                        with a bound      without
-//   a branch in every 32 keys              79.5 / 66.4    83.8 / 71.5
-//   every masked tile by mask_tile         85.4 / 62.0    90.8 / 67.2
-//   as now                                 68.5 / 61.8    76.2 / 67.0
-//   (since the rest has changed            65.3 / 59.2    71.4 / 62.1)
+//   a branch in every 32 keys              1.16 / 1.07    1.10 / 1.07
+//   every masked tile by mask_tile         1.25 / 1.00    1.19 / 1.00
+//   as now                            us   65.3 / 59.2    71.4 / 62.1
 // With a bound a tile's softmax stands twice in the code, with the masks in line and without.
 // Without one the 128 scores are in registers at once: rows that see nothing of a tile take one
 // select per score, and only tiles that some row sees a part of go through mask_tile.  A second
 // copy there is slower where launches are short, since each reads the code anew (six launches of
-// 412 text rows: 68.7 instead of 66.1 us), and so are the bits of all masks in registers (66.5 us,
-// 80 us with 64 text rows).
+// 412 text rows: 4 %), and so are the bits of all masks in registers (1 %, 5 % with 64 text rows).
 __device__ __forceinline__ void mask_scores(uint32_t *s, int key0, int limit, int pad_lo, int pad_hi) {
     const uint32_t visible =
         low_bits(limit - key0) & ~(low_bits(pad_hi - key0) & ~low_bits(pad_lo - key0));
@@ -435,16 +431,16 @@ __device__ __forceinline__ void mask_tile(uint32_t tmem_s, int key0, int limit, 
 // 32 output rows of a warp, one destination: out = (w_own * O_own + w_other * O_other) * inv,
 // rounded to bf16.  A thread has a row in TMEM; 32 columns at a time go through a box of 32 rows
 // x 64 bytes in shared memory (16-byte pieces XOR-swizzled by the row, two boxes in turn) and from
-// there to global memory with four lanes per row.  (tmem_own, tmem_other: kNoTmem where there is none.  Every
-// lane takes part in the warp-collective TMEM loads.)
+// there to global memory with four lanes per row.  (tmem_own, tmem_other: kNoTmem where there is
+// none.  Every lane takes part in the warp-collective TMEM loads.)
 //
 // Plain stores end with the instruction; a TMA store of the tile had to be waited for until it
 // had read shared memory, 1100 clocks at the end of every CTA.  And a function of its own: its
 // registers in one allocation with the softmax loop's cost that loop more than all of this (in
-// line, 8188 x 8211 keys took 1020 us instead of 955).  Six layers of 33 to 412 text rows took 45.2 to
-// 65.8 us and take 42.3 to 64.7; eight layers of six heads, 4352 keys, 555 -> 540 us.  (A function's
-// registers beyond some 60 are saved on the stack at its call: all 128 columns at once cost half a
-// microsecond a launch more; with 64 at a time six layers of 1500 text rows took 205.1 us, now 202.6.)
+// line, 8188 x 8211 keys took 7 % longer).  Against the TMA stores layers of 33 to 412 text rows
+// gained 6 to 2 %, of six heads, 4352 keys, 3 %.  (A function's registers beyond some 60 are saved
+// on the stack at its call: all 128 columns at once cost half a microsecond a launch, 64 at a time
+// 1 % of a layer of 1500 text rows.)
 constexpr uint32_t kNoTmem = 0xffffffffu;
 __device__ __noinline__ void write_rows(uint32_t tmem_own, uint32_t tmem_other, float w_own,
                                         float w_other, float inv, uint32_t box, __nv_bfloat16 *out,
@@ -831,8 +827,8 @@ __device__ __forceinline__ void mma_role(const KernelParams &p, SharedControl *c
     // to 110 even where nothing is left to wait for.  So the next tiles of K and of V are waited
     // for behind the first parts of P V, where the warp waits for the rest of P anyway, and not both
     // in front of the step; and the two sub-tiles take turns in one loop, whose code is half as long.
-    // Eight layers of six heads, 4352 keys: 560 us before, 552 us, 537 us with the epilogue's
-    // registers out of the softmax's way as well (see write_rows).
+    // Layers of six heads, 4352 keys, gained 1.4 %, and 2.7 % more with the epilogue's registers out
+    // of the softmax's way (see write_rows).
     while (j < n_max) {
         const int jn = j + 1;
         const bool more = jn < n_max;

@@ -32,7 +32,7 @@
 // loops are rolled (a row's columns are read from TMEM twice instead of being held), and the
 // last tile's second box is staged in the ring instead of waiting for the first one's store.
 // 320 rows of 3072, clocks from complete accumulator to stores issued: 12700 -> 3700; chains of
-// four layers, 256^2 301 -> 283 us, 512^2 487 -> 472 us.
+// four layers, 256^2 279 -> 262 us, 512^2 477 -> 460 us.
 //
 // Every wait is bounded (status words, abort flag).  A CTA leaves nothing in flight, also
 // after a wait has run out: see the end of the kernel.

@@ -280,14 +280,14 @@ extern "C" int qwcu_layer_norm_mod_launch(const qwcu_rowwise_args *a, int sm_cou
     // With fewer rows than the warps of four CTAs per SM a CTA takes one row.  More rows:
     // warps that walk rows, in as many CTAs as the registers let be resident.  Started under
     // the tail of the kernel before it, a smaller grid would pile up on the SMs that are free
-    // first (8704 rows of 1024: 10.9 us with 4 per SM, 6.6 us with 8; of 2048: 14.1 us with 4,
-    // 10.6 us with 5), and a larger one has a second wave (of 4096: 39.5 us with 4, 31.5 us
+    // first (8704 rows of 1024: 10.3 us with 4 per SM, 8.4 us with 8; of 2048: 17.8 us with 4,
+    // 15.6 us with 5), and a larger one has a second wave (of 4096: 42.2 us with 4, 34.2 us
     // with 3).
     // A CTA per row would be quicker for many wide rows too (8704 rows of 3072 24.5 -> 19.8 us, of
-    // 4096 34.1 -> 24.2 us), but its four warps add a row's sums in another order, and two layers on
-    // the other roundings of one bf16 value are 3e-3 of the result.  With the order kept it is
-    // slower: partial sums handed from warp to warp 39.3 and 45.2 us, a warp per row held
-    // to 80 registers for six CTAs per SM 27.2 us (3072 columns).
+    // 4096 34.1 -> 24.2 us), but its four warps add a row's sums in another order: one output in a
+    // hundred thousand rounds the other way, and two layers make 3e-3 of their result of it.  With
+    // the order kept it is slower: partial sums handed from warp to warp 39.3 and 45.2 us, a warp
+    // per row held to 80 registers for six CTAs per SM 27.2 us (3072 columns).
     const unsigned sms = (unsigned)(sm_count > 0 ? sm_count : 148);
     const bool few = blocks <= sms * 4u;
     const uint32_t vecs_per_lane = (a->width / 8 + 31) / 32;
